@@ -1,0 +1,147 @@
+"""Corridors: the two-sided search that cuts a query's graph down before the
+label search, at the sizes where it can go wrong.
+
+Every case compares cost, delay and feasibility with the CPU oracle's label
+setting under exact Dijkstra bounds (cost and delay are integers: equality).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(n, arcs):
+    arcs = sorted(arcs)
+    row = np.zeros(n + 1, np.int64)
+    for a in arcs:
+        row[a[0] + 1] += 1
+    return (np.cumsum(row), np.array([a[1] for a in arcs], np.int32),
+            np.array([a[2] for a in arcs], np.float32), np.array([a[3] for a in arcs], np.float32))
+
+
+def _line(n, rng):
+    """A path graph with a fast and a slow arc a step (both directions)."""
+    out = []
+    for i in range(n - 1):
+        for u, x in ((i, i + 1), (i + 1, i)):
+            out.append((u, x, int(rng.integers(1, 50)), int(rng.integers(50, 100))))
+            out.append((u, x, int(rng.integers(50, 100)), int(rng.integers(1, 50))))
+    return n, out
+
+
+def _star(spokes, rng):
+    """Source -> spokes -> sink and a few chords: two hubs of `spokes` arcs."""
+    n, out = spokes + 2, []
+    for i in range(spokes):
+        out.append((0, 2 + i, int(rng.integers(1, 1000)), int(rng.integers(1, 1000))))
+        out.append((2 + i, 1, int(rng.integers(1, 1000)), int(rng.integers(1, 1000))))
+        if i % 7 == 0:
+            out.append((2 + i, 2 + int(rng.integers(spokes)), int(rng.integers(0, 9)), int(rng.integers(0, 9))))
+    return n, out
+
+
+def _layers(width, depth, rng, w=100):
+    """`depth` layers of `width` vertices, three arcs each to the next layer."""
+    n, out = width * depth, []
+    for d in range(depth - 1):
+        for i in range(width):
+            for _ in range(3):
+                out.append((d * width + i, (d + 1) * width + int(rng.integers(width)),
+                            int(rng.integers(0, w + 1)), int(rng.integers(0, w + 1))))
+    return n, out
+
+
+CASES = {
+    # name: (maker, source, sink)
+    "line2": (lambda r: _line(2, r), 0, 1),
+    "line33": (lambda r: _line(33, r), 0, 32),
+    "line700": (lambda r: _line(700, r), 3, 690),
+    "star31": (lambda r: _star(31, r), 0, 1),       # one warp
+    "star257": (lambda r: _star(257, r), 0, 1),     # hubs, shared by the block
+    "star5000": (lambda r: _star(5000, r), 0, 1),   # queue past its shared part
+    "layers": (lambda r: _layers(40, 30, r), 5, 29 * 40 + 7),
+    "layers_wide": (lambda r: _layers(3000, 10, r), 5, 9 * 3000 + 9),  # shrinks in steps
+    "heavy_arcs": (lambda r: _layers(30, 20, r, w=400000), 1, 19 * 30 + 2),
+}
+
+
+def _check(v, O, g, og, s, t, budgets, cfg):
+    h_len, h_del = O.lower_bounds(og, t)
+    src, dst = np.full(len(budgets), s, np.int32), np.full(len(budgets), t, np.int32)
+    res = v.solve(g, src, dst, np.asarray(budgets, np.float32), cfg)
+    for q, b in enumerate(budgets):
+        want = O.solve_label_setting(og, s, t, float(b), h_len, h_del, use_incumbent=True)
+        assert bool(res.found[q]) == want["found"], (q, b)
+        if not want["found"]:
+            continue
+        assert (float(res.cost[q]), float(res.delay[q])) == (want["cost"], want["delay"]), (q, b)
+        p = res.path(q)
+        assert p[0] == s and p[-1] == t
+        low_cost = low_delay = 0.0  # parallel arcs: the path's sums lie at or above these
+        for u, x in zip(p[:-1], p[1:]):
+            heads, ln, dl = g.out_edges(int(u))
+            assert (heads == x).any()
+            low_cost += float(ln[heads == x].min())
+            low_delay += float(dl[heads == x].min())
+        assert low_cost <= want["cost"] and low_delay <= want["delay"] <= b
+
+
+@pytest.mark.parametrize("threads,table", [(512, 13), (128, 11), (64, 6)])
+@pytest.mark.parametrize("name", list(CASES))
+def test_matches_oracle(name, threads, table):
+    import vine_b200 as v
+    from oracle import oracle as O
+    make, s, t = CASES[name]
+    n, arcs = make(np.random.default_rng(17))
+    csr = _graph(n, arcs)
+    g, og = v.Graph(*csr), O.CsrGraph(*csr)
+    lo = O.dijkstra(og, s, "delay")[0][t]
+    hi = O.dijkstra(og, s, "len")[1][t]
+    if not np.isfinite(lo):
+        lo, hi = 50.0, 100.0
+    budgets = [lo - 1, lo, lo + 0.5, lo + 0.1 * (hi - lo), lo + 0.5 * (hi - lo), hi, 2 * hi + 10,
+               2.0 ** 24, np.inf]  # the last two: the whole-graph bounds
+    cfg = v.Config(use_bounds=1, policy="ar", block_threads=threads, table_log2=table,
+                   pool_labels=1 << 24)
+    _check(v, O, g, og, s, t, budgets, cfg)
+    _check(v, O, g, og, s, t, budgets, v.Config(use_bounds=1, sync_rounds=1, pool_labels=1 << 24))
+    g.close()
+
+
+def test_corridor_past_its_capacity():
+    """70,000 equal two-arc ways: more vertices than a local graph holds, so
+    the query is answered with the bounds over the whole graph."""
+    import vine_b200 as v
+    k = 70000
+    n, arcs = k + 2, []
+    for i in range(k):
+        arcs += [(0, 2 + i, 5, 7), (2 + i, 1, 6, 8)]
+    g = v.Graph(*_graph(n, arcs))
+    res = v.solve(g, [0, 0], [1, 1], [15, 14], v.Config(use_bounds=1, pool_labels=1 << 24))
+    assert res.found.tolist() == [1, 0]
+    assert (res.cost[0], res.delay[0]) == (11, 15)
+    g.close()
+
+
+def test_costs_past_2_24():
+    """A path cost of 2^24 or more goes to the whole-graph bounds; the same
+    graph's cheaper sink does not."""
+    import vine_b200 as v
+    arcs = [(0, 1, 16000000, 3), (1, 2, 16000000, 3), (0, 2, 33000000 // 2, 9)]
+    g = v.Graph(*_graph(3, arcs))
+    res = v.solve(g, [0, 0, 0], [1, 2, 2], [10, 6, 9], v.Config(use_bounds=1, pool_labels=1 << 24))
+    assert res.found.tolist() == [1, 1, 1]
+    assert res.cost.tolist() == [16000000, 32000000, 16500000]
+    assert res.delay.tolist() == [3, 6, 9]
+    g.close()
+
+
+def test_zero_weights_and_unreachable():
+    import vine_b200 as v
+    arcs = [(0, 1, 0, 0), (1, 2, 0, 0), (2, 0, 0, 0), (2, 3, 0, 4), (0, 3, 2, 0), (4, 0, 1, 1)]
+    g = v.Graph(*_graph(5, arcs))
+    cfg = v.Config(use_bounds=1, pool_labels=1 << 24)
+    res = v.solve(g, [0, 0, 0, 0, 1], [2, 3, 3, 4, 1], [0, 0, 4, 1e6, 0], cfg)
+    assert res.found.tolist() == [1, 1, 1, 0, 1]
+    assert res.cost[:3].tolist() == [0, 2, 0] and res.delay[:3].tolist() == [0, 0, 4]
+    g.close()

@@ -25,6 +25,7 @@
 //                      algorithm/bucket.cuh:217-245)
 //   * arena         -- every accepted label with its parent, for paths
 
+#include "corridor.cuh"
 #include "engine_host.h"
 #include "search.cuh"
 
@@ -276,16 +277,17 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
       e = __ldcg(&ring[(h + (uint32_t)lane) & P.near_mask]);
       // an entry outside the arena or the vertex range would mean a protocol
       // slip: fail the query instead of following it
-      entry_ok = (uint64_t)e.x < (uint64_t)P.pool_cap && e.y < (uint32_t)P.g.n;
+      entry_ok = (uint64_t)e.x < (uint64_t)P.pool_cap && e.y < (uint32_t)c.g.n;
       if (!entry_ok) fail_query(st, VINE_ERR_INTERNAL, kSiteRing);
     }
     if (entry_ok) {
       idx = e.x;
       const int v = (int)e.y;
       const Label lab = load_label(&P.pool[idx]);  // issued together with the loads below
-      const VView s = P.use_bounds ? c.view(v) : VView{0.0f, true, 0.0f, 0.0f, 0u};
-      const int r0 = __ldg(&P.g.row[v]);
-      const int r1 = __ldg(&P.g.row[v + 1]);
+      const VView s = c.bounds != kBoundsNone ? c.view(v) : VView{0.0f, true, 0.0f, 0.0f, 0u, 0u};
+      // (plain loads: a local graph is written by this kernel)
+      const int r0 = c.g.row[v];
+      const int r1 = c.g.row[v + 1];
       d = lab.d;
       dl = lab.dl;
       bool live = !(lab.vid & (int)kDeadBit);
@@ -294,7 +296,9 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
         if (!(f < hi)) live = false;
         if (live && P.mode == VINE_MODE_OPTIMAL) {
           const uint64_t key = pack_key(f, dl + s.hdel);
-          if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) live = false;
+          const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
+          if (key >= inc) live = false;
+          else if (c.bounds == kBoundsLocal && beyond_mix(st, d, dl, s.hmix, inc)) live = false;
         }
       }
       if (live) {
@@ -353,8 +357,8 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
         int u = 0;
         if (e < total) {
           const int j = obeg + (e - oex);
-          u = __ldg(&P.g.col[j]);
-          const float2 w = __ldg(&P.g.w[j]);
+          u = c.g.col[j];
+          const float2 w = c.g.w[j];
           const VView s = c.view(u);
           offer_with(c, u, od + w.x, odl + w.y, oidx, false, s, &nidx);
         }
@@ -692,7 +696,46 @@ __device__ __forceinline__ void tile_issue_bins(TileStage &ts, int k, const Labe
   ts.busy |= 1u << k;
 }
 
-__global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
+// Lays out worker `slot`'s corridor arrays (one thread).
+__device__ __forceinline__ void corridor_mem(const SearchParams &P, int slot, CorridorMem &M) {
+  M.rf = P.rf + (size_t)slot * P.g.n;
+  M.touch[0] = P.touch + (size_t)slot * 2 * P.g.n;
+  M.touch[1] = M.touch[0] + P.g.n;
+  M.ovf[0] = P.nearq + (size_t)slot * 2 * (P.near_mask + 1u);
+  M.ovf[1] = M.ovf[0] + (P.near_mask + 1u);
+  M.ovf_cap = P.near_mask + 1u;
+  M.far[0] = reinterpret_cast<unsigned long long *>(P.far + (size_t)slot * P.far_cap * 4);
+  M.far[1] = reinterpret_cast<unsigned long long *>(P.rest + (size_t)slot * P.rest_cap);
+  M.far_cap = (uint32_t)min(min(P.far_cap * 4, P.rest_cap) * 2, (int64_t)0x7fffffff);
+  M.lv = P.lv;
+  M.la = P.la;
+  const size_t lv = (size_t)P.lv, la = (size_t)P.la;
+  int32_t *ip = P.lint + (size_t)slot * corridor_ints(P.lv, P.la);
+  float2 *wp = P.lw + (size_t)slot * 4 * la;
+  for (int k = 0; k < 2; ++k) {
+    DevGraph &g = M.loc[k].g;
+    g.m = 0;
+    g.n = 0;
+    g.row = ip;
+    g.rrow = ip + lv + 1;
+    g.col = ip + 2 * (lv + 1);
+    g.rcol = g.col + la;
+    M.loc[k].gid = const_cast<int32_t *>(g.rcol) + la;
+    ip = M.loc[k].gid + lv;
+    g.w = wp;
+    g.rw = wp + la;
+    wp += 2 * la;
+  }
+  M.map = reinterpret_cast<uint32_t *>(ip);
+  for (int k = 0; k < 4; ++k) M.dist[k] = P.ldist + ((size_t)slot * 4 + k) * lv;
+  M.lvs = P.lvs + (size_t)slot * lv;
+}
+
+// kBounds: the call uses lower bounds (corridors).  Without them the corridor
+// code and its state are compiled out: they would cost the plain bucketed
+// search registers (12 % on a 45 x 45 grid with default settings).
+template <bool kBounds>
+__global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ SearchParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int H = 1 << P.table_log2;
   const int NL = 1 << P.lock_log2;
@@ -703,7 +746,9 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
   float2 *tw = reinterpret_cast<float2 *>(tv + H);
   uint32_t *ti = reinterpret_cast<uint32_t *>(tw + H);
   int *locks = reinterpret_cast<int *>(ti + H);
-  uint32_t *r_idx = reinterpret_cast<uint32_t *>(locks + NL);
+  // the corridor's wave state lies over the table and its locks
+  WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  uint32_t *r_idx = reinterpret_cast<uint32_t *>(smem + table_region_bytes(P.table_log2, P.lock_log2));
   int *r_vid = reinterpret_cast<int *>(r_idx + RC);
   float *r_d = reinterpret_cast<float *>(r_vid + RC);
   float *r_dl = r_d + RC;
@@ -724,8 +769,10 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
   const int tid = threadIdx.x, G = blockDim.x;
   const int slot = blockIdx.x;
   Ctx c(P, st);
+  c.bounds = kBounds ? kBoundsGlobal : kBoundsNone;
   const RoundBuf rb{r_idx, r_vid, r_d, r_dl, r_beg, r_off, scan, RC};
-  c.vs = P.vs + (size_t)slot * P.g.n;
+  VState *const global_vs = P.vs + (size_t)slot * P.g.n;
+  c.vs = global_vs;
   c.nearq = P.nearq + (size_t)slot * 2 * (P.near_mask + 1u);  // uint2 entries
   c.far = P.far + (size_t)slot * P.far_cap * 4;
   c.rest = P.rest + (size_t)slot * P.rest_cap;
@@ -811,6 +858,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
       st.split_cycles = st.split_items = st.policy_cycles = st.rest_items = 0;
       st.idle_cycles = st.publish_cycles = 0;
       st.load_cycles = st.relax_cycles = 0;
+      st.lam_a = st.lam_b = st.lam_bB = 0;
       st.hist_n = 0;
       st.sink_n = 0;
       st.b_labels = st.b_expanded = st.b_rounds = st.b_dominated = 0;
@@ -846,18 +894,47 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
       }
     }
     __syncthreads();
+    if (kBounds) {
+      c.g = P.g;
+      c.vs = c.bt.vs = global_vs;
+      c.bounds = kBoundsGlobal;
+      c.gid = nullptr;
+    }
     if (!st.done && !st.abort) {
-      if (P.use_bounds) {
+      if (kBounds) {
         const long long t_b = clock64();
         const long long r_b = st.n_rounds;
-        cta_reverse_search(c, rb, 0, st.budget, P.delta_del);
-        cta_reverse_search(c, rb, 1, INFINITY, P.delta_len);
+        int how = kCorridorNone, which = 0;
+        if (P.rf != nullptr && st.budget < kIntLimit) {
+          if (tid == 0) corridor_mem(P, slot, W.m);
+          __syncthreads();
+          how = corridor_prepare(P, st, &which);
+          const LocalGraph loc = W.m.loc[which];
+          VState *const lvs = W.m.lvs;
+          __syncthreads();
+          for (int i = tid; i < H; i += G) tv[i] = kEmpty;  // the wave state lay here
+          for (int i = tid; i < NL; i += G) locks[i] = 0;
+          if (how == kCorridorReady) {
+            c.g = loc.g;
+            c.gid = loc.gid;
+            c.vs = c.bt.vs = lvs;
+            c.bounds = kBoundsLocal;
+            if (tid == 0) P.pool[st.inc_idx].vid = st.src;
+          } else if (how == kCorridorInfeasible && tid == 0) {
+            st.done = 1;
+          }
+          __syncthreads();
+        }
+        if (how == kCorridorNone && !st.abort) {
+          cta_reverse_search(c, rb, 0, st.budget, P.delta_del);
+          cta_reverse_search(c, rb, 1, INFINITY, P.delta_len);
+        }
         if (tid == 0) {
           st.bound_cycles = clock64() - t_b;
           st.n_bound_rounds = st.n_rounds - r_b;
         }
       }
-      if (tid == 0 && !st.abort) {
+      if (tid == 0 && !st.abort && !st.done) {
         const VView sv = c.view(st.src);
         const uint32_t idx = st.inc_idx;
         st.inc_idx = 0xffffffffu;
@@ -1198,9 +1275,10 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(SearchParams P) {
     }
     __syncthreads();
     if (tid == 0) {
-      copy_out_path(P, st, q, st.abort == 0 && st.inc_key != ~0ull);
+      // a corridor seeds inc_key with its cost bound before a label has it
       const bool ok = st.abort == 0;
-      const bool found = ok && st.inc_key != ~0ull;
+      const bool found = ok && st.inc_key != ~0ull && st.inc_idx != 0xffffffffu;
+      copy_out_path(P, st, q, found, c.gid);
       P.status[q] = ok ? VINE_OK : st.abort;
       P.found[q] = found ? 1 : 0;
       P.cost[q] = found ? key_d(st.inc_key) : INFINITY;
@@ -1247,14 +1325,17 @@ __global__ void epoch_kernel(unsigned long long *counters, int32_t nq) {
 
 size_t batch_smem_bytes(int table_log2, int lock_log2, int round_cap, int block_threads,
                         int staging) {
-  size_t b = ((sizeof(int32_t) + sizeof(float2) + sizeof(uint32_t)) << table_log2) +
-             (sizeof(int) << lock_log2) +
-             (size_t)round_cap * 24 + kScanScratch * sizeof(int);
+  size_t b = table_region_bytes(table_log2, lock_log2) + (size_t)round_cap * 24 + kScanScratch * sizeof(int);
   b = (b + 15) & ~(size_t)15;
   b += sizeof(QueryState) + 16;
   if (!staging) return b;
   // two staged label tiles (128-byte aligned) and their barriers
   return b + 128 + 2 * (size_t)block_threads * kSplitBatch * sizeof(Label) + 2 * sizeof(uint64_t);
+}
+
+using BatchKernel = void (*)(SearchParams);
+BatchKernel kernel_for(const vine_config &c) {
+  return c.use_bounds ? batch_kernel<true> : batch_kernel<false>;
 }
 
 int lock_log2_for(int table_log2) { return std::max(5, table_log2 - 1); }
@@ -1279,8 +1360,43 @@ void BatchWorkspace::release() {
   cudaFree(counters);
   cudaFree(order);
   cudaFree(trace);
+  cudaFree(rf);
+  cudaFree(touch);
+  cudaFree(lint);
+  cudaFree(lw);
+  cudaFree(ldist);
+  cudaFree(lvs);
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   *this = BatchWorkspace();
+}
+
+// The corridor arrays of every worker, allocated by the first call that uses
+// the bounds.  A graph so large that they would take more than an eighth of
+// the device's memory (some 10 million vertices) goes without them: its
+// queries get the two reverse searches over the whole graph.
+static int ensure_corridor(vine_graph *g, const Resolved &r) {
+  BatchWorkspace &w = g->batch;
+  if (!r.cfg.use_bounds || w.rf != nullptr) return VINE_OK;
+  const size_t n = (size_t)g->n;
+  const size_t lv = std::min<size_t>(n, kCorridorVertices);
+  const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
+  const size_t ints = corridor_ints((int)lv, (int)la);
+  const size_t per = n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
+                     lv * (4 * sizeof(unsigned long long) + sizeof(VState));
+  size_t free_b = 0, total_b = 0;
+  VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+  if (per * r.slots > total_b / 8) return VINE_OK;
+  const size_t k = (size_t)r.slots;
+  VINE_CUDA_TRY(cudaMalloc(&w.touch, sizeof(uint32_t) * 2 * n * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lvs, sizeof(VState) * lv * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
+  VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
+  w.lv = (int)lv;
+  w.la = (int)la;
+  return VINE_OK;
 }
 
 static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) {
@@ -1320,6 +1436,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     w.pool_cap = c.pool_labels;
     w.epoch_next = 1;
   }
+  VINE_TRY(ensure_corridor(g, r));
   if (w.q_cap < nq) {
     cudaFree(w.order);
     cudaFree(w.path_start);
@@ -1365,7 +1482,7 @@ int batch_prepare(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t str
   const size_t smem = batch_smem_bytes(r.cfg.table_log2, lock_log2_for(r.cfg.table_log2),
                                        r.cfg.sync_rounds ? r.round_cap : 0, r.cfg.block_threads,
                                        r.cfg.split_staging);
-  VINE_CUDA_TRY(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(r.cfg), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   return VINE_OK;
 }
@@ -1438,6 +1555,23 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.split_staging = c.split_staging;
   P.wait_limit = c.wait_limit;
   P.time_limit_ns = c.time_limit_ms > 0 ? (unsigned long long)c.time_limit_ms * 1000000ull : 0ull;
+  P.rf = c.use_bounds ? w.rf : nullptr;
+  P.touch = w.touch;
+  P.lint = w.lint;
+  P.lw = w.lw;
+  P.ldist = w.ldist;
+  P.lvs = w.lvs;
+  P.lv = w.lv;
+  P.la = w.la;
+  P.mean_len = g->mean_len;
+  P.mean_delay = g->mean_delay;
+  // Buckets of the corridor searches: some mean arcs wide on sparse graphs.
+  // With more arcs a vertex improves more often per bucket, so they narrow
+  // with the square of the mean degree (degree 18, 100,000 vertices: 12 ms of
+  // two-sided search for 64 queries with the linear rule, 7 ms so).
+  const float deg = (float)g->m / (float)std::max(1, g->n);
+  const float thin = std::min(1.0f, 3.0f / std::max(1.0f, deg));
+  P.wave_mult = 6.0f * thin * thin;
   P.mlp = (c.policy == VINE_POLICY_MLP && c.mlp) ? c.mlp->params : nullptr;
   P.trace = c.trace ? w.trace : nullptr;
   P.trace_top = w.counters + 3;
@@ -1448,7 +1582,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   VINE_CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(unsigned long long) * 4, stream));
   epoch_kernel<<<1, 1, 0, stream>>>(w.counters, nq);
   if (c.order_queries) VINE_TRY(order_queries(nq, d_budget, w.order, stream));
-  batch_kernel<<<r.slots, c.block_threads, smem, stream>>>(P);
+  kernel_for(c)<<<r.slots, c.block_threads, smem, stream>>>(P);
   VINE_CUDA_TRY(cudaGetLastError());
   if (paths) {
     paths->arena = w.path_arena;
@@ -1469,10 +1603,10 @@ int batch_slots(const vine_graph *g, const vine_config &c, int round_cap, int *s
   const size_t smem =
       batch_smem_bytes(c.table_log2, lock_log2_for(c.table_log2), c.sync_rounds ? round_cap : 0,
                        c.block_threads, c.split_staging);
-  VINE_CUDA_TRY(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   int per_sm = 0;
-  VINE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel,
+  VINE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_for(c),
                                                               c.block_threads, smem));
   if (per_sm < 1) return fail(VINE_ERR_INVALID, "batch kernel does not fit on an SM with this configuration");
   if (c.ctas_per_sm > 0) per_sm = std::min(per_sm, c.ctas_per_sm);

@@ -1,0 +1,1206 @@
+// Corridor of a query: the part of the graph that can still hold its answer.
+//
+// A query asks for the cheapest path with delay <= B.  For a multiplier
+// lambda = b / a the combined weight a * len + b * delay gives every feasible
+// path p (delay(p) <= B) the bound a * cost(p) + b * delay(p) <=
+// a * cost(p) + b * B, so with any feasible path of cost UB in hand
+//
+//     T = a * UB + b * B
+//
+// only vertices v with F(v) + H(v) <= T matter, F / H being the combined
+// distances source -> v and v -> sink (Lagrangian relaxation of the budget;
+// Handler and Zang, "A dual algorithm for the constrained shortest path
+// problem", Networks 10, 1980).  The same bound prunes single labels during
+// the search: a * d + b * delay + H(v) > T.  Equal cost never prunes, so the
+// (cost, delay) answer is untouched.
+//
+// Everything here is integer arithmetic: weights are integers below 2^24,
+// keys are kept below 2^31 by the choice of (a, b), and a key that would pass
+// that limit is larger than any T, hence prunable.
+//
+// Per query, by one CTA:
+//   1. bi_run: both ends grow at once in the combined weight until their
+//      radii cover the best meeting key (the two-sided Dijkstra test), every
+//      vertex touched from both ends offering a real path (its delay is
+//      carried beside the key) as UB; then on under F + H <= T.  That touches
+//      two half-radius balls instead of the full balls around the sink that
+//      two reverse searches over the graph need.
+//   2. the vertices with F + H <= T are copied out with the arcs between
+//      them, renumbered, into a small CSR of the worker (build_local); while
+//      it is large, a better multiplier shrinks it again the same way.
+//   3. on that CSR: delay and length distances to the sink and the
+//      multiplier that maximises the lower bound (a few one-sided passes).
+// The label search then runs on the small CSR with all three bounds.
+#pragma once
+
+#include "search.cuh"
+
+namespace vine {
+
+constexpr unsigned long long kUnset = ~0ull;
+constexpr uint32_t kKeyMax = 0x7ffffffeu;      // largest path key that is kept
+constexpr uint32_t kNoKey = 0xffffffffu;
+constexpr uint32_t kMemberTag = 0xfffffffeu;   // rf[v].y high word: v has a local id
+constexpr float kIntLimit = 16777216.0f;       // 2^24: budgets and costs handled here
+constexpr int kWaveQ = 2048;                   // queue entries kept in shared memory
+constexpr int kCorridorVertices = 1 << 16;     // largest local graph
+constexpr double kWideGap = 0.3;               // (T - meeting key) / meeting key worth another multiplier
+constexpr int kShrinkTo = 1024;                // local graphs up to this size are not shrunk further
+constexpr int kHubs = 32;                      // see WaveShared::hub
+constexpr int kHubDegree = 256;
+constexpr int kArcBatch = 4;                   // arcs of a vertex whose loads go out together
+
+// A worker's local graph: CSR in both directions and the original ids.
+struct LocalGraph {
+  DevGraph g;
+  int32_t *gid;
+};
+
+// Where a worker's corridor arrays lie (set up once per kernel).
+struct CorridorMem {
+  ulonglong2 *rf;      // [n] (F, H) of the global search, all ones when unused
+  uint32_t *touch[2];  // [n] vertices first reached by each side
+  uint32_t *ovf[2];    // queue entries past kWaveQ
+  uint32_t ovf_cap;
+  unsigned long long *far[2];
+  uint32_t far_cap;
+  LocalGraph loc[2];
+  int lv, la;          // capacity of a local graph: vertices, arcs
+  uint32_t *map;       // [lv] old local id -> new local id
+  unsigned long long *dist[4];  // [lv] distances on the local graph
+  VState *lvs;         // [lv] label search state
+};
+
+// Shared-memory state of the wave searches.  It lies over the bucket table,
+// which is not in use before the label search starts.
+struct __align__(16) WaveShared {
+  uint32_t q[2][kWaveQ];
+  unsigned long long mu;    // best meeting: (key, delay), pure mode (delay, length)
+  unsigned long long best;  // best feasible: (a * cost + b * B, delay), pure mode (cost, delay)
+  uint32_t nq[2], nfar[2], ntouch[2];
+  uint32_t far_min, hi, rdone;
+  uint32_t cnt;
+  int cur;
+  CorridorMem m;  // the worker's arrays
+  uint32_t hub[kHubs], nhub;  // vertices of this round whose arcs the block shares
+  int clipped, overflow, stop;
+  int scan[kScanScratch];
+};
+
+// 32-bit words of a worker's two local graphs and the renumbering.
+__host__ __device__ constexpr size_t corridor_ints(int lv, int la) {
+  return 2 * (2 * ((size_t)lv + 1) + 2 * (size_t)la + (size_t)lv) + (size_t)lv;
+}
+
+constexpr size_t kWaveBytes = (sizeof(WaveShared) + 15) & ~(size_t)15;
+
+// Shared memory of the bucket table and its locks, or of the wave state that
+// lies over them when that needs more.
+__host__ __device__ constexpr size_t table_region_bytes(int table_log2, int lock_log2) {
+  const size_t t = ((sizeof(int32_t) + sizeof(float2) + sizeof(uint32_t)) << table_log2) +
+                   (sizeof(int) << lock_log2);
+  return ((t > kWaveBytes ? t : kWaveBytes) + 15) & ~(size_t)15;
+}
+
+__device__ __forceinline__ ulonglong2 ld_pair(const ulonglong2 *p) {
+  ulonglong2 r;
+  asm volatile("ld.global.cg.v2.u64 {%0,%1}, [%2];" : "=l"(r.x), "=l"(r.y) : "l"(p) : "memory");
+  return r;
+}
+__device__ __forceinline__ uint32_t key_hi(unsigned long long x) { return (uint32_t)(x >> 32); }
+__device__ __forceinline__ uint32_t vol(const uint32_t &x) {
+  return *reinterpret_cast<const volatile uint32_t *>(&x);
+}
+__device__ __forceinline__ unsigned long long vol(const unsigned long long &x) {
+  return *reinterpret_cast<const volatile unsigned long long *>(&x);
+}
+
+// Exclusive prefix sum of one value per thread; *total gets the sum.  All
+// threads must call.
+__device__ __forceinline__ int block_scan_one(int x, int *scratch, int *total) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (blockDim.x + 31) >> 5;
+  int incl = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) scratch[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const int v = lane < nw ? scratch[lane] : 0;
+    int vi = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, vi, o);
+      if (lane >= o) vi += y;
+    }
+    if (lane < nw) scratch[lane] = vi - v;
+    if (lane == nw - 1) scratch[32] = vi;
+  }
+  __syncthreads();
+  const int r = scratch[warp] + incl - x;
+  *total = scratch[32];
+  __syncthreads();
+  return r;
+}
+
+__device__ __forceinline__ uint32_t wave_get(const WaveShared &W, const CorridorMem &M, int cur,
+                                             uint32_t i) {
+  return i < (uint32_t)kWaveQ ? W.q[cur][i] : __ldcg(&M.ovf[cur][i - kWaveQ]);
+}
+
+__device__ __forceinline__ void wave_put(WaveShared &W, const CorridorMem &M, int nxt, uint32_t pos,
+                                         uint32_t e) {
+  if (pos < (uint32_t)kWaveQ) W.q[nxt][pos] = e;
+  else if (pos - kWaveQ < M.ovf_cap) M.ovf[nxt][pos - kWaveQ] = e;
+  else W.overflow = 1;
+}
+
+__device__ __forceinline__ void wave_push(WaveShared &W, const CorridorMem &M, int nxt, uint32_t e) {
+  wave_put(W, M, nxt, warp_agg_inc(&W.nq[nxt]), e);
+}
+
+__device__ __forceinline__ void far_push(WaveShared &W, const CorridorMem &M, int fb, uint32_t key,
+                                         uint32_t e) {
+  const uint32_t pos = warp_agg_inc(&W.nfar[fb]);
+  if (pos >= M.far_cap) {
+    W.overflow = 1;
+    return;
+  }
+  M.far[fb][pos] = ((unsigned long long)key << 32) | e;
+  atomicMin(&W.far_min, key);
+}
+
+// Queues what a warp's relaxations improved: entry e[k] with key[k] goes to
+// the next round (bit k of near) or to the far pile (bit k of far); vertices
+// first reached (bit k of first) are listed for their side (bit 0 of e[k])
+// when `sides`.  One shared atomic per list and warp: the lanes' counts are
+// summed as four bytes of one word.  All lanes call.
+template <int K>
+__device__ __forceinline__ void wave_emit(WaveShared &W, const CorridorMem &M, int nxt, int fb,
+                                          const uint32_t (&e)[K], const uint32_t (&key)[K],
+                                          uint32_t near, uint32_t far, uint32_t first, bool sides) {
+  static_assert(32 * K < 256, "a warp's counts share bytes of one word");
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  uint32_t f1 = 0;
+  if (sides) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) f1 |= (first >> k & 1u & e[k]) << k;
+  }
+  const uint32_t f0 = sides ? first & ~f1 : 0u;
+  const uint32_t mine = (uint32_t)__popc(near) | (uint32_t)__popc(far) << 8 |
+                        (uint32_t)__popc(f0) << 16 | (uint32_t)__popc(f1) << 24;
+  if (!__any_sync(FULL, mine != 0u)) return;
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const uint32_t total = __shfl_sync(FULL, incl, 31), excl = incl - mine;
+  uint32_t base = 0;  // lane l < 4 reserves in list l
+  if (lane < 4) {
+    const uint32_t n = total >> (8 * lane) & 255u;
+    uint32_t *ctr = lane == 0 ? &W.nq[nxt] : lane == 1 ? &W.nfar[fb] : &W.ntouch[lane - 2];
+    if (n) base = atomicAdd(ctr, n);
+  }
+  uint32_t pn = __shfl_sync(FULL, base, 0) + (excl & 255u);
+  uint32_t pf = __shfl_sync(FULL, base, 1) + (excl >> 8 & 255u);
+  uint32_t p0 = __shfl_sync(FULL, base, 2) + (excl >> 16 & 255u);
+  uint32_t p1 = __shfl_sync(FULL, base, 3) + (excl >> 24);
+  uint32_t least = kNoKey;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (near >> k & 1u) wave_put(W, M, nxt, pn++, e[k]);
+    if (far >> k & 1u) {
+      if (pf < M.far_cap) M.far[fb][pf] = ((unsigned long long)key[k] << 32) | e[k];
+      else W.overflow = 1;
+      ++pf;
+      least = min(least, key[k]);
+    }
+    if (f0 >> k & 1u) M.touch[0][p0++] = e[k] >> 1;
+    if (f1 >> k & 1u) M.touch[1][p1++] = e[k] >> 1;
+  }
+  if (total >> 8 & 255u) {
+    least = __reduce_min_sync(FULL, least);
+    if (lane == 0) atomicMin(&W.far_min, least);
+  }
+}
+
+// ------------------------------------------------------- two-sided search
+
+// Weights of one search.  pure: key = delay, the second value is the length;
+// otherwise key = a * len + b * delay and the second value is the delay.
+struct Combo {
+  uint32_t a, b;
+  bool pure;
+  uint32_t B;
+};
+
+__device__ __forceinline__ uint32_t combo_limit(const WaveShared &W, const Combo &k) {
+  if (k.pure) return k.B;
+  const unsigned long long t = vol(W.best) >> 32;
+  return t < kKeyMax ? (uint32_t)t : kKeyMax;
+}
+
+// A vertex reached from both ends: (k, s) is a real source -> sink path.
+__device__ __forceinline__ void meet(WaveShared &W, const Combo &c, unsigned long long x,
+                                     unsigned long long y) {
+  const uint32_t k = key_hi(x) + key_hi(y);  // both at most kKeyMax
+  const unsigned long long s64 = (x & 0xffffffffull) + (y & 0xffffffffull);
+  const uint32_t s = s64 > 0xfffffffeull ? 0xfffffffeu : (uint32_t)s64;
+  const unsigned long long m = ((unsigned long long)k << 32) | s;
+  if (m < vol(W.mu)) atomicMin(&W.mu, m);
+  unsigned long long f = kUnset;
+  if (c.pure) {
+    if (k <= c.B) f = ((unsigned long long)s << 32) | k;
+  } else if (s <= c.B) {
+    const unsigned long long t = (unsigned long long)k + (unsigned long long)c.b * (c.B - s);
+    if (t <= kKeyMax) f = (t << 32) | s;
+  }
+  if (f < vol(W.best)) atomicMin(&W.best, f);
+}
+
+// Relaxes up to K arcs a lane: vertex u[k], reached with (nk[k], ns[k]) on
+// side side[k] (0 from the source, 1 from the sink) where bit k of `on` is set.  The
+// pair reads go out together, then the atomics.  All lanes call.
+template <int K>
+__device__ __forceinline__ void bi_relax(WaveShared &W, const CorridorMem &M, const Combo &c,
+                                         uint32_t on, const int (&u)[K],
+                                         const unsigned long long (&nk)[K], const uint32_t (&ns)[K],
+                                         uint32_t side, uint32_t hi, uint32_t rdone, uint32_t limit,
+                                         int nxt, int fb) {
+  ulonglong2 pu[K];
+  unsigned long long old[K];
+  uint32_t e[K], key[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (on >> k & 1u) {
+      if (nk[k] > limit) {
+        if (nk[k] > kKeyMax) W.clipped = 1;
+        on &= ~(1u << k);
+      } else {
+        pu[k] = ld_pair(&M.rf[u[k]]);
+      }
+    }
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (on >> k & 1u) {
+      const bool back = side >> k & 1u;
+      const unsigned long long cand = (nk[k] << 32) | ns[k];
+      const unsigned long long mine = back ? pu[k].y : pu[k].x, other = back ? pu[k].x : pu[k].y;
+      // What the other side still needs from u, at least: its own distance
+      // where that is final, else the radius up to which it is complete.
+      const uint32_t lb = min(key_hi(other), rdone);
+      if (cand < mine && nk[k] + (unsigned long long)lb <= limit)
+        old[k] = atomicMin(reinterpret_cast<unsigned long long *>(&M.rf[u[k]]) + (back ? 1 : 0), cand);
+      else on &= ~(1u << k);
+    }
+  uint32_t near = 0, far = 0, first = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    e[k] = ((uint32_t)u[k] << 1) | (side >> k & 1u);
+    key[k] = (uint32_t)nk[k];
+    if (on >> k & 1u) {
+      const unsigned long long cand = (nk[k] << 32) | ns[k];
+      if (cand < old[k]) {
+        const unsigned long long other = side >> k & 1u ? pu[k].x : pu[k].y;
+        if (other != kUnset) meet(W, c, cand, other);
+        if (old[k] == kUnset) first |= 1u << k;
+        if (key[k] < hi) near |= 1u << k;
+        else far |= 1u << k;
+      }
+    }
+  }
+  wave_emit<K>(W, M, nxt, fb, e, key, near, far, first, true);
+}
+
+// The second value of a path past an arc, kept below the all-ones word.
+__device__ __forceinline__ uint32_t add_second(uint32_t s, uint32_t x) {
+  return s > 0xfffffffeu - x ? 0xfffffffeu : s + x;
+}
+
+// Clears the pairs that the last search wrote.
+__device__ __forceinline__ void bi_reset(WaveShared &W, const CorridorMem &M) {
+  __syncthreads();
+  for (int s = 0; s < 2; ++s)
+    for (uint32_t i = threadIdx.x; i < W.ntouch[s]; i += blockDim.x)
+      __stcg(&M.rf[M.touch[s][i]], make_ulonglong2(kUnset, kUnset));
+  __syncthreads();
+  if (threadIdx.x == 0) W.ntouch[0] = W.ntouch[1] = 0;
+  __syncthreads();
+}
+
+// One warp's share of a round: entries [i0, i0 + take) of the current queue.
+__device__ __forceinline__ uint32_t bi_chunk(const DevGraph &g, WaveShared &W, const CorridorMem &M,
+                                             const Combo &c, int cur, int fb, uint32_t i0,
+                                             uint32_t take) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, nxt = cur ^ 1;
+  const uint32_t hi = vol(W.hi), rdone = vol(W.rdone), limit = combo_limit(W, c);
+  int beg = 0, deg = 0;
+  uint32_t key = 0, sec = 0, side = 0;
+  if ((uint32_t)lane < take) {
+    const uint32_t e = wave_get(W, M, cur, i0 + (uint32_t)lane);
+    const int v = (int)(e >> 1);
+    side = e & 1u;
+    const ulonglong2 pv = ld_pair(&M.rf[v]);
+    const int32_t *row = side ? g.rrow : g.row;
+    beg = row[v];
+    deg = row[v + 1] - beg;
+    const unsigned long long mine = side ? pv.y : pv.x, other = side ? pv.x : pv.y;
+    if (other != kUnset) meet(W, c, mine, other);
+    key = key_hi(mine);
+    sec = (uint32_t)mine;
+    if (deg > kHubDegree) {
+      const uint32_t h = atomicAdd(&W.nhub, 1u);
+      if (h < (uint32_t)kHubs) {
+        W.hub[h] = e;
+        deg = 0;
+      }
+    }
+  }
+  int u[kArcBatch];
+  unsigned long long nk[kArcBatch];
+  uint32_t ns[kArcBatch];
+  {
+    const int32_t *col = side ? g.rcol : g.col;
+    const float2 *wt = side ? g.rw : g.w;
+    float2 w[kArcBatch];
+    uint32_t on = 0;
+#pragma unroll
+    for (int k = 0; k < kArcBatch; ++k)
+      if (k < deg) {
+        u[k] = col[beg + k];
+        w[k] = wt[beg + k];
+        on |= 1u << k;
+      }
+#pragma unroll
+    for (int k = 0; k < kArcBatch; ++k)
+      if (k < deg) {
+        const uint32_t ln = (uint32_t)w[k].x, dl = (uint32_t)w[k].y;
+        nk[k] = key + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
+        ns[k] = add_second(sec, c.pure ? ln : dl);
+      }
+    bi_relax<kArcBatch>(W, M, c, on, u, nk, ns, side ? 0xfu : 0u, hi, rdone, limit, nxt, fb);
+  }
+  // arcs past the first few, dealt to the lanes of the warp
+  const int rem = max(0, deg - kArcBatch);
+  if (__any_sync(FULL, rem > 0)) {
+    int incl = rem;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int total = __shfl_sync(FULL, incl, 31), excl = incl - rem;
+    for (int e0 = 0; e0 < total; e0 += 32 * kArcBatch) {
+      uint32_t on = 0, sides = 0;
+#pragma unroll
+      for (int b = 0; b < kArcBatch; ++b) {
+        const int e = e0 + 32 * b + lane;
+        int k = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+          const int ex = __shfl_sync(FULL, excl, (k + step) & 31);
+          if (k + step < 32 && ex <= e) k += step;
+        }
+        const int obeg = __shfl_sync(FULL, beg, k), oex = __shfl_sync(FULL, excl, k);
+        const uint32_t oside = __shfl_sync(FULL, side, k);
+        const uint32_t okey = __shfl_sync(FULL, key, k), osec = __shfl_sync(FULL, sec, k);
+        if (e < total) {
+          const int j = obeg + kArcBatch + (e - oex);
+          u[b] = (oside ? g.rcol : g.col)[j];
+          const float2 w = (oside ? g.rw : g.w)[j];
+          const uint32_t ln = (uint32_t)w.x, dl = (uint32_t)w.y;
+          nk[b] = okey + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
+          ns[b] = add_second(osec, c.pure ? ln : dl);
+          on |= 1u << b;
+          sides |= oside << b;
+        }
+      }
+      bi_relax<kArcBatch>(W, M, c, on, u, nk, ns, sides, hi, rdone, limit, nxt, fb);
+    }
+  }
+  return (uint32_t)deg;
+}
+
+// The arcs of the round's hubs, dealt to the whole block.
+__device__ __forceinline__ uint32_t bi_hubs(const DevGraph &g, WaveShared &W, const CorridorMem &M,
+                                            const Combo &c, int cur, int fb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t hi = vol(W.hi), rdone = vol(W.rdone), limit = combo_limit(W, c);
+  const int nh = (int)min(W.nhub, (uint32_t)kHubs);
+  uint32_t relaxed = 0;
+  for (int h = 0; h < nh; ++h) {
+    const uint32_t e = W.hub[h], side = e & 1u;
+    const int v = (int)(e >> 1);
+    const ulonglong2 pv = ld_pair(&M.rf[v]);
+    const int32_t *row = side ? g.rrow : g.row, *col = side ? g.rcol : g.col;
+    const float2 *wt = side ? g.rw : g.w;
+    const unsigned long long mine = side ? pv.y : pv.x;
+    const uint32_t key = key_hi(mine), sec = (uint32_t)mine;
+    const int end = row[v + 1];
+    for (int j0 = row[v] + warp * 32 * kArcBatch; j0 < end; j0 += nw * 32 * kArcBatch) {
+      int u[kArcBatch];
+      unsigned long long nk[kArcBatch];
+      uint32_t ns[kArcBatch], on = 0;
+#pragma unroll
+      for (int k = 0; k < kArcBatch; ++k) {
+        const int j = j0 + 32 * k + lane;
+        if (j < end) {
+          u[k] = col[j];
+          const float2 w = wt[j];
+          const uint32_t ln = (uint32_t)w.x, dl = (uint32_t)w.y;
+          nk[k] = key + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
+          ns[k] = add_second(sec, c.pure ? ln : dl);
+          on |= 1u << k;
+        }
+      }
+      relaxed += (uint32_t)__popc(on);
+      bi_relax<kArcBatch>(W, M, c, on, u, nk, ns, side ? 0xfu : 0u, hi, rdone, limit, cur ^ 1, fb);
+    }
+  }
+  return relaxed;
+}
+
+// Runs rounds until the queue is empty (all threads).  Returns arcs relaxed
+// by the calling thread.
+//
+// Bound by latency: a round is a chain of dependent reads (queue, row and
+// pair, arcs, their pairs), one atomic and the push.  A lane takes a whole
+// vertex of a road graph (at most kArcBatch arcs, the loads and then the
+// atomics of all of them in flight together); arcs past that are dealt to the
+// lanes of the warp and those of hubs to the block, so hubs do not serialise.
+// While a round fits one warp, warp 0 runs on alone without block barriers.
+__device__ __forceinline__ uint32_t bi_rounds(QueryState &st, const DevGraph &g, WaveShared &W,
+                                              const CorridorMem &M, const Combo &c, int *pcur,
+                                              int fb) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  int cur = *pcur;
+  uint32_t relaxed = 0;
+  for (;;) {
+    __syncthreads();
+    const uint32_t nc = min(W.nq[cur], (uint32_t)kWaveQ + M.ovf_cap);
+    if (nc == 0 || W.stop) break;  // W.stop changes only between the barriers below
+    if (nc <= 32u) __syncthreads();  // every warp has read the count
+    const bool narrow = nc <= 32u;
+    const uint32_t take = narrow ? 32u : min(32u, (nc + (uint32_t)nw - 1u) / (uint32_t)nw);
+    uint32_t n = nc;
+    if (!narrow || warp == 0) {
+      for (;;) {
+        for (uint32_t base = (uint32_t)warp * take; base < n; base += (uint32_t)nw * take)
+          relaxed += bi_chunk(g, W, M, c, cur, fb, base, min(take, n - base));
+        if (!narrow) break;
+        __syncwarp();
+        if (lane == 0) {
+          W.nq[cur] = 0;
+          st.n_rounds++;
+        }
+        cur ^= 1;
+        __syncwarp();
+        n = vol(W.nq[cur]);
+        if (n == 0 || n > 32u || vol(W.nhub) != 0) break;
+      }
+    }
+    if (!narrow) __syncthreads();
+    if (tid == 0) {
+      if (!narrow) {
+        W.nq[cur] = 0;
+        cur ^= 1;
+        st.n_rounds++;
+      }
+      W.cur = cur;
+      if (W.overflow || st.abort) W.stop = 1;
+    }
+    __syncthreads();
+    cur = W.cur;
+    if (W.nhub != 0) {
+      relaxed += bi_hubs(g, W, M, c, cur ^ 1, fb);
+      __syncthreads();
+      if (tid == 0) W.nhub = 0;
+    }
+  }
+  *pcur = cur;
+  return relaxed;
+}
+
+// Starts a two-sided search: both ends queued, `best0` what W.best starts from.
+__device__ __forceinline__ void bi_start(WaveShared &W, const CorridorMem &M, int s, int t,
+                                         unsigned long long best0, uint32_t delta) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    W.mu = kUnset;
+    W.best = best0;
+    W.nq[0] = 2;
+    W.nq[1] = 0;
+    W.nhub = 0;
+    W.nfar[0] = W.nfar[1] = 0;
+    W.far_min = kNoKey;
+    W.hi = delta;
+    W.rdone = 0;
+    W.clipped = 0;
+    W.stop = 0;
+    W.ntouch[0] = W.ntouch[1] = 1;
+    M.touch[0][0] = (uint32_t)s;
+    M.touch[1][0] = (uint32_t)t;
+    __stcg(&M.rf[s], make_ulonglong2(0ull, kUnset));
+    __stcg(&M.rf[t], make_ulonglong2(kUnset, 0ull));
+    W.q[0][0] = (uint32_t)s << 1;
+    W.q[0][1] = ((uint32_t)t << 1) | 1u;
+  }
+}
+
+// Grows both sides, bucket after bucket of width `delta`: to_meeting: until
+// the radii cover the best meeting key (W.mu is then the combined distance);
+// else until nothing is left below the limit, when every vertex with
+// F + H <= T has both its distances: on a shortest way to such a vertex no
+// vertex is pruned, since what it is charged for the other side, its distance
+// there or the radius of that side, is never more than the truth.
+// *pcur / *pfb: queue and far pile in use.
+__device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, const DevGraph &g,
+                                        Combo c, bool to_meeting, uint32_t delta, int *pcur,
+                                        int *pfb) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  const CorridorMem &M = W.m;
+  int cur = *pcur, fb = *pfb;
+  uint32_t relaxed = 0;
+  for (;;) {
+    relaxed += bi_rounds(st, g, W, M, c, &cur, fb);
+    // nothing unsettled lies below far_min on either side
+    const uint32_t fm = W.far_min, lo = max(W.hi, fm);
+    const bool stop = fm == kNoKey || W.stop || (to_meeting && 2ull * lo >= (vol(W.mu) >> 32));
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      W.rdone = fm == kNoKey ? kKeyMax : lo;
+      if (!stop) {
+        if (over_time(P, st)) W.stop = 1;
+        W.hi = min(lo, kKeyMax + 1u - delta) + delta;
+        W.far_min = kNoKey;
+        W.nfar[fb ^ 1] = 0;
+      }
+    }
+    __syncthreads();
+    if (stop) break;
+    // far entries below the new upper key join the queue; one that a shorter
+    // way overtook or that the bound rules out is dropped
+    const uint32_t fn = min(W.nfar[fb], M.far_cap), hi = W.hi, limit = combo_limit(W, c), rdone = W.rdone;
+    for (uint32_t i = threadIdx.x; i < fn; i += blockDim.x) {
+      const unsigned long long x = __ldcg(&M.far[fb][i]);
+      const uint32_t key = key_hi(x), e = (uint32_t)x;
+      if (key < hi) {
+        const ulonglong2 pv = ld_pair(&M.rf[e >> 1]);
+        const unsigned long long mine = e & 1u ? pv.y : pv.x, other = e & 1u ? pv.x : pv.y;
+        if (key_hi(mine) == key && key + (unsigned long long)min(key_hi(other), rdone) <= limit)
+          wave_push(W, M, cur, e);
+      } else if (key <= limit) {
+        far_push(W, M, fb ^ 1, key, e);
+      }
+    }
+    fb ^= 1;
+  }
+  *pcur = cur;
+  *pfb = fb;
+  return relaxed;
+}
+
+// ---------------------------------------------------------------- local CSR
+
+// One direction of a renumbered CSR: vertex i is old_of(i) of the old graph,
+// arcs to vertices without a new id (new_of < 0) are left out.  False when
+// the arcs do not fit (all threads agree).
+template <typename OldOf, typename NewOf>
+__device__ __forceinline__ bool build_csr(WaveShared &W, const int32_t *orow, const int32_t *ocol,
+                                          const float2 *ow, int ne, OldOf old_of, NewOf new_of,
+                                          int32_t *row, int32_t *col, float2 *w, int cap) {
+  constexpr int kKeep = 6;  // arcs of a vertex whose new ids stay in registers
+  const unsigned FULL = 0xffffffffu;
+  const int G = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+  int run = 0;
+  for (int base = 0; base < ne; base += G) {
+    const int i = base + tid;
+    int beg = 0, deg = 0, cnt = 0;
+    int nid[kKeep];
+    if (i < ne) {
+      const int v = old_of(i);
+      beg = orow[v];
+      deg = orow[v + 1] - beg;
+    }
+    const bool wide = deg > kKeep;
+    if (!wide) {
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k) nid[k] = k < deg ? ocol[beg + k] : -1;
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k) nid[k] = k < deg ? new_of(nid[k]) : -1;
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k) cnt += nid[k] >= 0;
+    }
+    const unsigned wm = __ballot_sync(FULL, wide);
+    for (unsigned m = wm; m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const int b = __shfl_sync(FULL, beg, l), e = b + __shfl_sync(FULL, deg, l);
+      int n = 0;
+      for (int j = b + lane; j < e; j += 32) n += new_of(ocol[j]) >= 0;
+      n = __reduce_add_sync(FULL, n);
+      if (lane == l) cnt = n;
+    }
+    int total;
+    int at = run + block_scan_one(cnt, W.scan, &total);
+    run += total;
+    if (run > cap) return false;
+    if (i < ne) row[i] = at;
+    if (!wide) {
+#pragma unroll
+      for (int k = 0; k < kKeep; ++k)
+        if (nid[k] >= 0) {
+          col[at] = nid[k];
+          w[at] = ow[beg + k];
+          ++at;
+        }
+    }
+    for (unsigned m = wm; m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const int b = __shfl_sync(FULL, beg, l), e = b + __shfl_sync(FULL, deg, l);
+      int to = __shfl_sync(FULL, at, l);
+      for (int j0 = b; j0 < e; j0 += 32) {
+        const int j = j0 + lane;
+        const int id = j < e ? new_of(ocol[j]) : -1;
+        const unsigned hit = __ballot_sync(FULL, id >= 0);
+        if (id >= 0) {
+          const int p = to + __popc(hit & ((1u << lane) - 1u));
+          col[p] = id;
+          w[p] = ow[j];
+        }
+        to += __popc(hit);
+      }
+    }
+  }
+  if (tid == 0) row[ne] = run;
+  __syncthreads();
+  return true;
+}
+
+// Copies the corridor of the finished two-sided search on graph g into L
+// (og: original ids of g's vertices, null for the whole graph).  The new ids
+// of g's vertices stay in rf until the next reset.  Returns the vertex count;
+// -1 (nothing copied) when it does not fit or exceeds `most`.
+__device__ __noinline__ int build_local(const DevGraph &g, const int32_t *og, Combo c, LocalGraph &L,
+                                        int most) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  const CorridorMem &M = W.m;
+  const int G = blockDim.x, tid = threadIdx.x;
+  __syncthreads();
+  if (tid == 0) W.cnt = 0;
+  __syncthreads();
+  const uint32_t nt = W.ntouch[0], limit = combo_limit(W, c), cap = (uint32_t)min(M.lv, most);
+  for (uint32_t i = tid; i < nt; i += G) {
+    const uint32_t v = __ldcg(&M.touch[0][i]);
+    const ulonglong2 p = ld_pair(&M.rf[v]);
+    if (p.y != kUnset && (unsigned long long)key_hi(p.x) + key_hi(p.y) <= limit) {
+      const uint32_t id = warp_agg_inc(&W.cnt);
+      if (id < cap) {
+        M.map[id] = v;
+        L.gid[id] = og ? og[v] : (int32_t)v;
+        __stcg(reinterpret_cast<unsigned long long *>(&M.rf[v]) + 1,
+               ((unsigned long long)kMemberTag << 32) | id);
+      }
+    }
+  }
+  __syncthreads();
+  if (W.cnt > cap) return -1;
+  const int ne = (int)W.cnt;
+  const uint32_t *map = M.map;
+  auto old_of = [map](int i) { return (int)map[i]; };
+  const ulonglong2 *rf = M.rf;
+  auto new_of = [rf](int v) {
+    const unsigned long long h = __ldcg(reinterpret_cast<const unsigned long long *>(&rf[v]) + 1);
+    return key_hi(h) == kMemberTag ? (int)(uint32_t)h : -1;
+  };
+  if (!build_csr(W, g.row, g.col, g.w, ne, old_of, new_of, const_cast<int32_t *>(L.g.row),
+                 const_cast<int32_t *>(L.g.col), const_cast<float2 *>(L.g.w), M.la))
+    return -1;
+  if (!build_csr(W, g.rrow, g.rcol, g.rw, ne, old_of, new_of, const_cast<int32_t *>(L.g.rrow),
+                 const_cast<int32_t *>(L.g.rcol), const_cast<float2 *>(L.g.rw), M.la))
+    return -1;
+  if (tid == 0) L.g.n = ne;
+  __syncthreads();
+  return ne;
+}
+
+// Distances of a local pass: in shared memory (behind the wave state) where
+// the graph fits, else in the worker's global array.
+template <bool kShared>
+struct DistArray {
+  unsigned long long *p;
+  __device__ __forceinline__ unsigned long long get(int i) const {
+    if (kShared) return *reinterpret_cast<const volatile unsigned long long *>(p + i);
+    return __ldcg(p + i);
+  }
+  __device__ __forceinline__ void set(int i, unsigned long long x) const {
+    if (kShared) *reinterpret_cast<volatile unsigned long long *>(p + i) = x;
+    else __stcg(p + i, x);
+  }
+};
+
+// What a local pass computes: distances from `root` along (row, col, w) under
+// c; keys above `limit` are dropped.
+struct PassArgs {
+  const int32_t *row, *col;
+  const float2 *w;
+  int n, root;
+  uint32_t limit;
+  uint32_t delta;
+};
+
+template <bool kShared>
+__device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const CorridorMem &M, const PassArgs &A,
+                                                const Combo &c, const DistArray<kShared> &D, int cur,
+                                                int fb, uint32_t i0, uint32_t take) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, nxt = cur ^ 1;
+  const uint32_t hi = vol(W.hi), limit = A.limit;
+  int beg = 0, deg = 0;
+  uint32_t key = 0, sec = 0;
+  if ((uint32_t)lane < take) {
+    const int v = (int)wave_get(W, M, cur, i0 + (uint32_t)lane);
+    const unsigned long long x = D.get(v);
+    beg = A.row[v];
+    deg = A.row[v + 1] - beg;
+    key = key_hi(x);
+    sec = (uint32_t)x;
+  }
+  auto relax = [&](uint32_t on, const int (&u)[kArcBatch], const float2 (&w)[kArcBatch],
+                   const uint32_t (&k0)[kArcBatch], const uint32_t (&s0)[kArcBatch]) {
+    unsigned long long cand[kArcBatch], old[kArcBatch];
+    uint32_t e[kArcBatch], nkey[kArcBatch], near = 0, far = 0;
+#pragma unroll
+    for (int k = 0; k < kArcBatch; ++k) {
+      cand[k] = 0;
+      if (on >> k & 1u) {
+        const uint32_t ln = (uint32_t)w[k].x, dl = (uint32_t)w[k].y;
+        const unsigned long long nk =
+            k0[k] + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
+        if (nk > limit) {
+          on &= ~(1u << k);
+        } else {
+          cand[k] = (nk << 32) | add_second(s0[k], c.pure ? ln : dl);
+          if (cand[k] >= D.get(u[k])) on &= ~(1u << k);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kArcBatch; ++k)
+      if (on >> k & 1u) old[k] = atomicMin(&D.p[u[k]], cand[k]);
+#pragma unroll
+    for (int k = 0; k < kArcBatch; ++k) {
+      e[k] = (uint32_t)u[k];
+      nkey[k] = key_hi(cand[k]);
+      if ((on >> k & 1u) && cand[k] < old[k]) {
+        if (nkey[k] < hi) near |= 1u << k;
+        else far |= 1u << k;
+      }
+    }
+    wave_emit<kArcBatch>(W, M, nxt, fb, e, nkey, near, far, 0u, false);
+  };
+  int u[kArcBatch];
+  float2 w[kArcBatch];
+  uint32_t k0[kArcBatch], s0[kArcBatch], on = 0;
+#pragma unroll
+  for (int k = 0; k < kArcBatch; ++k) {
+    k0[k] = key;
+    s0[k] = sec;
+    if (k < deg) {
+      u[k] = A.col[beg + k];
+      w[k] = A.w[beg + k];
+      on |= 1u << k;
+    }
+  }
+  relax(on, u, w, k0, s0);
+  unsigned wide = __ballot_sync(FULL, deg > kArcBatch);
+  for (; wide; wide &= wide - 1) {  // the further arcs of one vertex after the other
+    const int l = __ffs(wide) - 1;
+    const int b0 = __shfl_sync(FULL, beg, l) + kArcBatch, e0 = b0 - kArcBatch + __shfl_sync(FULL, deg, l);
+    const uint32_t ok = __shfl_sync(FULL, key, l), os = __shfl_sync(FULL, sec, l);
+    for (int j0 = b0; j0 < e0; j0 += 32 * kArcBatch) {
+      on = 0;
+#pragma unroll
+      for (int k = 0; k < kArcBatch; ++k) {
+        const int j = j0 + 32 * k + lane;
+        k0[k] = ok;
+        s0[k] = os;
+        if (j < e0) {
+          u[k] = A.col[j];
+          w[k] = A.w[j];
+          on |= 1u << k;
+        }
+      }
+      relax(on, u, w, k0, s0);
+    }
+  }
+  return (uint32_t)deg;
+}
+
+// Runs a local pass with the whole block; `out` receives the distances.
+// Latency-bound like bi_rounds; a corridor is long and narrow, so most rounds
+// fit one warp and run without block barriers, on shared-memory distances.
+template <bool kShared>
+__device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState &st, PassArgs A,
+                                               Combo c, unsigned long long *out) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  const CorridorMem &M = W.m;
+  const int G = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = G >> 5;
+  DistArray<kShared> D;
+  D.p = kShared ? reinterpret_cast<unsigned long long *>(smem + kWaveBytes) : out;
+  __syncthreads();
+  for (int i = tid; i < A.n; i += G) D.set(i, i == A.root ? 0ull : kUnset);
+  if (tid == 0) {
+    W.nq[0] = 1;
+    W.nq[1] = 0;
+    W.nfar[0] = W.nfar[1] = 0;
+    W.far_min = kNoKey;
+    W.hi = A.delta;
+    W.stop = 0;
+    W.mu = kUnset;
+    W.q[0][0] = (uint32_t)A.root;
+  }
+  uint32_t relaxed = 0;
+  int cur = 0, fb = 0;
+  for (;;) {
+    __syncthreads();
+    const uint32_t nc = min(W.nq[cur], (uint32_t)kWaveQ + M.ovf_cap);
+    if (W.stop) break;  // changes only between the barriers below
+    if (nc == 0) {
+      const uint32_t fm = W.far_min, fn = min(W.nfar[fb], M.far_cap);
+      if (fm == kNoKey) break;
+      __syncthreads();
+      if (tid == 0) {
+        over_time(P, st);
+        if (W.overflow || st.abort) W.stop = 1;
+        W.hi = min(max(W.hi, fm), kKeyMax + 1u - A.delta) + A.delta;
+        W.far_min = kNoKey;
+        W.nfar[fb ^ 1] = 0;
+      }
+      __syncthreads();
+      const uint32_t hi = W.hi;
+      for (uint32_t i = tid; i < fn; i += G) {
+        const unsigned long long x = __ldcg(&M.far[fb][i]);
+        if (key_hi(x) < hi) {
+          if (key_hi(D.get((int)(uint32_t)x)) == key_hi(x)) wave_push(W, M, cur, (uint32_t)x);
+        } else {
+          far_push(W, M, fb ^ 1, key_hi(x), (uint32_t)x);
+        }
+      }
+      fb ^= 1;
+      continue;
+    }
+    if (nc <= 32u) {
+      __syncthreads();  // every warp has read the count
+      if (warp == 0) {
+        uint32_t n = nc;
+        do {
+          relaxed += local_chunk<kShared>(W, M, A, c, D, cur, fb, 0, n);
+          __syncwarp();
+          if (lane == 0) {
+            W.nq[cur] = 0;
+            st.n_rounds++;
+          }
+          cur ^= 1;
+          __syncwarp();
+          n = vol(W.nq[cur]);
+        } while (n != 0 && n <= 32u);
+        if (lane == 0) W.cur = cur;
+      }
+    } else {
+      const uint32_t take = min(32u, (nc + (uint32_t)nw - 1u) / (uint32_t)nw);
+      for (uint32_t base = (uint32_t)warp * take; base < nc; base += (uint32_t)nw * take)
+        relaxed += local_chunk<kShared>(W, M, A, c, D, cur, fb, base, min(take, nc - base));
+      __syncthreads();
+      if (tid == 0) {
+        W.nq[cur] = 0;
+        W.cur = cur ^ 1;
+        st.n_rounds++;
+      }
+    }
+    if (tid == 0 && (W.overflow || st.abort)) W.stop = 1;
+    __syncthreads();
+    cur = W.cur;
+  }
+  __syncthreads();
+  if (kShared) {
+    for (int i = tid; i < A.n; i += G) __stcg(&out[i], D.get(i));
+    __syncthreads();
+  }
+  return relaxed;
+}
+
+__device__ __forceinline__ uint32_t local_pass(const SearchParams &P, QueryState &st, const PassArgs &A,
+                                               const Combo &c, unsigned long long *out) {
+  const int cap = (int)((table_region_bytes(P.table_log2, P.lock_log2) - kWaveBytes) / sizeof(unsigned long long));
+  return A.n <= cap ? local_pass_in<true>(P, st, A, c, out) : local_pass_in<false>(P, st, A, c, out);
+}
+
+// ----------------------------------------------------------------- multipliers
+
+// (a, b) with b / a close to lambda and a * ub + b * B <= kKeyMax.  False when
+// one of them would vanish.
+__device__ inline bool pick_combo(double lambda, double ub, double B, Combo *c) {
+  const double s = (double)(kKeyMax - 1u) / fmax(1.0, ub + lambda * B);
+  const double a = floor(fmin(s, 1073741824.0)), b = floor(fmin(lambda * s, 1073741824.0));
+  if (!(a >= 1.0) || !(b >= 1.0)) return false;
+  c->a = (uint32_t)a;
+  c->b = (uint32_t)b;
+  c->pure = false;
+  return true;
+}
+
+// Bucket width of a wave in key units: a few mean arcs.
+__device__ __forceinline__ uint32_t combo_delta(const SearchParams &P, const Combo &c, float mult) {
+  const double d = (double)mult * ((double)c.a * P.mean_len + (double)c.b * P.mean_delay);
+  return (uint32_t)fmin(fmax(d, 1.0), 536870912.0);
+}
+
+enum CorridorResult { kCorridorNone = 0, kCorridorReady = 1, kCorridorInfeasible = 2 };
+
+// What is known about a query's paths while its corridor is built.  (len,
+// delay) pairs of real paths: p1 the best combined path that is too slow, p2
+// the best combined path within the budget; ub the smallest cost of any path
+// within the budget.  < 0: none yet.
+struct Duals {
+  double ub, ub_delay, len1, del1, len2, del2;
+
+  __device__ void feasible(double len, double del) {
+    if (ub < 0.0 || len < ub) {
+      ub = len;
+      ub_delay = del;
+    }
+  }
+  // The best path under (c.a, c.b), as (key, delay).
+  __device__ void optimum(const Combo &c, unsigned long long x) {
+    const double del = (double)(uint32_t)x;
+    const double len = floor(((double)(x >> 32) - (double)c.b * del) / (double)c.a);
+    if (del <= (double)c.B) {
+      feasible(len, del);
+      len2 = len;
+      del2 = del;
+    } else {
+      len1 = len;
+      del1 = del;
+    }
+  }
+  // Slope between the best paths on both sides of the budget (Handler and
+  // Zang's next multiplier), < 0 while one is missing.
+  __device__ double slope() const {
+    if (len1 < 0.0) return -1.0;
+    const double l2 = len2 >= 0.0 ? len2 : ub, d2 = len2 >= 0.0 ? del2 : ub_delay;
+    if (l2 < 0.0 || !(del1 > d2) || !(l2 > len1)) return -1.0;
+    return (l2 - len1) / (del1 - d2);
+  }
+  __device__ uint32_t T(const Combo &c) const {
+    return (uint32_t)((unsigned long long)c.a * (unsigned long long)ub + (unsigned long long)c.b * c.B);
+  }
+};
+
+// Builds the query's corridor (all threads; every thread computes the same
+// multipliers).  kCorridorReady: local graph *which holds it, M.lvs is
+// initialised, st.src / st.dst are local ids, st.inc_key carries the cost
+// bound and st.lam_* the multiplier; kCorridorInfeasible: no path within the
+// budget; kCorridorNone: not handled here (costs from 2^24 on, or a corridor
+// past the local capacity).
+__device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &st, int *which) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  CorridorMem &M = W.m;
+  const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, G = blockDim.x;
+  const uint32_t B = (uint32_t)floorf(st.budget);
+  const int s = st.src, t = st.dst;
+  const double unit = fmax((double)P.mean_len, 1e-3) / fmax((double)P.mean_delay, 1e-3);
+  if (tid == 0) {
+    W.overflow = 0;
+    W.stop = 0;
+    W.ntouch[0] = W.ntouch[1] = 0;
+  }
+  uint32_t relaxed = 0;
+  Duals k{-1.0, 0.0, -1.0, 0.0, -1.0, 0.0};
+  double lambda = unit;  // a unit of delay weighs like a unit of length
+  int result = kCorridorNone, ne = -1, cl = -1, ls = s, lt = t;  // cl: graph searched (-1: the whole one)
+  bool pure = false;
+  Combo c;
+  c.B = B;
+  for (int attempt = 0;; ++attempt) {
+    // before a path is known its cost is taken to be at most 16 times what
+    // the budget suggests; where that fails the pure delay search answers
+    const double guess = k.ub >= 0.0 ? k.ub : fmin((double)kIntLimit, 16.0 * (B + P.mean_delay) * unit);
+    if (!pure && !pick_combo(lambda, guess, (double)B, &c)) {
+      if (k.ub >= 0.0) break;
+      pure = true;
+    }
+    if (pure) {
+      c.a = 0;
+      c.b = 1;
+    }
+    c.pure = pure;
+    unsigned long long best0 = kUnset;
+    if (k.ub >= 0.0)
+      best0 = ((unsigned long long)(pure ? (uint32_t)k.ub : k.T(c)) << 32) | (uint32_t)k.ub_delay;
+    const DevGraph &g = cl < 0 ? P.g : M.loc[cl].g;
+    const uint32_t delta = combo_delta(P, c, P.wave_mult);
+    int cur = 0, fb = 0;
+    bi_start(W, M, ls, lt, best0, delta);
+    relaxed += bi_run(P, st, g, c, true, delta, &cur, &fb);
+    if (W.stop) break;
+    const unsigned long long mu = W.mu, best = W.best;
+    if (best != kUnset) {
+      const double cost = pure ? (double)(best >> 32)
+                               : floor((double)((best >> 32) - (unsigned long long)c.b * B) / (double)c.a);
+      k.feasible(cost, (double)(uint32_t)best);
+    }
+    if (mu != kUnset && !pure) k.optimum(c, mu);
+    if (k.ub < 0.0) {
+      // nothing feasible seen: unreachable, or weigh the delay more, at last alone
+      if (pure || (mu == kUnset && !W.clipped)) {
+        result = kCorridorInfeasible;
+        break;
+      }
+      bi_reset(W, M);
+      if (attempt == 0 && mu != kUnset) lambda *= 4.0;
+      else pure = true;
+      continue;
+    }
+    if (k.ub >= (double)kIntLimit) break;
+    // The next multiplier to try: the slope once both sides of the budget
+    // are known, else less weight on the delay.
+    double next = k.slope();
+    if (next < 0.0) next = (pure ? unit : lambda) * 0.2;
+    const bool settled = !pure && fabs(next - lambda) <= 0.1 * lambda;
+    // A wide gap between T and the meeting key means a poor multiplier:
+    // another search now costs less than completing this one.
+    const double gap = pure ? 1.0 : ((double)k.T(c) - (double)(mu >> 32)) / fmax(1.0, (double)(mu >> 32));
+    if (attempt >= 4 || settled || cl >= 0 || !(gap > kWideGap)) {
+      __syncthreads();
+      relaxed += bi_run(P, st, g, c, false, delta, &cur, &fb);
+      if (W.stop) break;
+      const unsigned long long b2 = W.best;
+      k.feasible(pure ? (double)(b2 >> 32)
+                      : floor((double)((b2 >> 32) - (unsigned long long)c.b * B) / (double)c.a),
+                 (double)(uint32_t)b2);
+      const int to = cl < 0 ? 0 : cl ^ 1;
+      const int n2 = build_local(g, cl < 0 ? nullptr : M.loc[cl].gid, c, M.loc[to],
+                                 cl < 0 ? M.lv : ne - ne / 4);
+      if (n2 >= 0) {
+        ls = (int)(uint32_t)__ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[ls]) + 1);
+        lt = (int)(uint32_t)__ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[lt]) + 1);
+        cl = to;
+        ne = n2;
+      }
+      if (settled || attempt >= 6 || (ne >= 0 && ne <= kShrinkTo)) break;
+    }
+    bi_reset(W, M);
+    lambda = next;
+    pure = false;
+  }
+  const bool stopped = W.stop != 0;
+  bi_reset(W, M);
+  if (stopped) ne = -1;
+
+  unsigned long long *D0 = M.dist[0], *D1 = M.dist[1], *Hbest = M.dist[2], *Hcur = M.dist[3];
+  Combo use;
+  use.a = use.b = 0;
+  if (ne >= 0) {
+    // ---- bounds on the corridor: delay, length, best multiplier
+    const DevGraph &g = M.loc[cl].g;
+    const bool wide = ne > 4096;  // one bucket on small graphs
+    const uint32_t one = 0x40000000u;
+    Combo cd{0u, 1u, true, B}, cl_{1u, 0u, false, B};
+    PassArgs A{g.rrow, g.rcol, g.rw, ne, lt, B, wide ? combo_delta(P, cd, P.wave_mult) : one};
+    relaxed += local_pass(P, st, A, cd, D0);
+    const unsigned long long xd = __ldcg(&D0[ls]);  // the fastest path
+    if (xd != kUnset) {
+      k.feasible((double)(uint32_t)xd, (double)(xd >> 32));
+      if (k.len2 < 0.0) {
+        k.len2 = (double)(uint32_t)xd;
+        k.del2 = (double)(xd >> 32);
+      }
+    }
+    A.limit = (uint32_t)k.ub;
+    A.delta = wide ? combo_delta(P, cl_, P.wave_mult) : one;
+    relaxed += local_pass(P, st, A, cl_, D1);
+    const unsigned long long xl = __ldcg(&D1[ls]);  // the shortest path
+    if (xl != kUnset) {
+      const double l0 = (double)(xl >> 32), d0 = (double)(uint32_t)xl;
+      if (d0 <= (double)B) {
+        k.feasible(l0, d0);  // the answer's cost
+      } else {
+        if (k.len1 < 0.0) {
+          k.len1 = l0;
+          k.del1 = d0;
+        }
+        double lb = -1.0;
+        for (int it = 0; it < 8 && !st.abort && !W.overflow; ++it) {
+          const double next = k.slope();
+          if (next < 0.0 || !pick_combo(next, k.ub, (double)B, &c)) break;
+          const double l2 = k.len2, d2 = k.del2, l1 = k.len1, d1 = k.del1;
+          A.limit = k.T(c);
+          A.delta = wide ? combo_delta(P, c, P.wave_mult) : one;
+          relaxed += local_pass(P, st, A, c, Hcur);
+          const unsigned long long x = __ldcg(&Hcur[ls]);
+          if (x == kUnset) break;
+          const double low = ((double)(x >> 32) - (double)c.b * (double)B) / (double)c.a;
+          if (use.a == 0 || low > lb) {
+            lb = low;
+            use = c;
+            unsigned long long *h = Hbest;
+            Hbest = Hcur;
+            Hcur = h;
+          }
+          k.optimum(c, x);
+          // done when no path lies below the line through the two points, or
+          // when the bound meets the cost
+          const double line = fmin((double)c.a * l1 + (double)c.b * d1, (double)c.a * l2 + (double)c.b * d2);
+          if ((double)(x >> 32) >= line || ceil(low) >= k.ub) break;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  relaxed = __reduce_add_sync(FULL, relaxed);
+  if ((tid & 31) == 0)
+    atomicAdd(reinterpret_cast<unsigned long long *>(&st.n_relaxed), (unsigned long long)relaxed);
+  if (W.overflow && tid == 0 && !st.abort) fail_query(st, VINE_ERR_CAPACITY, kSiteBand);
+  if (ne >= 0) {
+    for (int i = tid; i < ne; i += G) {
+      const unsigned long long hd = __ldcg(&D0[i]), hl = __ldcg(&D1[i]);
+      const uint32_t hm = use.a ? key_hi(__ldcg(&Hbest[i])) : 0u;
+      const bool in = hd != kUnset && hl != kUnset && hm != kNoKey;
+      VState v;
+      v.epoch = st.epoch;
+      v.sdel = INFINITY;
+      v.e_del = hm;
+      v.hdel = in ? (float)key_hi(hd) : 0.0f;
+      v.bep = 0;
+      v.bmin = 0.0f;
+      v.hlen = in ? (float)key_hi(hl) : INFINITY;
+      v.bhead = kNone;
+      M.lvs[i] = v;
+    }
+    if (tid == 0) {
+      st.src = ls;
+      st.dst = lt;
+      st.lam_a = use.a;
+      st.lam_b = use.b;
+      st.lam_bB = use.b * B;
+      st.inc_key = pack_key((float)k.ub, INFINITY);
+    }
+    *which = cl;
+    result = kCorridorReady;
+  }
+  __syncthreads();
+  return result;
+}
+
+}  // namespace vine

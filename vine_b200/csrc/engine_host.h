@@ -46,6 +46,15 @@ struct BatchWorkspace {
   int64_t q_cap = 0;
   float *trace = nullptr;
   int64_t trace_cap = 0;
+  // corridors (calls with bounds): two-sided distances, touched vertices and
+  // the local graphs of every worker
+  ulonglong2 *rf = nullptr;
+  uint32_t *touch = nullptr;
+  int32_t *lint = nullptr;
+  float2 *lw = nullptr;
+  unsigned long long *ldist = nullptr;
+  VState *lvs = nullptr;
+  int lv = 0, la = 0;
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape
   cudaGraphExec_t graph_exec = nullptr;

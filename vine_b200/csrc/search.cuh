@@ -92,6 +92,16 @@ struct SearchParams {
   int split_staging;                 // bucket opening reads tiles through bulk copies
   long long wait_limit;              // polls / lock attempts of a bounded wait
   unsigned long long time_limit_ns;  // per query, 0 = none
+  // corridor of a query (batch engine with bounds; null rf = not used)
+  ulonglong2 *rf;
+  uint32_t *touch;
+  int32_t *lint;   // local graphs: rows, heads, ids, renumbering
+  float2 *lw;
+  unsigned long long *ldist;
+  VState *lvs;
+  int lv, la;
+  float mean_len, mean_delay;
+  float wave_mult;  // bucket width of the corridor searches in mean arcs
   const float *mlp;
   float *trace;
   unsigned long long *trace_top;
@@ -113,6 +123,7 @@ struct __align__(16) QueryState {
   uint32_t chunk_fill, chunk_end;
   double hist[kHist];
   int q, src, dst;
+  uint32_t lam_a, lam_b, lam_bB;  // multiplier b / a of the query's corridor and b * B
   float budget;
   uint32_t epoch;
   uint32_t inc_idx;
@@ -183,6 +194,9 @@ struct Ctx {
   QueryState &st;
   BucketTable bt;
   VState *vs;
+  DevGraph g;              // the whole graph, or the corridor's local one
+  int bounds;              // BoundsKind
+  const int32_t *gid = nullptr;  // local vertex -> vertex of the whole graph
   uint32_t *nearq;
   Label *far;
   Label *rest;
@@ -194,11 +208,12 @@ struct Ctx {
   // async mode: arena slots come from this warp's slab (slab_fill points at
   // its fill counter; the slab always has room for the 32 arcs in flight)
   uint32_t *slab_fill = nullptr;
-  __device__ Ctx(const SearchParams &p, QueryState &s) : P(p), st(s) {}
+  __device__ Ctx(const SearchParams &p, QueryState &s)
+      : P(p), st(s), g(p.g), bounds(p.use_bounds ? kBoundsGlobal : kBoundsNone) {}
   // One arena slot (kBadIdx when the arena is exhausted).
   __device__ __forceinline__ uint32_t alloc_one();
   __device__ VView view(int v) const {
-    return view_vs(&vs[v], st.epoch, st.qbase, st.bcur, P.use_bounds != 0);
+    return view_vs(&vs[v], st.epoch, st.qbase, st.bcur, bounds);
   }
   // Forward-search ring entries: (arena index, vertex).  The reverse bound
   // searches use the same memory as a ring of vertex ids.
@@ -206,7 +221,7 @@ struct Ctx {
 };
 
 __device__ __forceinline__ float key_of(const Ctx &c, int32_t vid, float d) {
-  return c.P.use_bounds ? d + c.view(vid).hlen : d;
+  return c.bounds != kBoundsNone ? d + c.view(vid).hlen : d;
 }
 
 // Records the first failure of the query (status + where it happened).
@@ -342,7 +357,9 @@ __device__ inline void pool_rewind(const SearchParams &P, QueryState &st) {
 
 // Copies the answer's path (source .. sink) out of the arena into the path
 // arena (one thread).  Two walks of the parent chain: count, then write.
-__device__ inline void copy_out_path(const SearchParams &P, QueryState &st, int q, bool found) {
+// gid: original ids of a local graph's vertices (null: the ids as they are).
+__device__ inline void copy_out_path(const SearchParams &P, QueryState &st, int q, bool found,
+                                     const int32_t *gid = nullptr) {
   P.path_len[q] = 0;
   P.path_start[q] = 0;
   if (!found || P.path_arena == nullptr) return;
@@ -354,8 +371,10 @@ __device__ inline void copy_out_path(const SearchParams &P, QueryState &st, int 
     return;
   }
   int64_t pos = (int64_t)base + n - 1;
-  for (int32_t k = (int32_t)st.inc_idx; k >= 0; k = __ldcg(&P.pool[k].parent))
-    P.path_arena[pos--] = __ldcg(&P.pool[k].vid) & 0x7fffffff;
+  for (int32_t k = (int32_t)st.inc_idx; k >= 0; k = __ldcg(&P.pool[k].parent)) {
+    const int32_t v = __ldcg(&P.pool[k].vid) & 0x7fffffff;
+    P.path_arena[pos--] = gid ? gid[v] : v;
+  }
   P.path_start[q] = (int64_t)base;
   P.path_len[q] = n;
 }
@@ -433,6 +452,17 @@ __device__ __forceinline__ void push_far(Ctx &c, const Label &l, float f) {
   }
 }
 
+// True when the combined bound rules a label (d, dl) at a vertex with combined
+// distance hmix out: a * d + b * dl + hmix > a * UB + b * B.  The caller has
+// checked d <= UB and dl <= B, so each sum stays below 2^32 (corridor.cuh
+// keeps a * UB + b * B below 2^31).
+__device__ __forceinline__ bool beyond_mix(const QueryState &st, float d, float dl, uint32_t hmix,
+                                           unsigned long long inc) {
+  const uint32_t a = st.lam_a;
+  if (a == 0u) return false;
+  return a * (uint32_t)d + st.lam_b * (uint32_t)dl + hmix > a * (uint32_t)key_d(inc) + st.lam_bB;
+}
+
 // Offers one label (v, nd, ndl) to the search, given v's state view s.
 // from_far = true when it comes from the far pile (budget already checked);
 // returns true when a far label must stay in the far pile.  A label accepted
@@ -455,7 +485,9 @@ __device__ __forceinline__ bool offer_with(Ctx &c, int32_t v, float nd, float nd
   const float f = nd + s.hlen;
   if (P.mode == VINE_MODE_OPTIMAL) {
     const uint64_t key = pack_key(f, lb_dl);
-    if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) return false;
+    const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
+    if (key >= inc) return false;
+    if (c.bounds == kBoundsLocal && beyond_mix(st, nd, ndl, s.hmix, inc)) return false;
     if (v == st.dst) {
       sink_improve(c, v, nd, ndl, parent, key);
       return false;
@@ -543,14 +575,14 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
       if (i0 + b * G < n) lab[b] = load_label(&P.pool[idx[b]]);
 #pragma unroll
     for (int b = 0; b < kBatch; ++b)
-      if (i0 + b * G < n && (uint32_t)(lab[b].vid & 0x7fffffff) >= (uint32_t)P.g.n) {
+      if (i0 + b * G < n && (uint32_t)(lab[b].vid & 0x7fffffff) >= (uint32_t)c.g.n) {
         fail_query(st, VINE_ERR_INTERNAL, kSiteRing);
         lab[b].vid = (int)kDeadBit;  // vertex 0, dead: expands nothing
       }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
-      s[b] = VView{0.0f, true, 0.0f, 0.0f, 0u};
-      if (P.use_bounds && i0 + b * G < n) s[b] = c.view(lab[b].vid & 0x7fffffff);
+      s[b] = VView{0.0f, true, 0.0f, 0.0f, 0u, 0u};
+      if (c.bounds != kBoundsNone && i0 + b * G < n) s[b] = c.view(lab[b].vid & 0x7fffffff);
     }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
@@ -564,12 +596,14 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
         if (!(f < hi)) live = false;
         if (live && P.mode == VINE_MODE_OPTIMAL) {
           const uint64_t key = pack_key(f, lab[b].dl + s[b].hdel);
-          if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) live = false;
+          const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
+          if (key >= inc) live = false;
+          else if (c.bounds == kBoundsLocal && beyond_mix(st, lab[b].d, lab[b].dl, s[b].hmix, inc)) live = false;
         }
       }
       if (live) {
-        beg = __ldg(&P.g.row[v]);
-        deg = __ldg(&P.g.row[v + 1]) - beg;
+        beg = c.g.row[v];  // (not through the read-only path: a local graph is
+        deg = c.g.row[v + 1] - beg;  // written by this kernel)
         if (deg > 0) warp_agg_inc(&st.r_live);
       }
       rb.idx[i] = idx[b];
@@ -606,8 +640,8 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
       if (e < total) {
         const int k = upper_index(rb.off, n, e);
         const int j = rb.beg[k] + (e - rb.off[k]);
-        vv[b] = __ldg(&P.g.col[j]);
-        const float2 w = __ldg(&P.g.w[j]);
+        vv[b] = c.g.col[j];
+        const float2 w = c.g.w[j];
         nd[b] = rb.d[k] + w.x;
         nl[b] = rb.dl[k] + w.y;
         par[b] = rb.idx[k];
@@ -638,7 +672,7 @@ __device__ inline void reverse_expand_block(Ctx &c, const RoundBuf &rb, int whic
   for (int i = sid; i < n; i += G) {
     const int v = (int)c.nearq[(first + (uint32_t)i) & P.near_mask];
     const int beg = __ldg(&P.g.rrow[v]);
-    const VView s = view_vs(&c.vs[v], st.epoch, st.qbase, st.bcur, true);
+    const VView s = view_vs(&c.vs[v], st.epoch, st.qbase, st.bcur, kBoundsGlobal);
     rb.vid[i] = v;
     rb.d[i] = which == 0 ? s.hdel : s.hlen;
     rb.beg[i] = beg;
@@ -690,7 +724,7 @@ __device__ inline void reverse_expand_block(Ctx &c, const RoundBuf &rb, int whic
 
 // Current reverse distance of v in pass `which` (+inf when unset).
 __device__ __forceinline__ float reverse_dist(const Ctx &c, int which, int v) {
-  const VView s = view_vs(&c.vs[v], c.st.epoch, c.st.qbase, c.st.bcur, true);
+  const VView s = view_vs(&c.vs[v], c.st.epoch, c.st.qbase, c.st.bcur, kBoundsGlobal);
   if (which == 0) return __ldcg(&c.vs[v].e_del) == c.st.epoch ? s.hdel : INFINITY;
   return __ldcg(&c.vs[v].e_del) == c.st.epoch ? s.hlen : INFINITY;
 }
