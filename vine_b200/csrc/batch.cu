@@ -28,6 +28,7 @@
 #include "corridor.cuh"
 #include "engine_host.h"
 #include "search.cuh"
+#include "wave_search.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -277,17 +278,16 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
       e = __ldcg(&ring[(h + (uint32_t)lane) & P.near_mask]);
       // an entry outside the arena or the vertex range would mean a protocol
       // slip: fail the query instead of following it
-      entry_ok = (uint64_t)e.x < (uint64_t)P.pool_cap && e.y < (uint32_t)c.g.n;
+      entry_ok = (uint64_t)e.x < (uint64_t)P.pool_cap && e.y < (uint32_t)P.g.n;
       if (!entry_ok) fail_query(st, VINE_ERR_INTERNAL, kSiteRing);
     }
     if (entry_ok) {
       idx = e.x;
       const int v = (int)e.y;
       const Label lab = load_label(&P.pool[idx]);  // issued together with the loads below
-      const VView s = c.bounds != kBoundsNone ? c.view(v) : VView{0.0f, true, 0.0f, 0.0f, 0u, 0u};
-      // (plain loads: a local graph is written by this kernel)
-      const int r0 = c.g.row[v];
-      const int r1 = c.g.row[v + 1];
+      const VView s = P.use_bounds ? c.view(v) : VView{0.0f, true, 0.0f, 0.0f, 0u};
+      const int r0 = __ldg(&P.g.row[v]);
+      const int r1 = __ldg(&P.g.row[v + 1]);
       d = lab.d;
       dl = lab.dl;
       bool live = !(lab.vid & (int)kDeadBit);
@@ -296,9 +296,7 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
         if (!(f < hi)) live = false;
         if (live && P.mode == VINE_MODE_OPTIMAL) {
           const uint64_t key = pack_key(f, dl + s.hdel);
-          const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
-          if (key >= inc) live = false;
-          else if (c.bounds == kBoundsLocal && beyond_mix(st, d, dl, s.hmix, inc)) live = false;
+          if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) live = false;
         }
       }
       if (live) {
@@ -357,8 +355,8 @@ __device__ __forceinline__ void bucket_async(Ctx &c) {
         int u = 0;
         if (e < total) {
           const int j = obeg + (e - oex);
-          u = c.g.col[j];
-          const float2 w = c.g.w[j];
+          u = __ldg(&P.g.col[j]);
+          const float2 w = __ldg(&P.g.w[j]);
           const VView s = c.view(u);
           offer_with(c, u, od + w.x, odl + w.y, oidx, false, s, &nidx);
         }
@@ -728,7 +726,7 @@ __device__ __forceinline__ void corridor_mem(const SearchParams &P, int slot, Co
   }
   M.map = reinterpret_cast<uint32_t *>(ip);
   for (int k = 0; k < 4; ++k) M.dist[k] = P.ldist + ((size_t)slot * 4 + k) * lv;
-  M.lvs = P.lvs + (size_t)slot * lv;
+  M.state = P.lstate + (size_t)slot * lv;
 }
 
 // kBounds: the call uses lower bounds (corridors).  Without them the corridor
@@ -769,10 +767,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
   const int tid = threadIdx.x, G = blockDim.x;
   const int slot = blockIdx.x;
   Ctx c(P, st);
-  c.bounds = kBounds ? kBoundsGlobal : kBoundsNone;
   const RoundBuf rb{r_idx, r_vid, r_d, r_dl, r_beg, r_off, scan, RC};
-  VState *const global_vs = P.vs + (size_t)slot * P.g.n;
-  c.vs = global_vs;
+  c.vs = P.vs + (size_t)slot * P.g.n;
   c.nearq = P.nearq + (size_t)slot * 2 * (P.near_mask + 1u);  // uint2 entries
   c.far = P.far + (size_t)slot * P.far_cap * 4;
   c.rest = P.rest + (size_t)slot * P.rest_cap;
@@ -858,7 +854,6 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       st.split_cycles = st.split_items = st.policy_cycles = st.rest_items = 0;
       st.idle_cycles = st.publish_cycles = 0;
       st.load_cycles = st.relax_cycles = 0;
-      st.lam_a = st.lam_b = st.lam_bB = 0;
       st.hist_n = 0;
       st.sink_n = 0;
       st.b_labels = st.b_expanded = st.b_rounds = st.b_dominated = 0;
@@ -894,12 +889,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       }
     }
     __syncthreads();
-    if (kBounds) {
-      c.g = P.g;
-      c.vs = c.bt.vs = global_vs;
-      c.bounds = kBoundsGlobal;
-      c.gid = nullptr;
-    }
+    const int32_t *gid = nullptr;  // original ids, once the search ran on a local graph
     if (!st.done && !st.abort) {
       if (kBounds) {
         const long long t_b = clock64();
@@ -909,27 +899,55 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           if (tid == 0) corridor_mem(P, slot, W.m);
           __syncthreads();
           how = corridor_prepare(P, st, &which);
-          const LocalGraph loc = W.m.loc[which];
-          VState *const lvs = W.m.lvs;
-          __syncthreads();
-          for (int i = tid; i < H; i += G) tv[i] = kEmpty;  // the wave state lay here
-          for (int i = tid; i < NL; i += G) locks[i] = 0;
           if (how == kCorridorReady) {
-            c.g = loc.g;
-            c.gid = loc.gid;
-            c.vs = c.bt.vs = lvs;
-            c.bounds = kBoundsLocal;
-            if (tid == 0) P.pool[st.inc_idx].vid = st.src;
+            gid = W.m.loc[which].gid;
+            __syncthreads();  // read by all: the search's state lies over it
+            if (tid == 0) {
+              const CorridorMem M = W.m;
+              const LocalGraph L = M.loc[which];
+              WaveSearch &S = reinterpret_cast<SearchShared *>(smem)->s;
+              S.row = L.g.row;
+              S.col = L.g.col;
+              S.w = L.g.w;
+              S.state = M.state;
+              S.n = L.g.n;
+              S.sink = st.dst;
+              S.B = (uint32_t)floorf(st.budget);
+              S.a = st.lam_a;
+              S.b = st.lam_b;
+              S.bB = st.lam_bB;
+              S.pa = st.ord_a;
+              S.pb = st.ord_b;
+              S.pool = P.pool;
+              S.next = P.next;
+              S.head = M.map;
+              for (int b = 0; b < 2; ++b) {
+                S.novf[b] = reinterpret_cast<uint4 *>(M.ovf[b]);
+                S.fovf[b] = reinterpret_cast<uint4 *>(M.far[b]);
+              }
+              S.novf_cap = M.ovf_cap / 4;
+              S.fovf_cap = M.far_cap / 2;
+            }
+            if (tid == 0) {
+              st.bound_cycles = clock64() - t_b;
+              st.n_bound_rounds = st.n_rounds - r_b;
+            }
+            const long long t_w = clock64();
+            wave_search(P, st);
+            if (tid == 0) st.relax_cycles += clock64() - t_w;
           } else if (how == kCorridorInfeasible && tid == 0) {
             st.done = 1;
           }
+          // the bucket table lay under the wave state
+          for (int i = tid; i < H; i += G) tv[i] = kEmpty;
+          for (int i = tid; i < NL; i += G) locks[i] = 0;
           __syncthreads();
         }
         if (how == kCorridorNone && !st.abort) {
           cta_reverse_search(c, rb, 0, st.budget, P.delta_del);
           cta_reverse_search(c, rb, 1, INFINITY, P.delta_len);
         }
-        if (tid == 0) {
+        if (tid == 0 && how != kCorridorReady) {
           st.bound_cycles = clock64() - t_b;
           st.n_bound_rounds = st.n_rounds - r_b;
         }
@@ -1278,7 +1296,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       // a corridor seeds inc_key with its cost bound before a label has it
       const bool ok = st.abort == 0;
       const bool found = ok && st.inc_key != ~0ull && st.inc_idx != 0xffffffffu;
-      copy_out_path(P, st, q, found, c.gid);
+      copy_out_path(P, st, q, found, gid);
       P.status[q] = ok ? VINE_OK : st.abort;
       P.found[q] = found ? 1 : 0;
       P.cost[q] = found ? key_d(st.inc_key) : INFINITY;
@@ -1365,7 +1383,7 @@ void BatchWorkspace::release() {
   cudaFree(lint);
   cudaFree(lw);
   cudaFree(ldist);
-  cudaFree(lvs);
+  cudaFree(lstate);
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   *this = BatchWorkspace();
 }
@@ -1382,7 +1400,7 @@ static int ensure_corridor(vine_graph *g, const Resolved &r) {
   const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
   const size_t ints = corridor_ints((int)lv, (int)la);
   const size_t per = n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
-                     lv * (4 * sizeof(unsigned long long) + sizeof(VState));
+                     lv * (4 * sizeof(unsigned long long) + sizeof(uint4));
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   if (per * r.slots > total_b / 8) return VINE_OK;
@@ -1391,7 +1409,7 @@ static int ensure_corridor(vine_graph *g, const Resolved &r) {
   VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * k));
   VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lvs, sizeof(VState) * lv * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * k));
   VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
   VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
   w.lv = (int)lv;
@@ -1560,7 +1578,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.lint = w.lint;
   P.lw = w.lw;
   P.ldist = w.ldist;
-  P.lvs = w.lvs;
+  P.lstate = w.lstate;
   P.lv = w.lv;
   P.la = w.la;
   P.mean_len = g->mean_len;
@@ -1571,7 +1589,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   // two-sided search for 64 queries with the linear rule, 7 ms so).
   const float deg = (float)g->m / (float)std::max(1, g->n);
   const float thin = std::min(1.0f, 3.0f / std::max(1.0f, deg));
-  P.wave_mult = 6.0f * thin * thin;
+  P.wave_mult = 12.0f * thin * thin;
   P.mlp = (c.policy == VINE_POLICY_MLP && c.mlp) ? c.mlp->params : nullptr;
   P.trace = c.trace ? w.trace : nullptr;
   P.trace_top = w.counters + 3;

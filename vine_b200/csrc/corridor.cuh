@@ -44,6 +44,7 @@ constexpr uint32_t kMemberTag = 0xfffffffeu;   // rf[v].y high word: v has a loc
 constexpr float kIntLimit = 16777216.0f;       // 2^24: budgets and costs handled here
 constexpr int kWaveQ = 2048;                   // queue entries kept in shared memory
 constexpr int kCorridorVertices = 1 << 16;     // largest local graph
+constexpr double kFirstLambda = 0.5;           // first multiplier, in mean lengths per mean delay
 constexpr double kWideGap = 0.3;               // (T - meeting key) / meeting key worth another multiplier
 constexpr int kShrinkTo = 1024;                // local graphs up to this size are not shrunk further
 constexpr int kHubs = 32;                      // see WaveShared::hub
@@ -68,7 +69,25 @@ struct CorridorMem {
   int lv, la;          // capacity of a local graph: vertices, arcs
   uint32_t *map;       // [lv] old local id -> new local id
   unsigned long long *dist[4];  // [lv] distances on the local graph
-  VState *lvs;         // [lv] label search state
+  uint4 *state;        // [lv] delay, length and combined distance to the sink
+};
+
+// Weights of one search.  pure: key = delay, the second value is the length;
+// otherwise key = a * len + b * delay and the second value is the delay.
+struct Combo {
+  uint32_t a, b;
+  bool pure;
+  uint32_t B;
+};
+
+// What a local pass computes: distances from `root` along (row, col, w) under
+// c; keys above `limit` are dropped.
+struct PassArgs {
+  const int32_t *row, *col;
+  const float2 *w;
+  int n, root;
+  uint32_t limit;
+  uint32_t delta;
 };
 
 // Shared-memory state of the wave searches.  It lies over the bucket table,
@@ -82,6 +101,14 @@ struct __align__(16) WaveShared {
   uint32_t cnt;
   int cur;
   CorridorMem m;  // the worker's arrays
+  // What the search in progress works on.  Kept here and not passed by value:
+  // by-value structs of called functions live in local memory, whose lines
+  // the waves' gathers push out of L1 (7.0e6 of 9.8e6 loads of a profile).
+  Combo c;
+  PassArgs a;
+  DevGraph g;
+  uint32_t delta;
+  int fb;
   uint32_t hub[kHubs], nhub;  // vertices of this round whose arcs the block shares
   int clipped, overflow, stop;
   int scan[kScanScratch];
@@ -230,14 +257,6 @@ __device__ __forceinline__ void wave_emit(WaveShared &W, const CorridorMem &M, i
 }
 
 // ------------------------------------------------------- two-sided search
-
-// Weights of one search.  pure: key = delay, the second value is the length;
-// otherwise key = a * len + b * delay and the second value is the delay.
-struct Combo {
-  uint32_t a, b;
-  bool pure;
-  uint32_t B;
-};
 
 __device__ __forceinline__ uint32_t combo_limit(const WaveShared &W, const Combo &k) {
   if (k.pure) return k.B;
@@ -475,11 +494,11 @@ __device__ __forceinline__ uint32_t bi_hubs(const DevGraph &g, WaveShared &W, co
 // atomics of all of them in flight together); arcs past that are dealt to the
 // lanes of the warp and those of hubs to the block, so hubs do not serialise.
 // While a round fits one warp, warp 0 runs on alone without block barriers.
-__device__ __forceinline__ uint32_t bi_rounds(QueryState &st, const DevGraph &g, WaveShared &W,
-                                              const CorridorMem &M, const Combo &c, int *pcur,
-                                              int fb) {
+__device__ __forceinline__ uint32_t bi_rounds(QueryState &st, WaveShared &W, int &cur, int fb) {
+  const DevGraph &g = W.g;
+  const CorridorMem &M = W.m;
+  const Combo &c = W.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  int cur = *pcur;
   uint32_t relaxed = 0;
   for (;;) {
     __syncthreads();
@@ -523,15 +542,20 @@ __device__ __forceinline__ uint32_t bi_rounds(QueryState &st, const DevGraph &g,
       if (tid == 0) W.nhub = 0;
     }
   }
-  *pcur = cur;
   return relaxed;
 }
 
 // Starts a two-sided search: both ends queued, `best0` what W.best starts from.
-__device__ __forceinline__ void bi_start(WaveShared &W, const CorridorMem &M, int s, int t,
+__device__ __forceinline__ void bi_start(WaveShared &W, const DevGraph &g, const Combo &c, int s, int t,
                                          unsigned long long best0, uint32_t delta) {
+  const CorridorMem &M = W.m;
   __syncthreads();
   if (threadIdx.x == 0) {
+    W.g = g;
+    W.c = c;
+    W.delta = delta;
+    W.cur = 0;
+    W.fb = 0;
     W.mu = kUnset;
     W.best = best0;
     W.nq[0] = 2;
@@ -559,17 +583,17 @@ __device__ __forceinline__ void bi_start(WaveShared &W, const CorridorMem &M, in
 // F + H <= T has both its distances: on a shortest way to such a vertex no
 // vertex is pruned, since what it is charged for the other side, its distance
 // there or the radius of that side, is never more than the truth.
-// *pcur / *pfb: queue and far pile in use.
-__device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, const DevGraph &g,
-                                        Combo c, bool to_meeting, uint32_t delta, int *pcur,
-                                        int *pfb) {
+// W.cur / W.fb: queue and far pile in use.
+__device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, bool to_meeting) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   const CorridorMem &M = W.m;
-  int cur = *pcur, fb = *pfb;
+  const Combo &c = W.c;
+  __syncthreads();
+  int cur = W.cur, fb = W.fb;
   uint32_t relaxed = 0;
   for (;;) {
-    relaxed += bi_rounds(st, g, W, M, c, &cur, fb);
+    relaxed += bi_rounds(st, W, cur, fb);
     // nothing unsettled lies below far_min on either side
     const uint32_t fm = W.far_min, lo = max(W.hi, fm);
     const bool stop = fm == kNoKey || W.stop || (to_meeting && 2ull * lo >= (vol(W.mu) >> 32));
@@ -578,9 +602,12 @@ __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, c
       W.rdone = fm == kNoKey ? kKeyMax : lo;
       if (!stop) {
         if (over_time(P, st)) W.stop = 1;
-        W.hi = min(lo, kKeyMax + 1u - delta) + delta;
+        W.hi = min(lo, kKeyMax + 1u - W.delta) + W.delta;
         W.far_min = kNoKey;
         W.nfar[fb ^ 1] = 0;
+      } else {
+        W.cur = cur;
+        W.fb = fb;
       }
     }
     __syncthreads();
@@ -602,8 +629,6 @@ __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, c
     }
     fb ^= 1;
   }
-  *pcur = cur;
-  *pfb = fb;
   return relaxed;
 }
 
@@ -683,14 +708,15 @@ __device__ __forceinline__ bool build_csr(WaveShared &W, const int32_t *orow, co
   return true;
 }
 
-// Copies the corridor of the finished two-sided search on graph g into L
-// (og: original ids of g's vertices, null for the whole graph).  The new ids
-// of g's vertices stay in rf until the next reset.  Returns the vertex count;
+// Copies the corridor of the finished two-sided search (graph W.g) into L
+// (og: original ids of its vertices, null for the whole graph).  The new ids
+// of those vertices stay in rf until the next reset.  Returns the vertex count;
 // -1 (nothing copied) when it does not fit or exceeds `most`.
-__device__ __noinline__ int build_local(const DevGraph &g, const int32_t *og, Combo c, LocalGraph &L,
-                                        int most) {
+__device__ __noinline__ int build_local(const int32_t *og, LocalGraph &L, int most) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
+  const DevGraph &g = W.g;
+  const Combo &c = W.c;
   const CorridorMem &M = W.m;
   const int G = blockDim.x, tid = threadIdx.x;
   __syncthreads();
@@ -746,20 +772,12 @@ struct DistArray {
   }
 };
 
-// What a local pass computes: distances from `root` along (row, col, w) under
-// c; keys above `limit` are dropped.
-struct PassArgs {
-  const int32_t *row, *col;
-  const float2 *w;
-  int n, root;
-  uint32_t limit;
-  uint32_t delta;
-};
-
 template <bool kShared>
-__device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const CorridorMem &M, const PassArgs &A,
-                                                const Combo &c, const DistArray<kShared> &D, int cur,
+__device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<kShared> &D, int cur,
                                                 int fb, uint32_t i0, uint32_t take) {
+  const CorridorMem &M = W.m;
+  const PassArgs &A = W.a;
+  const Combo &c = W.c;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, nxt = cur ^ 1;
   const uint32_t hi = vol(W.hi), limit = A.limit;
@@ -848,11 +866,12 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const CorridorMem
 // Latency-bound like bi_rounds; a corridor is long and narrow, so most rounds
 // fit one warp and run without block barriers, on shared-memory distances.
 template <bool kShared>
-__device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState &st, PassArgs A,
-                                               Combo c, unsigned long long *out) {
+__device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState &st,
+                                               unsigned long long *out) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   const CorridorMem &M = W.m;
+  const PassArgs &A = W.a;
   const int G = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = G >> 5;
   DistArray<kShared> D;
   D.p = kShared ? reinterpret_cast<unsigned long long *>(smem + kWaveBytes) : out;
@@ -903,7 +922,7 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
       if (warp == 0) {
         uint32_t n = nc;
         do {
-          relaxed += local_chunk<kShared>(W, M, A, c, D, cur, fb, 0, n);
+          relaxed += local_chunk<kShared>(W, D, cur, fb, 0, n);
           __syncwarp();
           if (lane == 0) {
             W.nq[cur] = 0;
@@ -918,7 +937,7 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
     } else {
       const uint32_t take = min(32u, (nc + (uint32_t)nw - 1u) / (uint32_t)nw);
       for (uint32_t base = (uint32_t)warp * take; base < nc; base += (uint32_t)nw * take)
-        relaxed += local_chunk<kShared>(W, M, A, c, D, cur, fb, base, min(take, nc - base));
+        relaxed += local_chunk<kShared>(W, D, cur, fb, base, min(take, nc - base));
       __syncthreads();
       if (tid == 0) {
         W.nq[cur] = 0;
@@ -938,10 +957,17 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
   return relaxed;
 }
 
-__device__ __forceinline__ uint32_t local_pass(const SearchParams &P, QueryState &st, const PassArgs &A,
-                                               const Combo &c, unsigned long long *out) {
+__device__ __forceinline__ uint32_t local_pass(const SearchParams &P, QueryState &st, WaveShared &W,
+                                               const PassArgs &A, const Combo &c,
+                                               unsigned long long *out) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    W.a = A;
+    W.c = c;
+  }
+  __syncthreads();
   const int cap = (int)((table_region_bytes(P.table_log2, P.lock_log2) - kWaveBytes) / sizeof(unsigned long long));
-  return A.n <= cap ? local_pass_in<true>(P, st, A, c, out) : local_pass_in<false>(P, st, A, c, out);
+  return A.n <= cap ? local_pass_in<true>(P, st, out) : local_pass_in<false>(P, st, out);
 }
 
 // ----------------------------------------------------------------- multipliers
@@ -1006,9 +1032,9 @@ struct Duals {
 };
 
 // Builds the query's corridor (all threads; every thread computes the same
-// multipliers).  kCorridorReady: local graph *which holds it, M.lvs is
-// initialised, st.src / st.dst are local ids, st.inc_key carries the cost
-// bound and st.lam_* the multiplier; kCorridorInfeasible: no path within the
+// multipliers).  kCorridorReady: local graph *which holds it, M.state is
+// filled, st.src / st.dst are local ids, st.inc_key carries the cost bound,
+// st.lam_* the multiplier and st.ord_* the order of the search; kCorridorInfeasible: no path within the
 // budget; kCorridorNone: not handled here (costs from 2^24 on, or a corridor
 // past the local capacity).
 __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &st, int *which) {
@@ -1027,7 +1053,7 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
   }
   uint32_t relaxed = 0;
   Duals k{-1.0, 0.0, -1.0, 0.0, -1.0, 0.0};
-  double lambda = unit;  // a unit of delay weighs like a unit of length
+  double lambda = unit * kFirstLambda;
   int result = kCorridorNone, ne = -1, cl = -1, ls = s, lt = t;  // cl: graph searched (-1: the whole one)
   bool pure = false;
   Combo c;
@@ -1050,9 +1076,8 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
       best0 = ((unsigned long long)(pure ? (uint32_t)k.ub : k.T(c)) << 32) | (uint32_t)k.ub_delay;
     const DevGraph &g = cl < 0 ? P.g : M.loc[cl].g;
     const uint32_t delta = combo_delta(P, c, P.wave_mult);
-    int cur = 0, fb = 0;
-    bi_start(W, M, ls, lt, best0, delta);
-    relaxed += bi_run(P, st, g, c, true, delta, &cur, &fb);
+    bi_start(W, g, c, ls, lt, best0, delta);
+    relaxed += bi_run(P, st, true);
     if (W.stop) break;
     const unsigned long long mu = W.mu, best = W.best;
     if (best != kUnset) {
@@ -1076,21 +1101,31 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
     // The next multiplier to try: the slope once both sides of the budget
     // are known, else less weight on the delay.
     double next = k.slope();
-    if (next < 0.0) next = (pure ? unit : lambda) * 0.2;
+    if (next < 0.0) {
+      // the more of the budget the best combined path leaves, the smaller the
+      // multiplier: on the road graphs a path with 0.95 of the budget met
+      // multipliers about half as large, 0.92 a quarter (ratio^16)
+      const float used = k.len2 >= 0.0 && !pure ? (float)(k.del2 / fmax(1.0, (double)B)) : 0.9f;
+      float f = used * used;
+      f *= f;
+      f *= f;
+      f *= f;
+      next = (pure ? unit : lambda) * (double)fminf(0.7f, fmaxf(0.1f, f));
+    }
     const bool settled = !pure && fabs(next - lambda) <= 0.1 * lambda;
     // A wide gap between T and the meeting key means a poor multiplier:
     // another search now costs less than completing this one.
     const double gap = pure ? 1.0 : ((double)k.T(c) - (double)(mu >> 32)) / fmax(1.0, (double)(mu >> 32));
     if (attempt >= 4 || settled || cl >= 0 || !(gap > kWideGap)) {
       __syncthreads();
-      relaxed += bi_run(P, st, g, c, false, delta, &cur, &fb);
+      relaxed += bi_run(P, st, false);
       if (W.stop) break;
       const unsigned long long b2 = W.best;
       k.feasible(pure ? (double)(b2 >> 32)
                       : floor((double)((b2 >> 32) - (unsigned long long)c.b * B) / (double)c.a),
                  (double)(uint32_t)b2);
       const int to = cl < 0 ? 0 : cl ^ 1;
-      const int n2 = build_local(g, cl < 0 ? nullptr : M.loc[cl].gid, c, M.loc[to],
+      const int n2 = build_local(cl < 0 ? nullptr : M.loc[cl].gid, M.loc[to],
                                  cl < 0 ? M.lv : ne - ne / 4);
       if (n2 >= 0) {
         ls = (int)(uint32_t)__ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[ls]) + 1);
@@ -1118,7 +1153,7 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
     const uint32_t one = 0x40000000u;
     Combo cd{0u, 1u, true, B}, cl_{1u, 0u, false, B};
     PassArgs A{g.rrow, g.rcol, g.rw, ne, lt, B, wide ? combo_delta(P, cd, P.wave_mult) : one};
-    relaxed += local_pass(P, st, A, cd, D0);
+    relaxed += local_pass(P, st, W, A, cd, D0);
     const unsigned long long xd = __ldcg(&D0[ls]);  // the fastest path
     if (xd != kUnset) {
       k.feasible((double)(uint32_t)xd, (double)(xd >> 32));
@@ -1129,7 +1164,7 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
     }
     A.limit = (uint32_t)k.ub;
     A.delta = wide ? combo_delta(P, cl_, P.wave_mult) : one;
-    relaxed += local_pass(P, st, A, cl_, D1);
+    relaxed += local_pass(P, st, W, A, cl_, D1);
     const unsigned long long xl = __ldcg(&D1[ls]);  // the shortest path
     if (xl != kUnset) {
       const double l0 = (double)(xl >> 32), d0 = (double)(uint32_t)xl;
@@ -1147,7 +1182,7 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
           const double l2 = k.len2, d2 = k.del2, l1 = k.len1, d1 = k.del1;
           A.limit = k.T(c);
           A.delta = wide ? combo_delta(P, c, P.wave_mult) : one;
-          relaxed += local_pass(P, st, A, c, Hcur);
+          relaxed += local_pass(P, st, W, A, c, Hcur);
           const unsigned long long x = __ldcg(&Hcur[ls]);
           if (x == kUnset) break;
           const double low = ((double)(x >> 32) - (double)c.b * (double)B) / (double)c.a;
@@ -1177,16 +1212,7 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
       const unsigned long long hd = __ldcg(&D0[i]), hl = __ldcg(&D1[i]);
       const uint32_t hm = use.a ? key_hi(__ldcg(&Hbest[i])) : 0u;
       const bool in = hd != kUnset && hl != kUnset && hm != kNoKey;
-      VState v;
-      v.epoch = st.epoch;
-      v.sdel = INFINITY;
-      v.e_del = hm;
-      v.hdel = in ? (float)key_hi(hd) : 0.0f;
-      v.bep = 0;
-      v.bmin = 0.0f;
-      v.hlen = in ? (float)key_hi(hl) : INFINITY;
-      v.bhead = kNone;
-      M.lvs[i] = v;
+      M.state[i] = make_uint4(key_hi(hd), in ? key_hi(hl) : kNoKey, hm, 0u);
     }
     if (tid == 0) {
       st.src = ls;
@@ -1195,6 +1221,10 @@ __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &
       st.lam_b = use.b;
       st.lam_bB = use.b * B;
       st.inc_key = pack_key((float)k.ub, INFINITY);
+      Combo o = use;  // the search's order: the same weights, else both criteria alike
+      if (use.a == 0 && !pick_combo(unit, k.ub, (double)B, &o)) o.a = o.b = 1;
+      st.ord_a = o.a;
+      st.ord_b = o.b;
     }
     *which = cl;
     result = kCorridorReady;

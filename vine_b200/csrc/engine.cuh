@@ -40,9 +40,7 @@ struct Label {
 // for the query / bucket whose tag sits beside it.  32 bytes = one sector.
 //   (epoch, sdel)  smallest delay of labels at v in finished buckets whose
 //                  table entries were folded (8-byte CAS pair)
-//   (e_del, hdel)  reverse delay distance to the sink (bounds mode, CAS pair);
-//                  on a corridor's local graph e_del holds the combined
-//                  distance to the sink under the query's multiplier
+//   (e_del, hdel)  reverse delay distance to the sink (bounds mode, CAS pair)
 //   (bep, bmin)    bucket id and smallest delay of v's overflow chain; a
 //                  chain of an earlier bucket of the same query counts as
 //                  settled (8-byte pair, written under v's stripe lock)
@@ -68,19 +66,11 @@ struct VView {
   bool reach;   // bounds valid: v can lie on a feasible path
   float hdel, hlen;
   uint32_t bep; // chain tag
-  uint32_t hmix; // combined distance to the sink (kBoundsLocal)
-};
-
-// Which lower bounds a query's vertex states carry.
-enum BoundsKind {
-  kBoundsNone = 0,    // none
-  kBoundsGlobal = 1,  // delay and length, written by the reverse searches
-  kBoundsLocal = 2    // delay, length and combined distance on a local graph
 };
 
 // qbase / bcur: first bucket id of the query and id of the open bucket.
 __device__ __forceinline__ VView view_vs(const VState *p, uint32_t epoch, uint32_t qbase,
-                                         uint32_t bcur, int bounds) {
+                                         uint32_t bcur, bool bounds) {
   // the whole 32-byte state in one 256-bit load (L2, like __ldcg); VState
   // is 32-byte aligned
   uint4 a, b;
@@ -94,9 +84,8 @@ __device__ __forceinline__ VView view_vs(const VState *p, uint32_t epoch, uint32
   if (b.x >= qbase && b.x < bcur) sd = fminf(sd, __uint_as_float(b.y));
   v.sdel = sd;
   v.bep = b.x;
-  v.hmix = a.z;
-  if (bounds != kBoundsNone) {
-    v.reach = (bounds == kBoundsLocal || a.z == epoch) && __uint_as_float(b.z) < INFINITY;
+  if (bounds) {
+    v.reach = a.z == epoch && __uint_as_float(b.z) < INFINITY;
     v.hdel = __uint_as_float(a.w);
     v.hlen = __uint_as_float(b.z);
   } else {

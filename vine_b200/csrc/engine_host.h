@@ -53,7 +53,7 @@ struct BatchWorkspace {
   int32_t *lint = nullptr;
   float2 *lw = nullptr;
   unsigned long long *ldist = nullptr;
-  VState *lvs = nullptr;
+  uint4 *lstate = nullptr;
   int lv = 0, la = 0;
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape

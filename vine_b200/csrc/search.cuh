@@ -98,7 +98,7 @@ struct SearchParams {
   int32_t *lint;   // local graphs: rows, heads, ids, renumbering
   float2 *lw;
   unsigned long long *ldist;
-  VState *lvs;
+  uint4 *lstate;
   int lv, la;
   float mean_len, mean_delay;
   float wave_mult;  // bucket width of the corridor searches in mean arcs
@@ -123,7 +123,8 @@ struct __align__(16) QueryState {
   uint32_t chunk_fill, chunk_end;
   double hist[kHist];
   int q, src, dst;
-  uint32_t lam_a, lam_b, lam_bB;  // multiplier b / a of the query's corridor and b * B
+  // corridor: multiplier b / a and b * B of the bound, weights of the wave order
+  uint32_t lam_a, lam_b, lam_bB, ord_a, ord_b;
   float budget;
   uint32_t epoch;
   uint32_t inc_idx;
@@ -194,9 +195,6 @@ struct Ctx {
   QueryState &st;
   BucketTable bt;
   VState *vs;
-  DevGraph g;              // the whole graph, or the corridor's local one
-  int bounds;              // BoundsKind
-  const int32_t *gid = nullptr;  // local vertex -> vertex of the whole graph
   uint32_t *nearq;
   Label *far;
   Label *rest;
@@ -208,12 +206,11 @@ struct Ctx {
   // async mode: arena slots come from this warp's slab (slab_fill points at
   // its fill counter; the slab always has room for the 32 arcs in flight)
   uint32_t *slab_fill = nullptr;
-  __device__ Ctx(const SearchParams &p, QueryState &s)
-      : P(p), st(s), g(p.g), bounds(p.use_bounds ? kBoundsGlobal : kBoundsNone) {}
+  __device__ Ctx(const SearchParams &p, QueryState &s) : P(p), st(s) {}
   // One arena slot (kBadIdx when the arena is exhausted).
   __device__ __forceinline__ uint32_t alloc_one();
   __device__ VView view(int v) const {
-    return view_vs(&vs[v], st.epoch, st.qbase, st.bcur, bounds);
+    return view_vs(&vs[v], st.epoch, st.qbase, st.bcur, P.use_bounds != 0);
   }
   // Forward-search ring entries: (arena index, vertex).  The reverse bound
   // searches use the same memory as a ring of vertex ids.
@@ -221,7 +218,7 @@ struct Ctx {
 };
 
 __device__ __forceinline__ float key_of(const Ctx &c, int32_t vid, float d) {
-  return c.bounds != kBoundsNone ? d + c.view(vid).hlen : d;
+  return c.P.use_bounds ? d + c.view(vid).hlen : d;
 }
 
 // Records the first failure of the query (status + where it happened).
@@ -452,17 +449,6 @@ __device__ __forceinline__ void push_far(Ctx &c, const Label &l, float f) {
   }
 }
 
-// True when the combined bound rules a label (d, dl) at a vertex with combined
-// distance hmix out: a * d + b * dl + hmix > a * UB + b * B.  The caller has
-// checked d <= UB and dl <= B, so each sum stays below 2^32 (corridor.cuh
-// keeps a * UB + b * B below 2^31).
-__device__ __forceinline__ bool beyond_mix(const QueryState &st, float d, float dl, uint32_t hmix,
-                                           unsigned long long inc) {
-  const uint32_t a = st.lam_a;
-  if (a == 0u) return false;
-  return a * (uint32_t)d + st.lam_b * (uint32_t)dl + hmix > a * (uint32_t)key_d(inc) + st.lam_bB;
-}
-
 // Offers one label (v, nd, ndl) to the search, given v's state view s.
 // from_far = true when it comes from the far pile (budget already checked);
 // returns true when a far label must stay in the far pile.  A label accepted
@@ -485,9 +471,7 @@ __device__ __forceinline__ bool offer_with(Ctx &c, int32_t v, float nd, float nd
   const float f = nd + s.hlen;
   if (P.mode == VINE_MODE_OPTIMAL) {
     const uint64_t key = pack_key(f, lb_dl);
-    const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
-    if (key >= inc) return false;
-    if (c.bounds == kBoundsLocal && beyond_mix(st, nd, ndl, s.hmix, inc)) return false;
+    if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) return false;
     if (v == st.dst) {
       sink_improve(c, v, nd, ndl, parent, key);
       return false;
@@ -575,14 +559,14 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
       if (i0 + b * G < n) lab[b] = load_label(&P.pool[idx[b]]);
 #pragma unroll
     for (int b = 0; b < kBatch; ++b)
-      if (i0 + b * G < n && (uint32_t)(lab[b].vid & 0x7fffffff) >= (uint32_t)c.g.n) {
+      if (i0 + b * G < n && (uint32_t)(lab[b].vid & 0x7fffffff) >= (uint32_t)P.g.n) {
         fail_query(st, VINE_ERR_INTERNAL, kSiteRing);
         lab[b].vid = (int)kDeadBit;  // vertex 0, dead: expands nothing
       }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
-      s[b] = VView{0.0f, true, 0.0f, 0.0f, 0u, 0u};
-      if (c.bounds != kBoundsNone && i0 + b * G < n) s[b] = c.view(lab[b].vid & 0x7fffffff);
+      s[b] = VView{0.0f, true, 0.0f, 0.0f, 0u};
+      if (P.use_bounds && i0 + b * G < n) s[b] = c.view(lab[b].vid & 0x7fffffff);
     }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
@@ -596,14 +580,12 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
         if (!(f < hi)) live = false;
         if (live && P.mode == VINE_MODE_OPTIMAL) {
           const uint64_t key = pack_key(f, lab[b].dl + s[b].hdel);
-          const unsigned long long inc = *reinterpret_cast<volatile unsigned long long *>(&st.inc_key);
-          if (key >= inc) live = false;
-          else if (c.bounds == kBoundsLocal && beyond_mix(st, lab[b].d, lab[b].dl, s[b].hmix, inc)) live = false;
+          if (key >= *reinterpret_cast<volatile unsigned long long *>(&st.inc_key)) live = false;
         }
       }
       if (live) {
-        beg = c.g.row[v];  // (not through the read-only path: a local graph is
-        deg = c.g.row[v + 1] - beg;  // written by this kernel)
+        beg = __ldg(&P.g.row[v]);
+        deg = __ldg(&P.g.row[v + 1]) - beg;
         if (deg > 0) warp_agg_inc(&st.r_live);
       }
       rb.idx[i] = idx[b];
@@ -640,8 +622,8 @@ __device__ __forceinline__ void expand_block(Ctx &c, const RoundBuf &rb, uint32_
       if (e < total) {
         const int k = upper_index(rb.off, n, e);
         const int j = rb.beg[k] + (e - rb.off[k]);
-        vv[b] = c.g.col[j];
-        const float2 w = c.g.w[j];
+        vv[b] = __ldg(&P.g.col[j]);
+        const float2 w = __ldg(&P.g.w[j]);
         nd[b] = rb.d[k] + w.x;
         nl[b] = rb.dl[k] + w.y;
         par[b] = rb.idx[k];
@@ -672,7 +654,7 @@ __device__ inline void reverse_expand_block(Ctx &c, const RoundBuf &rb, int whic
   for (int i = sid; i < n; i += G) {
     const int v = (int)c.nearq[(first + (uint32_t)i) & P.near_mask];
     const int beg = __ldg(&P.g.rrow[v]);
-    const VView s = view_vs(&c.vs[v], st.epoch, st.qbase, st.bcur, kBoundsGlobal);
+    const VView s = view_vs(&c.vs[v], st.epoch, st.qbase, st.bcur, true);
     rb.vid[i] = v;
     rb.d[i] = which == 0 ? s.hdel : s.hlen;
     rb.beg[i] = beg;
@@ -724,7 +706,7 @@ __device__ inline void reverse_expand_block(Ctx &c, const RoundBuf &rb, int whic
 
 // Current reverse distance of v in pass `which` (+inf when unset).
 __device__ __forceinline__ float reverse_dist(const Ctx &c, int which, int v) {
-  const VView s = view_vs(&c.vs[v], c.st.epoch, c.st.qbase, c.st.bcur, kBoundsGlobal);
+  const VView s = view_vs(&c.vs[v], c.st.epoch, c.st.qbase, c.st.bcur, true);
   if (which == 0) return __ldcg(&c.vs[v].e_del) == c.st.epoch ? s.hdel : INFINITY;
   return __ldcg(&c.vs[v].e_del) == c.st.epoch ? s.hlen : INFINITY;
 }
