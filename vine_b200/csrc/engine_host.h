@@ -126,6 +126,11 @@ struct vine_mlp {
   float *adam_m = nullptr;
   float *adam_v = nullptr;
   int64_t step = 0;
+  // device memory of the host-buffer calls, kept between them (mlp.cu); calls
+  // on one model take turns
+  mutable std::mutex scratch_mu;
+  mutable char *scratch = nullptr;
+  mutable size_t scratch_cap = 0;
 };
 
 namespace vine {
