@@ -322,6 +322,7 @@ void vine_graph_destroy(vine_graph *g) {
   if (g->stream) cudaStreamSynchronize(g->stream);
   g->batch.release();
   g->plain.release();
+  g->variant.release();
   if (g->io_cache) {
     static_cast<IoCache *>(g->io_cache)->b.release();
     delete static_cast<IoCache *>(g->io_cache);

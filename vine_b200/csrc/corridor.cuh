@@ -88,6 +88,12 @@ struct PassArgs {
   int n, root;
   uint32_t limit;
   uint32_t delta;
+  // whole-graph passes (kWhole): arcs longer than max_len or with less delay
+  // than min_delay are left out, every arc adds `hop` to the key, and with
+  // target >= 0 nothing farther than that vertex is wanted
+  float max_len = INFINITY, min_delay = -INFINITY;
+  uint32_t hop = 0;
+  int target = -1;
 };
 
 // Shared-memory state of the wave searches.  It lies over the bucket table,
@@ -584,7 +590,7 @@ __device__ __forceinline__ void bi_start(WaveShared &W, const DevGraph &g, const
 // vertex is pruned, since what it is charged for the other side, its distance
 // there or the radius of that side, is never more than the truth.
 // W.cur / W.fb: queue and far pile in use.
-__device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, bool to_meeting) {
+static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState &st, bool to_meeting) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   const CorridorMem &M = W.m;
@@ -712,7 +718,7 @@ __device__ __forceinline__ bool build_csr(WaveShared &W, const int32_t *orow, co
 // (og: original ids of its vertices, null for the whole graph).  The new ids
 // of those vertices stay in rf until the next reset.  Returns the vertex count;
 // -1 (nothing copied) when it does not fit or exceeds `most`.
-__device__ __noinline__ int build_local(const int32_t *og, LocalGraph &L, int most) {
+static __device__ __noinline__ int build_local(const int32_t *og, LocalGraph &L, int most) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   const DevGraph &g = W.g;
@@ -772,7 +778,7 @@ struct DistArray {
   }
 };
 
-template <bool kShared>
+template <bool kShared, bool kWhole>
 __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<kShared> &D, int cur,
                                                 int fb, uint32_t i0, uint32_t take) {
   const CorridorMem &M = W.m;
@@ -800,9 +806,11 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
       cand[k] = 0;
       if (on >> k & 1u) {
         const uint32_t ln = (uint32_t)w[k].x, dl = (uint32_t)w[k].y;
-        const unsigned long long nk =
+        unsigned long long nk =
             k0[k] + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
-        if (nk > limit) {
+        if (kWhole) nk += A.hop;
+        if (nk > limit || (kWhole && (w[k].x > A.max_len || w[k].y < A.min_delay))) {
+          if (kWhole && nk > kKeyMax) W.clipped = 1;
           on &= ~(1u << k);
         } else {
           cand[k] = (nk << 32) | add_second(s0[k], c.pure ? ln : dl);
@@ -865,9 +873,8 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
 // Runs a local pass with the whole block; `out` receives the distances.
 // Latency-bound like bi_rounds; a corridor is long and narrow, so most rounds
 // fit one warp and run without block barriers, on shared-memory distances.
-template <bool kShared>
-__device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState &st,
-                                               unsigned long long *out) {
+template <bool kShared, bool kWhole = false, typename Params, typename State>
+static __device__ __noinline__ uint32_t local_pass_in(const Params &P, State &st, unsigned long long *out) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   const CorridorMem &M = W.m;
@@ -900,6 +907,7 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
       if (tid == 0) {
         over_time(P, st);
         if (W.overflow || st.abort) W.stop = 1;
+        if (kWhole && A.target >= 0) W.a.limit = min(A.limit, key_hi(D.get(A.target)));
         W.hi = min(max(W.hi, fm), kKeyMax + 1u - A.delta) + A.delta;
         W.far_min = kNoKey;
         W.nfar[fb ^ 1] = 0;
@@ -922,7 +930,7 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
       if (warp == 0) {
         uint32_t n = nc;
         do {
-          relaxed += local_chunk<kShared>(W, D, cur, fb, 0, n);
+          relaxed += local_chunk<kShared, kWhole>(W, D, cur, fb, 0, n);
           __syncwarp();
           if (lane == 0) {
             W.nq[cur] = 0;
@@ -937,7 +945,7 @@ __device__ __noinline__ uint32_t local_pass_in(const SearchParams &P, QueryState
     } else {
       const uint32_t take = min(32u, (nc + (uint32_t)nw - 1u) / (uint32_t)nw);
       for (uint32_t base = (uint32_t)warp * take; base < nc; base += (uint32_t)nw * take)
-        relaxed += local_chunk<kShared>(W, D, cur, fb, base, min(take, nc - base));
+        relaxed += local_chunk<kShared, kWhole>(W, D, cur, fb, base, min(take, nc - base));
       __syncthreads();
       if (tid == 0) {
         W.nq[cur] = 0;
@@ -1037,7 +1045,7 @@ struct Duals {
 // st.lam_* the multiplier and st.ord_* the order of the search; kCorridorInfeasible: no path within the
 // budget; kCorridorNone: not handled here (costs from 2^24 on, or a corridor
 // past the local capacity).
-__device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &st, int *which) {
+static __device__ __noinline__ int corridor_prepare(const SearchParams &P, QueryState &st, int *which) {
   extern __shared__ __align__(16) unsigned char smem[];
   WaveShared &W = *reinterpret_cast<WaveShared *>(smem);
   CorridorMem &M = W.m;

@@ -87,6 +87,15 @@ struct PlainWorkspace {
   void release();
 };
 
+// Device block of the variant engine, kept between calls (variants.cu).
+struct VariantWorkspace {
+  char *base = nullptr;
+  size_t cap = 0;
+  size_t head_bytes = 0;  // part of the block that holds valid (epoch, label) heads
+  uint32_t epoch_next = 1;
+  void release();
+};
+
 }  // namespace vine
 
 struct vine_graph {
@@ -104,6 +113,7 @@ struct vine_graph {
   std::mutex mu;  // one solve at a time per handle
   vine::BatchWorkspace batch;
   vine::PlainWorkspace plain;
+  vine::VariantWorkspace variant;
   std::vector<float> last_trace;  // host copy of the last trace
   void *io_cache = nullptr;       // device in/out buffers of vine_solve, kept between calls
   vine::DevGraph dev() const {

@@ -480,7 +480,7 @@ __device__ __forceinline__ void batch_block(const SearchParams &P, QueryState &s
 }
 
 // Runs the search set up in SearchShared::s (all threads).  On return st.inc_key / st.inc_idx hold the answer.
-__device__ __noinline__ void wave_search(const SearchParams &P, QueryState &st) {
+static __device__ __noinline__ void wave_search(const SearchParams &P, QueryState &st) {
   extern __shared__ __align__(16) unsigned char smem[];
   SearchShared &Q = *reinterpret_cast<SearchShared *>(smem);
   WaveSearch &S = Q.s;
