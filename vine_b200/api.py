@@ -201,10 +201,14 @@ def solve(graph: Graph, src, dst, budget, config=None, paths: bool = True,
     res.found, res.status = _ptr(r.found), _ptr(r.status)
     if paths:
         cap = path_capacity if path_capacity is not None else max(1024, nq * 64)
+        # Room for 4096 vertices a query (up to 1 GB; zeroed pages that nothing
+        # touches cost nothing): with a buffer of `cap` the queries of long
+        # paths were solved twice, the second time with the size reported.
+        room = cap if path_capacity is not None else max(cap, min(nq * 4096, 1 << 28))
         r.path_offsets = np.zeros(nq + 1, np.int64)
-        r.path_vertices = np.zeros(cap, np.int32)
+        r.path_vertices = np.zeros(room, np.int32)
         res.path_offsets, res.path = _ptr(r.path_offsets), _ptr(r.path_vertices)
-        res.path_capacity = cap
+        res.path_capacity = room
     if pareto_stride > 0:
         r.pareto_d = np.zeros((nq, pareto_stride), np.float32)
         r.pareto_delay = np.zeros((nq, pareto_stride), np.float32)
@@ -220,6 +224,8 @@ def solve(graph: Graph, src, dst, budget, config=None, paths: bool = True,
         # path buffer too small: grow it to the size the library reported, retry once
         return solve(graph, src, dst, budget, config, paths, pareto_stride, stats,
                      path_capacity=int(r.path_offsets[nq]), raise_on_error=raise_on_error)
+    if paths:  # the size it always had: `cap`, or what longer paths need
+        r.path_vertices = r.path_vertices[:max(cap, int(r.path_offsets[nq]))]
     r.rc = rc
     r.retried = int(res.retried)
     if raise_on_error:

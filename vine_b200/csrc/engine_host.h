@@ -202,7 +202,8 @@ int order_queries(int32_t nq, const float *d_budget, int32_t *d_order, cudaStrea
 // Packs the paths of `p` in query order: offsets[q] = exclusive prefix sum of
 // the lengths (offsets[nq] = total), then path[offsets[q] ..] = path of q.
 int path_offsets(const PathOut &p, int32_t nq, int64_t *d_offsets, cudaStream_t stream);
+// At most `cap` vertices are written.
 int path_gather(const PathOut &p, int32_t nq, const int64_t *d_offsets, int32_t *d_path,
-                cudaStream_t stream);
+                int64_t cap, cudaStream_t stream);
 
 }  // namespace vine

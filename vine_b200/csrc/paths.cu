@@ -105,15 +105,16 @@ __global__ void scan_i64_kernel(int64_t *a, int32_t n) {
   if (tid == 0) a[n] = carry;
 }
 
-// One warp per query copies its path segment.
+// One warp per query copies its path segment; nothing is written past `cap`.
 __global__ void path_gather_kernel(const int32_t *arena, const int64_t *start,
                                    const int32_t *len, int32_t nq, const int64_t *off,
-                                   int32_t *path) {
+                                   int32_t *path, int64_t cap) {
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (q >= nq) return;
   const int64_t s = start[q], o = off[q];
-  for (int32_t i = lane; i < len[q]; i += 32) path[o + i] = arena[s + i];
+  for (int32_t i = lane; i < len[q]; i += 32)
+    if (o + i < cap) path[o + i] = arena[s + i];
 }
 
 }  // namespace
@@ -137,10 +138,10 @@ int path_offsets(const PathOut &p, int32_t nq, int64_t *d_offsets, cudaStream_t 
 }
 
 int path_gather(const PathOut &p, int32_t nq, const int64_t *d_offsets, int32_t *d_path,
-                cudaStream_t stream) {
+                int64_t cap, cudaStream_t stream) {
   if (nq <= 0) return VINE_OK;
   path_gather_kernel<<<(nq * 32 + 255) / 256, 256, 0, stream>>>(p.arena, p.start, p.len, nq,
-                                                                 d_offsets, d_path);
+                                                                 d_offsets, d_path, cap);
   VINE_CUDA_TRY(cudaGetLastError());
   return VINE_OK;
 }

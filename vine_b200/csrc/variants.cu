@@ -844,7 +844,7 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
   }
   PathOut paths{P.path_arena, d_pstart, d_plen};
   if (rc == VINE_OK && call.paths) rc = path_offsets(paths, nq, d_off, s);
-  if (rc == VINE_OK && call.paths) rc = path_gather(paths, nq, d_off, d_path, s);
+  if (rc == VINE_OK && call.paths) rc = path_gather(paths, nq, d_off, d_path, path_cap, s);
   if (rc != VINE_OK) {
     cudaStreamSynchronize(s);
     return rc;
