@@ -145,3 +145,29 @@ def test_zero_weights_and_unreachable():
     assert res.found.tolist() == [1, 1, 1, 0, 1]
     assert res.cost[:3].tolist() == [0, 2, 0] and res.delay[:3].tolist() == [0, 0, 4]
     g.close()
+
+
+@pytest.mark.parametrize("name", ["line33", "star257", "layers", "layers_wide", "heavy_arcs"])
+def test_pareto_sets(name):
+    """The sink's Pareto set, of the delay corridor, against the oracle's label setting
+    without cost bounds."""
+    import vine_b200 as v
+    from oracle import oracle as O
+    make, s, t = CASES[name]
+    n, arcs = make(np.random.default_rng(17))
+    csr = _graph(n, arcs)
+    g, og = v.Graph(*csr), O.CsrGraph(*csr)
+    _, h_del = O.lower_bounds(og, t)
+    lo, hi = O.dijkstra(og, s, "delay")[0][t], O.dijkstra(og, s, "len")[1][t]
+    budgets = np.array([lo - 1, lo, lo + 0.3 * (hi - lo), hi, 2 * hi + 10, 2.0 ** 24], np.float32)
+    for cfg in (v.Config(mode="pareto", pool_labels=1 << 24),
+                v.Config(mode="pareto", policy="ar", block_threads=64, table_log2=6, pool_labels=1 << 24)):
+        r = v.solve(g, [s] * len(budgets), [t] * len(budgets), budgets, cfg, pareto_stride=2048)
+        for q, b in enumerate(budgets):
+            want = O.solve_label_setting(og, s, t, float(b), None, h_del, use_incumbent=False)
+            assert bool(r.found[q]) == want["found"] and r.pareto_n[q] == len(want["pareto"]), (q, b)
+            front = want["pareto"]
+            np.testing.assert_array_equal(r.pareto(q), front[np.argsort(front[:, 0])])
+            if want["found"]:
+                assert r.path(q)[0] == s and r.path(q)[-1] == t
+    g.close()

@@ -729,7 +729,7 @@ __device__ __forceinline__ void corridor_mem(const SearchParams &P, int slot, Co
   M.state = P.lstate + (size_t)slot * lv;
 }
 
-// kBounds: the call uses lower bounds (corridors).  Without them the corridor
+// kBounds: the call uses corridors (lower bounds, or a Pareto set).  Without them the corridor
 // code and its state are compiled out: they would cost the plain bucketed
 // search registers (12 % on a 45 x 45 grid with default settings).
 template <bool kBounds>
@@ -912,6 +912,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
               S.state = M.state;
               S.n = L.g.n;
               S.sink = st.dst;
+              S.sinks = P.mode == VINE_MODE_PARETO ? c.sinks : nullptr;
+              S.sink_cap = P.sink_cap;
               S.B = (uint32_t)floorf(st.budget);
               S.a = st.lam_a;
               S.b = st.lam_b;
@@ -943,7 +945,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           for (int i = tid; i < NL; i += G) locks[i] = 0;
           __syncthreads();
         }
-        if (how == kCorridorNone && !st.abort) {
+        if (how == kCorridorNone && P.use_bounds && !st.abort) {
           cta_reverse_search(c, rb, 0, st.budget, P.delta_del);
           cta_reverse_search(c, rb, 1, INFINITY, P.delta_len);
         }
@@ -1265,6 +1267,20 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       // alive sink labels are exactly the sink's Pareto set; rank-sort them
       const uint32_t k = min(st.sink_n, (uint32_t)P.sink_cap);
       __syncthreads();
+      if (kBounds && gid != nullptr) {
+        // waves never kill a label: drop those that a later one dominates
+        for (uint32_t i = tid; i < k; i += G) {
+          const Label a = load_label(&P.pool[c.sinks[i]]);
+          for (uint32_t j = 0; j < k; ++j) {
+            const Label b = load_label(&P.pool[c.sinks[j]]);
+            if (j != i && dominates(b.d, b.dl, a.d, a.dl)) {  // (no two are equal)
+              atomicOr(reinterpret_cast<unsigned int *>(&P.pool[c.sinks[i]].vid), kDeadBit);
+              break;
+            }
+          }
+        }
+        __syncthreads();
+      }
       uint32_t alive_local = 0;
       for (uint32_t i = tid; i < k; i += G) {
         const Label a = load_label(&P.pool[c.sinks[i]]);
@@ -1352,8 +1368,12 @@ size_t batch_smem_bytes(int table_log2, int lock_log2, int round_cap, int block_
 }
 
 using BatchKernel = void (*)(SearchParams);
-BatchKernel kernel_for(const vine_config &c) {
-  return c.use_bounds ? batch_kernel<true> : batch_kernel<false>;
+// Corridors serve calls with bounds and, on integral weights, Pareto sets.
+bool uses_corridors(const vine_graph *g, const vine_config &c) {
+  return c.use_bounds || (c.mode == VINE_MODE_PARETO && g->integral);
+}
+BatchKernel kernel_for(const vine_graph *g, const vine_config &c) {
+  return uses_corridors(g, c) ? batch_kernel<true> : batch_kernel<false>;
 }
 
 int lock_log2_for(int table_log2) { return std::max(5, table_log2 - 1); }
@@ -1394,7 +1414,7 @@ void BatchWorkspace::release() {
 // queries get the two reverse searches over the whole graph.
 static int ensure_corridor(vine_graph *g, const Resolved &r) {
   BatchWorkspace &w = g->batch;
-  if (!r.cfg.use_bounds || w.rf != nullptr) return VINE_OK;
+  if (!uses_corridors(g, r.cfg) || w.rf != nullptr) return VINE_OK;
   const size_t n = (size_t)g->n;
   const size_t lv = std::min<size_t>(n, kCorridorVertices);
   const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
@@ -1500,7 +1520,7 @@ int batch_prepare(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t str
   const size_t smem = batch_smem_bytes(r.cfg.table_log2, lock_log2_for(r.cfg.table_log2),
                                        r.cfg.sync_rounds ? r.round_cap : 0, r.cfg.block_threads,
                                        r.cfg.split_staging);
-  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(r.cfg), cudaFuncAttributeMaxDynamicSharedMemorySize,
+  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(g, r.cfg), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   return VINE_OK;
 }
@@ -1573,7 +1593,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.split_staging = c.split_staging;
   P.wait_limit = c.wait_limit;
   P.time_limit_ns = c.time_limit_ms > 0 ? (unsigned long long)c.time_limit_ms * 1000000ull : 0ull;
-  P.rf = c.use_bounds ? w.rf : nullptr;
+  P.rf = uses_corridors(g, c) ? w.rf : nullptr;
   P.touch = w.touch;
   P.lint = w.lint;
   P.lw = w.lw;
@@ -1600,7 +1620,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   VINE_CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(unsigned long long) * 4, stream));
   epoch_kernel<<<1, 1, 0, stream>>>(w.counters, nq);
   if (c.order_queries) VINE_TRY(order_queries(nq, d_budget, w.order, stream));
-  kernel_for(c)<<<r.slots, c.block_threads, smem, stream>>>(P);
+  kernel_for(g, c)<<<r.slots, c.block_threads, smem, stream>>>(P);
   VINE_CUDA_TRY(cudaGetLastError());
   if (paths) {
     paths->arena = w.path_arena;
@@ -1621,10 +1641,10 @@ int batch_slots(const vine_graph *g, const vine_config &c, int round_cap, int *s
   const size_t smem =
       batch_smem_bytes(c.table_log2, lock_log2_for(c.table_log2), c.sync_rounds ? round_cap : 0,
                        c.block_threads, c.split_staging);
-  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+  VINE_CUDA_TRY(cudaFuncSetAttribute(kernel_for(g, c), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   int per_sm = 0;
-  VINE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_for(c),
+  VINE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel_for(g, c),
                                                               c.block_threads, smem));
   if (per_sm < 1) return fail(VINE_ERR_INVALID, "batch kernel does not fit on an SM with this configuration");
   if (c.ctas_per_sm > 0) per_sm = std::min(per_sm, c.ctas_per_sm);

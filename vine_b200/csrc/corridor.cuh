@@ -1063,7 +1063,10 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
   Duals k{-1.0, 0.0, -1.0, 0.0, -1.0, 0.0};
   double lambda = unit * kFirstLambda;
   int result = kCorridorNone, ne = -1, cl = -1, ls = s, lt = t;  // cl: graph searched (-1: the whole one)
-  bool pure = false;
+  // the Pareto set takes every vertex on a way within the budget: the pure
+  // delay search alone
+  const bool pareto = P.mode == VINE_MODE_PARETO;
+  bool pure = pareto;
   Combo c;
   c.B = B;
   for (int attempt = 0;; ++attempt) {
@@ -1124,7 +1127,7 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
     // A wide gap between T and the meeting key means a poor multiplier:
     // another search now costs less than completing this one.
     const double gap = pure ? 1.0 : ((double)k.T(c) - (double)(mu >> 32)) / fmax(1.0, (double)(mu >> 32));
-    if (attempt >= 4 || settled || cl >= 0 || !(gap > kWideGap)) {
+    if (pareto || attempt >= 4 || settled || cl >= 0 || !(gap > kWideGap)) {
       __syncthreads();
       relaxed += bi_run(P, st, false);
       if (W.stop) break;
@@ -1141,7 +1144,7 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
         cl = to;
         ne = n2;
       }
-      if (settled || attempt >= 6 || (ne >= 0 && ne <= kShrinkTo)) break;
+      if (pareto || settled || attempt >= 6 || (ne >= 0 && ne <= kShrinkTo)) break;
     }
     bi_reset(W, M);
     lambda = next;
@@ -1163,18 +1166,23 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
     PassArgs A{g.rrow, g.rcol, g.rw, ne, lt, B, wide ? combo_delta(P, cd, P.wave_mult) : one};
     relaxed += local_pass(P, st, W, A, cd, D0);
     const unsigned long long xd = __ldcg(&D0[ls]);  // the fastest path
-    if (xd != kUnset) {
+    if (pareto) {
+      // no sink label longer than the fastest path (the shortest of those)
+      // is in the Pareto set
+      k.ub = xd != kUnset ? (double)(uint32_t)xd : (double)kIntLimit;
+      if (k.ub >= (double)kIntLimit) ne = -1;
+    } else if (xd != kUnset) {
       k.feasible((double)(uint32_t)xd, (double)(xd >> 32));
       if (k.len2 < 0.0) {
         k.len2 = (double)(uint32_t)xd;
         k.del2 = (double)(xd >> 32);
       }
     }
-    A.limit = (uint32_t)k.ub;
+    A.limit = ne >= 0 ? (uint32_t)k.ub : 0u;
     A.delta = wide ? combo_delta(P, cl_, P.wave_mult) : one;
     relaxed += local_pass(P, st, W, A, cl_, D1);
     const unsigned long long xl = __ldcg(&D1[ls]);  // the shortest path
-    if (xl != kUnset) {
+    if (xl != kUnset && !pareto) {
       const double l0 = (double)(xl >> 32), d0 = (double)(uint32_t)xl;
       if (d0 <= (double)B) {
         k.feasible(l0, d0);  // the answer's cost

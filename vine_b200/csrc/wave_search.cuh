@@ -38,6 +38,8 @@ struct WaveSearch {
   const float2 *w;
   const uint4 *state;  // per vertex: delay, length, combined distance to the sink
   int n, sink;
+  uint32_t *sinks;       // Pareto mode: arena slots of the sink's kept labels (null otherwise)
+  int sink_cap;
   uint32_t B, a, b, bB;  // budget, pruning multiplier, b * B
   uint32_t pa, pb;       // order
   Label *pool;
@@ -92,19 +94,22 @@ __device__ __forceinline__ bool label_beyond(const WaveSearch &S, const uint4 &h
 // True when a kept label of v has no larger d and no larger delay.  A run is
 // named by its first arena slot i, with the top bit set when it has one
 // label; next[i] is v's previous run, next[i + 1] the length of a longer one.
+// (Plain loads: runs are written once, by this SM, and the candidates of a
+// vertex probe the same few lines, so L1 serves most of them.  Read past L1
+// they took half of a Pareto query's time.)
 __device__ __forceinline__ bool run_dominates(const WaveSearch &S, uint32_t run, uint32_t d, uint32_t dl) {
   while (run != kNone) {
     const uint32_t i = run & 0x7fffffffu;
     int len = 1;
-    const uint32_t before = __ldcg(&S.next[i]);
-    if (!(run & 0x80000000u)) len = (int)__ldcg(&S.next[i + 1]);
+    const uint32_t before = S.next[i];
+    if (!(run & 0x80000000u)) len = (int)S.next[i + 1];
     int lo = 0, hi = len;  // labels [0, lo) have d no larger
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      if ((uint32_t)__ldcg(&S.pool[i + mid].d) <= d) lo = mid + 1;
+      if ((uint32_t)S.pool[i + mid].d <= d) lo = mid + 1;
       else hi = mid;
     }
-    if (lo > 0 && (uint32_t)__ldcg(&S.pool[i + lo - 1].dl) <= dl) return true;
+    if (lo > 0 && (uint32_t)S.pool[i + lo - 1].dl <= dl) return true;
     run = before;
   }
   return false;
@@ -213,7 +218,7 @@ __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearc
         const unsigned long long inc = vol(Q.inc);
         // (a single arc may be as long as 2^24: sums stay below 2^25)
         if (label_beyond(S, h[j], nd, nl, inc)) continue;
-        if (u[j] == S.sink) {
+        if (u[j] == S.sink && S.sinks == nullptr) {
           const unsigned long long c = (unsigned long long)nd << 32 | nl;
           if (c < *best && c < inc) {
             atomicMin(&Q.inc, c);
@@ -288,6 +293,15 @@ __device__ __forceinline__ uint32_t segment_min(uint32_t v, uint32_t dl, uint32_
   return lane > 0 && pv == v ? pm : 0xffffffffu;
 }
 
+// Pareto mode: a kept label of the sink is listed and not expanded.
+__device__ __forceinline__ bool list_sink(QueryState &st, const WaveSearch &S, bool kept, uint32_t v, uint32_t idx) {
+  if (S.sinks == nullptr || !kept || v != (uint32_t)S.sink) return false;
+  const uint32_t k = atomicAdd(&st.sink_n, 1u);
+  if (k < (uint32_t)S.sink_cap) S.sinks[k] = idx;
+  else fail_query(st, VINE_ERR_CAPACITY, kSiteSink);
+  return true;
+}
+
 struct RunCounters {
   uint32_t kept, dominated, relaxed;
 };
@@ -357,7 +371,8 @@ __device__ __forceinline__ void batch_warp(const SearchParams &P, QueryState &st
   __syncwarp();
   unsigned long long best = kUnset;
   uint32_t best_par = 0;
-  C.relaxed += expand_kept(Q, S, kept, k, idx, cur ^ 1, fbuf, &best, &best_par);
+  const bool listed = list_sink(st, S, kept, v, idx);
+  C.relaxed += expand_kept(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
   __syncwarp();
   if (best != kUnset && best == vol(Q.inc)) Q.inc_parent = best_par;
   __syncwarp();
@@ -472,8 +487,9 @@ __device__ __forceinline__ void batch_block(const SearchParams &P, QueryState &s
   }
   unsigned long long best = kUnset;
   uint32_t best_par = 0;
+  const bool listed = list_sink(st, S, kept, v, idx);
   if (warp * 32 < (int)n)
-    C.relaxed += expand_kept(Q, S, kept, k, idx, cur ^ 1, fbuf, &best, &best_par);
+    C.relaxed += expand_kept(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
   __syncthreads();
   if (best != kUnset && best == vol(Q.inc)) Q.inc_parent = best_par;
   __syncthreads();
@@ -660,6 +676,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
     st.n_buckets++;
     if (Q.overflow && !st.abort) fail_query(st, VINE_ERR_CAPACITY, Q.overflow == 1 ? kSiteNear : kSiteBand);
     st.inc_idx = 0xffffffffu;
+    if (S.sinks != nullptr) st.inc_key = ~0ull;  // the cost bound is no answer
     if (!st.abort && Q.inc_parent != kNone) {
       pool_reserve(P, st, 1);
       if (!st.abort) {
