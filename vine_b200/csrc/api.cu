@@ -355,6 +355,8 @@ void vine_graph_destroy(vine_graph *g) {
   cudaFree(g->rrow);
   cudaFree(g->rcol);
   cudaFree(g->rw);
+  cudaFree(g->line);
+  cudaFree(g->rline);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }

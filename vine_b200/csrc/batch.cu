@@ -710,16 +710,19 @@ __device__ __forceinline__ void corridor_mem(const SearchParams &P, int slot, Co
   const size_t lv = (size_t)P.lv, la = (size_t)P.la;
   int32_t *ip = P.lint + (size_t)slot * corridor_ints(P.lv, P.la);
   float2 *wp = P.lw + (size_t)slot * 4 * la;
+  int4 *lp = P.lline + (size_t)slot * 16 * lv;
   for (int k = 0; k < 2; ++k) {
     DevGraph &g = M.loc[k].g;
     g.m = 0;
     g.n = 0;
-    g.row = ip;
-    g.rrow = ip + lv + 1;
-    g.col = ip + 2 * (lv + 1);
-    g.rcol = g.col + la;
-    M.loc[k].gid = const_cast<int32_t *>(g.rcol) + la;
-    ip = M.loc[k].gid + lv;
+    g.row = g.rrow = nullptr;
+    g.line = lp;
+    g.rline = lp + 4 * lv;
+    lp += 8 * lv;
+    g.col = ip;
+    g.rcol = ip + la;
+    M.loc[k].gid = ip + 2 * la;
+    ip += 2 * la + lv;
     g.w = wp;
     g.rw = wp + la;
     wp += 2 * la;
@@ -906,7 +909,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
               const CorridorMem M = W.m;
               const LocalGraph L = M.loc[which];
               WaveSearch &S = reinterpret_cast<SearchShared *>(smem)->s;
-              S.row = L.g.row;
+              S.line = L.g.line;
               S.col = L.g.col;
               S.w = L.g.w;
               S.state = M.state;
@@ -1404,6 +1407,7 @@ void BatchWorkspace::release() {
   cudaFree(lw);
   cudaFree(ldist);
   cudaFree(lstate);
+  cudaFree(lline);
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   *this = BatchWorkspace();
 }
@@ -1420,16 +1424,18 @@ static int ensure_corridor(vine_graph *g, const Resolved &r) {
   const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
   const size_t ints = corridor_ints((int)lv, (int)la);
   const size_t per = n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
-                     lv * (4 * sizeof(unsigned long long) + sizeof(uint4));
+                     lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4));
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   if (per * r.slots > total_b / 8) return VINE_OK;
   const size_t k = (size_t)r.slots;
+  VINE_TRY(ensure_lines(g));
   VINE_CUDA_TRY(cudaMalloc(&w.touch, sizeof(uint32_t) * 2 * n * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * k));
   VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lline, sizeof(int4) * 16 * lv * k));
   VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
   VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
   w.lv = (int)lv;
@@ -1599,6 +1605,7 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.lw = w.lw;
   P.ldist = w.ldist;
   P.lstate = w.lstate;
+  P.lline = w.lline;
   P.lv = w.lv;
   P.la = w.la;
   P.mean_len = g->mean_len;

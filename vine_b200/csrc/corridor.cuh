@@ -43,15 +43,32 @@ constexpr uint32_t kNoKey = 0xffffffffu;
 constexpr uint32_t kMemberTag = 0xfffffffeu;   // rf[v].y high word: v has a local id
 constexpr float kIntLimit = 16777216.0f;       // 2^24: budgets and costs handled here
 constexpr int kWaveQ = 2048;                   // queue entries kept in shared memory
-constexpr int kCorridorVertices = 1 << 16;     // largest local graph
+constexpr int kCorridorVertices = 1 << 15;     // largest local graph
 constexpr double kFirstLambda = 0.5;           // first multiplier, in mean lengths per mean delay
 constexpr double kWideGap = 0.3;               // (T - meeting key) / meeting key worth another multiplier
 constexpr int kShrinkTo = 1024;                // local graphs up to this size are not shrunk further
 constexpr int kHubs = 32;                      // see WaveShared::hub
 constexpr int kHubDegree = 256;
+// A vertex's arc line: 64 bytes with its first four arcs as {head, length,
+// delay, x}, x = the degree in the first and the index of its first arc in
+// (col, w) in the second; heads past the degree are -1.  One read instead of
+// row, then heads and weights: a round of a wave search is a chain of
+// dependent reads, and this takes one of its four out; road vertices
+// seldom have more arcs.
+struct ArcLine {
+  int4 a[4];
+};
+__device__ __forceinline__ ArcLine load_line(const int4 *line, int v) {
+  ArcLine l;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) l.a[k] = line[4 * (size_t)v + k];  // (plain: local lines are written here)
+  return l;
+}
+
 constexpr int kArcBatch = 4;                   // arcs of a vertex whose loads go out together
 
-// A worker's local graph: CSR in both directions and the original ids.
+// A worker's local graph: lines and arcs in both directions (row is not used)
+// and the original ids.
 struct LocalGraph {
   DevGraph g;
   int32_t *gid;
@@ -83,7 +100,8 @@ struct Combo {
 // What a local pass computes: distances from `root` along (row, col, w) under
 // c; keys above `limit` are dropped.
 struct PassArgs {
-  const int32_t *row, *col;
+  const int4 *line;
+  const int32_t *col;
   const float2 *w;
   int n, root;
   uint32_t limit;
@@ -120,9 +138,9 @@ struct __align__(16) WaveShared {
   int scan[kScanScratch];
 };
 
-// 32-bit words of a worker's two local graphs and the renumbering.
+// 32-bit words of a worker's two local graphs (heads, ids) and the renumbering.
 __host__ __device__ constexpr size_t corridor_ints(int lv, int la) {
-  return 2 * (2 * ((size_t)lv + 1) + 2 * (size_t)la + (size_t)lv) + (size_t)lv;
+  return 2 * (2 * (size_t)la + (size_t)lv) + (size_t)lv;
 }
 
 constexpr size_t kWaveBytes = (sizeof(WaveShared) + 15) & ~(size_t)15;
@@ -205,60 +223,71 @@ __device__ __forceinline__ void far_push(WaveShared &W, const CorridorMem &M, in
   atomicMin(&W.far_min, key);
 }
 
+// Slots of the calling warp's flagged entries (bit k of `bits`) in the list
+// behind *ctr: one shared atomic for the warp; pos[k] of a flagged entry.
+template <int K>
+__device__ __forceinline__ void warp_slots(uint32_t *ctr, uint32_t bits, uint32_t (&pos)[K]) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  uint32_t total = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const unsigned b = __ballot_sync(FULL, bits >> k & 1u);
+    pos[k] = total + (uint32_t)__popc(b & below);
+    total += (uint32_t)__popc(b);
+  }
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(ctr, total);
+  base = __shfl_sync(FULL, base, 0);
+#pragma unroll
+  for (int k = 0; k < K; ++k) pos[k] += base;
+}
+
 // Queues what a warp's relaxations improved: entry e[k] with key[k] goes to
-// the next round (bit k of near) or to the far pile (bit k of far); vertices
-// first reached (bit k of first) are listed for their side (bit 0 of e[k])
-// when `sides`.  One shared atomic per list and warp: the lanes' counts are
-// summed as four bytes of one word.  All lanes call.
+// the next round (bit k of near) or to the far pile (bit k of far); vertices first reached (bit k of first) are
+// listed for their side (bit 0 of e[k]) when `sides`.  All lanes call.
 template <int K>
 __device__ __forceinline__ void wave_emit(WaveShared &W, const CorridorMem &M, int nxt, int fb,
                                           const uint32_t (&e)[K], const uint32_t (&key)[K],
                                           uint32_t near, uint32_t far, uint32_t first, bool sides) {
-  static_assert(32 * K < 256, "a warp's counts share bytes of one word");
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  uint32_t f1 = 0;
-  if (sides) {
+  uint32_t pos[K];
+  if (__any_sync(FULL, near)) {
+    warp_slots<K>(&W.nq[nxt], near, pos);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (near >> k & 1u) wave_put(W, M, nxt, pos[k], e[k]);
+  }
+  if (__any_sync(FULL, far)) {
+    warp_slots<K>(&W.nfar[fb], far, pos);
+    uint32_t least = kNoKey;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (far >> k & 1u) {
+        if (pos[k] < M.far_cap) M.far[fb][pos[k]] = ((unsigned long long)key[k] << 32) | e[k];
+        else W.overflow = 1;
+        least = min(least, key[k]);
+      }
+    least = __reduce_min_sync(FULL, least);
+    if ((threadIdx.x & 31) == 0) atomicMin(&W.far_min, least);
+  }
+  if (sides && __any_sync(FULL, first)) {
+    uint32_t f1 = 0;
 #pragma unroll
     for (int k = 0; k < K; ++k) f1 |= (first >> k & 1u & e[k]) << k;
-  }
-  const uint32_t f0 = sides ? first & ~f1 : 0u;
-  const uint32_t mine = (uint32_t)__popc(near) | (uint32_t)__popc(far) << 8 |
-                        (uint32_t)__popc(f0) << 16 | (uint32_t)__popc(f1) << 24;
-  if (!__any_sync(FULL, mine != 0u)) return;
-  uint32_t incl = mine;
+    if (__any_sync(FULL, first & ~f1)) {
+      warp_slots<K>(&W.ntouch[0], first & ~f1, pos);
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
-  }
-  const uint32_t total = __shfl_sync(FULL, incl, 31), excl = incl - mine;
-  uint32_t base = 0;  // lane l < 4 reserves in list l
-  if (lane < 4) {
-    const uint32_t n = total >> (8 * lane) & 255u;
-    uint32_t *ctr = lane == 0 ? &W.nq[nxt] : lane == 1 ? &W.nfar[fb] : &W.ntouch[lane - 2];
-    if (n) base = atomicAdd(ctr, n);
-  }
-  uint32_t pn = __shfl_sync(FULL, base, 0) + (excl & 255u);
-  uint32_t pf = __shfl_sync(FULL, base, 1) + (excl >> 8 & 255u);
-  uint32_t p0 = __shfl_sync(FULL, base, 2) + (excl >> 16 & 255u);
-  uint32_t p1 = __shfl_sync(FULL, base, 3) + (excl >> 24);
-  uint32_t least = kNoKey;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (near >> k & 1u) wave_put(W, M, nxt, pn++, e[k]);
-    if (far >> k & 1u) {
-      if (pf < M.far_cap) M.far[fb][pf] = ((unsigned long long)key[k] << 32) | e[k];
-      else W.overflow = 1;
-      ++pf;
-      least = min(least, key[k]);
+      for (int k = 0; k < K; ++k)
+        if ((first & ~f1) >> k & 1u) M.touch[0][pos[k]] = e[k] >> 1;
     }
-    if (f0 >> k & 1u) M.touch[0][p0++] = e[k] >> 1;
-    if (f1 >> k & 1u) M.touch[1][p1++] = e[k] >> 1;
-  }
-  if (total >> 8 & 255u) {
-    least = __reduce_min_sync(FULL, least);
-    if (lane == 0) atomicMin(&W.far_min, least);
+    if (__any_sync(FULL, f1)) {
+      warp_slots<K>(&W.ntouch[1], f1, pos);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (f1 >> k & 1u) M.touch[1][pos[k]] = e[k] >> 1;
+    }
   }
 }
 
@@ -292,8 +321,8 @@ __device__ __forceinline__ void meet(WaveShared &W, const Combo &c, unsigned lon
 // side side[k] (0 from the source, 1 from the sink) where bit k of `on` is set.  The
 // pair reads go out together, then the atomics.  All lanes call.
 template <int K>
-__device__ __forceinline__ void bi_relax(WaveShared &W, const CorridorMem &M, const Combo &c,
-                                         uint32_t on, const int (&u)[K],
+__device__ __forceinline__ void bi_relax(WaveShared &W, const CorridorMem &M,
+                                         const Combo &c, uint32_t on, const int (&u)[K],
                                          const unsigned long long (&nk)[K], const uint32_t (&ns)[K],
                                          uint32_t side, uint32_t hi, uint32_t rdone, uint32_t limit,
                                          int nxt, int fb) {
@@ -367,14 +396,15 @@ __device__ __forceinline__ uint32_t bi_chunk(const DevGraph &g, WaveShared &W, c
   const uint32_t hi = vol(W.hi), rdone = vol(W.rdone), limit = combo_limit(W, c);
   int beg = 0, deg = 0;
   uint32_t key = 0, sec = 0, side = 0;
+  ArcLine line;
   if ((uint32_t)lane < take) {
     const uint32_t e = wave_get(W, M, cur, i0 + (uint32_t)lane);
     const int v = (int)(e >> 1);
     side = e & 1u;
     const ulonglong2 pv = ld_pair(&M.rf[v]);
-    const int32_t *row = side ? g.rrow : g.row;
-    beg = row[v];
-    deg = row[v + 1] - beg;
+    line = load_line(side ? g.rline : g.line, v);
+    deg = line.a[0].w;
+    beg = line.a[1].w;
     const unsigned long long mine = side ? pv.y : pv.x, other = side ? pv.x : pv.y;
     if (other != kUnset) meet(W, c, mine, other);
     key = key_hi(mine);
@@ -391,23 +421,15 @@ __device__ __forceinline__ uint32_t bi_chunk(const DevGraph &g, WaveShared &W, c
   unsigned long long nk[kArcBatch];
   uint32_t ns[kArcBatch];
   {
-    const int32_t *col = side ? g.rcol : g.col;
-    const float2 *wt = side ? g.rw : g.w;
-    float2 w[kArcBatch];
     uint32_t on = 0;
 #pragma unroll
     for (int k = 0; k < kArcBatch; ++k)
       if (k < deg) {
-        u[k] = col[beg + k];
-        w[k] = wt[beg + k];
-        on |= 1u << k;
-      }
-#pragma unroll
-    for (int k = 0; k < kArcBatch; ++k)
-      if (k < deg) {
-        const uint32_t ln = (uint32_t)w[k].x, dl = (uint32_t)w[k].y;
+        const uint32_t ln = (uint32_t)line.a[k].y, dl = (uint32_t)line.a[k].z;
+        u[k] = line.a[k].x;
         nk[k] = key + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
         ns[k] = add_second(sec, c.pure ? ln : dl);
+        on |= 1u << k;
       }
     bi_relax<kArcBatch>(W, M, c, on, u, nk, ns, side ? 0xfu : 0u, hi, rdone, limit, nxt, fb);
   }
@@ -463,12 +485,13 @@ __device__ __forceinline__ uint32_t bi_hubs(const DevGraph &g, WaveShared &W, co
     const uint32_t e = W.hub[h], side = e & 1u;
     const int v = (int)(e >> 1);
     const ulonglong2 pv = ld_pair(&M.rf[v]);
-    const int32_t *row = side ? g.rrow : g.row, *col = side ? g.rcol : g.col;
+    const int4 *line = (side ? g.rline : g.line) + 4 * (size_t)v;
+    const int32_t *col = side ? g.rcol : g.col;
     const float2 *wt = side ? g.rw : g.w;
     const unsigned long long mine = side ? pv.y : pv.x;
     const uint32_t key = key_hi(mine), sec = (uint32_t)mine;
-    const int end = row[v + 1];
-    for (int j0 = row[v] + warp * 32 * kArcBatch; j0 < end; j0 += nw * 32 * kArcBatch) {
+    const int first = line[1].w, end = first + line[0].w;
+    for (int j0 = first + warp * 32 * kArcBatch; j0 < end; j0 += nw * 32 * kArcBatch) {
       int u[kArcBatch];
       unsigned long long nk[kArcBatch];
       uint32_t ns[kArcBatch], on = 0;
@@ -640,36 +663,51 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
 
 // ---------------------------------------------------------------- local CSR
 
-// One direction of a renumbered CSR: vertex i is old_of(i) of the old graph,
-// arcs to vertices without a new id (new_of < 0) are left out.  False when
-// the arcs do not fit (all threads agree).
+// One direction of a renumbered graph: vertex i is old_of(i) of the old graph,
+// arcs to vertices without a new id (new_of < 0) are left out.  Arcs of
+// vertices with more than a line holds go to (col, w) as well.  False when
+// they do not fit (all threads agree).
 template <typename OldOf, typename NewOf>
-__device__ __forceinline__ bool build_csr(WaveShared &W, const int32_t *orow, const int32_t *ocol,
+__device__ __forceinline__ bool build_csr(WaveShared &W, const int4 *oline, const int32_t *ocol,
                                           const float2 *ow, int ne, OldOf old_of, NewOf new_of,
-                                          int32_t *row, int32_t *col, float2 *w, int cap) {
-  constexpr int kKeep = 6;  // arcs of a vertex whose new ids stay in registers
+                                          int4 *line, int32_t *col, float2 *w, int cap) {
   const unsigned FULL = 0xffffffffu;
   const int G = blockDim.x, tid = threadIdx.x, lane = tid & 31;
   int run = 0;
   for (int base = 0; base < ne; base += G) {
     const int i = base + tid;
-    int beg = 0, deg = 0, cnt = 0;
-    int nid[kKeep];
+    int beg = 0, deg = 0, cnt = 0, large = 0;
     if (i < ne) {
-      const int v = old_of(i);
-      beg = orow[v];
-      deg = orow[v + 1] - beg;
+      ArcLine o = load_line(oline, old_of(i));
+      deg = o.a[0].w;
+      beg = o.a[1].w;
+      if (deg <= 4) {
+        int nid[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) nid[k] = k < deg ? new_of(o.a[k].x) : -1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          o.a[k].x = nid[k];
+          cnt += nid[k] >= 0;
+        }
+        // the kept arcs move to the front (four elements: three passes)
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if (o.a[k].x < 0) {
+              const int4 t = o.a[k];
+              o.a[k] = o.a[k + 1];
+              o.a[k + 1] = t;
+            }
+        o.a[0].w = cnt;
+        o.a[1].w = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) line[4 * (size_t)i + k] = o.a[k];
+      }
     }
-    const bool wide = deg > kKeep;
-    if (!wide) {
-#pragma unroll
-      for (int k = 0; k < kKeep; ++k) nid[k] = k < deg ? ocol[beg + k] : -1;
-#pragma unroll
-      for (int k = 0; k < kKeep; ++k) nid[k] = k < deg ? new_of(nid[k]) : -1;
-#pragma unroll
-      for (int k = 0; k < kKeep; ++k) cnt += nid[k] >= 0;
-    }
-    const unsigned wm = __ballot_sync(FULL, wide);
+    // wider vertices, one after the other by their warp: count, then write
+    const unsigned wm = __ballot_sync(FULL, deg > 4);
     for (unsigned m = wm; m; m &= m - 1) {
       const int l = __ffs(m) - 1;
       const int b = __shfl_sync(FULL, beg, l), e = b + __shfl_sync(FULL, deg, l);
@@ -678,38 +716,38 @@ __device__ __forceinline__ bool build_csr(WaveShared &W, const int32_t *orow, co
       n = __reduce_add_sync(FULL, n);
       if (lane == l) cnt = n;
     }
-    int total;
-    int at = run + block_scan_one(cnt, W.scan, &total);
-    run += total;
-    if (run > cap) return false;
-    if (i < ne) row[i] = at;
-    if (!wide) {
-#pragma unroll
-      for (int k = 0; k < kKeep; ++k)
-        if (nid[k] >= 0) {
-          col[at] = nid[k];
-          w[at] = ow[beg + k];
-          ++at;
-        }
+    if (deg > 4 && cnt > 4) large = cnt;
+    int at = 0;
+    if (__syncthreads_or((int)wm)) {
+      int total;
+      at = run + block_scan_one(large, W.scan, &total);
+      run += total;
+      if (run > cap) return false;
     }
     for (unsigned m = wm; m; m &= m - 1) {
       const int l = __ffs(m) - 1;
       const int b = __shfl_sync(FULL, beg, l), e = b + __shfl_sync(FULL, deg, l);
-      int to = __shfl_sync(FULL, at, l);
+      const int to = __shfl_sync(FULL, at, l), n = __shfl_sync(FULL, cnt, l), v = __shfl_sync(FULL, i, l);
+      int put = 0;
       for (int j0 = b; j0 < e; j0 += 32) {
         const int j = j0 + lane;
         const int id = j < e ? new_of(ocol[j]) : -1;
         const unsigned hit = __ballot_sync(FULL, id >= 0);
         if (id >= 0) {
-          const int p = to + __popc(hit & ((1u << lane) - 1u));
-          col[p] = id;
-          w[p] = ow[j];
+          const int p = put + __popc(hit & ((1u << lane) - 1u));
+          const float2 x = ow[j];
+          if (n > 4) {
+            col[to + p] = id;
+            w[to + p] = x;
+          }
+          if (p < 4) line[4 * (size_t)v + p] = make_int4(id, (int)x.x, (int)x.y, p == 0 ? n : p == 1 ? to : 0);
         }
-        to += __popc(hit);
+        put += __popc(hit);
       }
+      if (lane >= put && lane < 4) line[4 * (size_t)v + lane] = make_int4(-1, 0, 0, 0);
+      if (lane == 0 && n == 0) line[4 * (size_t)v].w = 0;
     }
   }
-  if (tid == 0) row[ne] = run;
   __syncthreads();
   return true;
 }
@@ -752,10 +790,10 @@ static __device__ __noinline__ int build_local(const int32_t *og, LocalGraph &L,
     const unsigned long long h = __ldcg(reinterpret_cast<const unsigned long long *>(&rf[v]) + 1);
     return key_hi(h) == kMemberTag ? (int)(uint32_t)h : -1;
   };
-  if (!build_csr(W, g.row, g.col, g.w, ne, old_of, new_of, const_cast<int32_t *>(L.g.row),
+  if (!build_csr(W, g.line, g.col, g.w, ne, old_of, new_of, const_cast<int4 *>(L.g.line),
                  const_cast<int32_t *>(L.g.col), const_cast<float2 *>(L.g.w), M.la))
     return -1;
-  if (!build_csr(W, g.rrow, g.rcol, g.rw, ne, old_of, new_of, const_cast<int32_t *>(L.g.rrow),
+  if (!build_csr(W, g.rline, g.rcol, g.rw, ne, old_of, new_of, const_cast<int4 *>(L.g.rline),
                  const_cast<int32_t *>(L.g.rcol), const_cast<float2 *>(L.g.rw), M.la))
     return -1;
   if (tid == 0) L.g.n = ne;
@@ -789,15 +827,17 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
   const uint32_t hi = vol(W.hi), limit = A.limit;
   int beg = 0, deg = 0;
   uint32_t key = 0, sec = 0;
+  ArcLine line;
   if ((uint32_t)lane < take) {
     const int v = (int)wave_get(W, M, cur, i0 + (uint32_t)lane);
     const unsigned long long x = D.get(v);
-    beg = A.row[v];
-    deg = A.row[v + 1] - beg;
+    line = load_line(A.line, v);
+    deg = line.a[0].w;
+    beg = line.a[1].w;
     key = key_hi(x);
     sec = (uint32_t)x;
   }
-  auto relax = [&](uint32_t on, const int (&u)[kArcBatch], const float2 (&w)[kArcBatch],
+  auto relax = [&](uint32_t on, const int (&u)[kArcBatch], const int2 (&w)[kArcBatch],
                    const uint32_t (&k0)[kArcBatch], const uint32_t (&s0)[kArcBatch]) {
     unsigned long long cand[kArcBatch], old[kArcBatch];
     uint32_t e[kArcBatch], nkey[kArcBatch], near = 0, far = 0;
@@ -809,7 +849,7 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
         unsigned long long nk =
             k0[k] + (unsigned long long)c.a * ln + (unsigned long long)c.b * dl;
         if (kWhole) nk += A.hop;
-        if (nk > limit || (kWhole && (w[k].x > A.max_len || w[k].y < A.min_delay))) {
+        if (nk > limit || (kWhole && ((float)w[k].x > A.max_len || (float)w[k].y < A.min_delay))) {
           if (kWhole && nk > kKeyMax) W.clipped = 1;
           on &= ~(1u << k);
         } else {
@@ -833,15 +873,15 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
     wave_emit<kArcBatch>(W, M, nxt, fb, e, nkey, near, far, 0u, false);
   };
   int u[kArcBatch];
-  float2 w[kArcBatch];
+  int2 w[kArcBatch];
   uint32_t k0[kArcBatch], s0[kArcBatch], on = 0;
 #pragma unroll
   for (int k = 0; k < kArcBatch; ++k) {
     k0[k] = key;
     s0[k] = sec;
     if (k < deg) {
-      u[k] = A.col[beg + k];
-      w[k] = A.w[beg + k];
+      u[k] = line.a[k].x;
+      w[k] = make_int2(line.a[k].y, line.a[k].z);
       on |= 1u << k;
     }
   }
@@ -859,8 +899,9 @@ __device__ __forceinline__ uint32_t local_chunk(WaveShared &W, const DistArray<k
         k0[k] = ok;
         s0[k] = os;
         if (j < e0) {
+          const float2 x = A.w[j];
           u[k] = A.col[j];
-          w[k] = A.w[j];
+          w[k] = make_int2((int)x.x, (int)x.y);
           on |= 1u << k;
         }
       }
@@ -1163,7 +1204,7 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
     const bool wide = ne > 4096;  // one bucket on small graphs
     const uint32_t one = 0x40000000u;
     Combo cd{0u, 1u, true, B}, cl_{1u, 0u, false, B};
-    PassArgs A{g.rrow, g.rcol, g.rw, ne, lt, B, wide ? combo_delta(P, cd, P.wave_mult) : one};
+    PassArgs A{g.rline, g.rcol, g.rw, ne, lt, B, wide ? combo_delta(P, cd, P.wave_mult) : one};
     relaxed += local_pass(P, st, W, A, cd, D0);
     const unsigned long long xd = __ldcg(&D0[ls]);  // the fastest path
     if (pareto) {

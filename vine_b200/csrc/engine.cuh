@@ -132,6 +132,9 @@ struct DevGraph {
   const int32_t *rrow; // reverse CSR (in-arcs)
   const int32_t *rcol;
   const float2 *rw;
+  // arc lines (corridor.cuh), on graphs with integral weights
+  const int4 *line;
+  const int4 *rline;
 };
 
 // ------------------------------------------------------------------ helpers

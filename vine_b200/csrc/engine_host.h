@@ -54,6 +54,7 @@ struct BatchWorkspace {
   float2 *lw = nullptr;
   unsigned long long *ldist = nullptr;
   uint4 *lstate = nullptr;
+  int4 *lline = nullptr;
   int lv = 0, la = 0;
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape
@@ -108,6 +109,7 @@ struct vine_graph {
   float mean_delay = 1.0f;
   int32_t *row = nullptr, *col = nullptr, *rrow = nullptr, *rcol = nullptr;
   float2 *w = nullptr, *rw = nullptr;
+  int4 *line = nullptr, *rline = nullptr;  // arc lines, made when first needed
   uint64_t fingerprint = 0;
   cudaStream_t stream = nullptr;
   std::mutex mu;  // one solve at a time per handle
@@ -126,6 +128,8 @@ struct vine_graph {
     g.rrow = rrow;
     g.rcol = rcol;
     g.rw = rw;
+    g.line = line;
+    g.rline = rline;
     return g;
   }
 };
@@ -178,6 +182,9 @@ struct Resolved {
 };
 
 int resolve_config(const vine_graph *g, const vine_config *in, Resolved *out);
+
+// Makes the graph's arc lines (integral weights only) unless it has them.
+int ensure_lines(vine_graph *g);
 
 // Batch engine: solves nq queries whose inputs are on the device.
 int batch_run(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d_src,

@@ -117,7 +117,40 @@ __global__ void path_gather_kernel(const int32_t *arena, const int64_t *start,
     if (o + i < cap) path[o + i] = arena[s + i];
 }
 
+// One thread a vertex writes its arc line (corridor.cuh).
+__global__ void line_kernel(int32_t n, const int32_t *row, const int32_t *col, const float2 *w, int4 *line) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n) return;
+  const int beg = row[v], deg = row[v + 1] - beg;
+  for (int k = 0; k < 4; ++k) {
+    int4 a = make_int4(-1, 0, 0, k == 0 ? deg : k == 1 ? beg : 0);
+    if (k < deg) {
+      const float2 x = w[beg + k];
+      a.x = col[beg + k];
+      a.y = (int)x.x;
+      a.z = (int)x.y;
+    }
+    line[4 * (size_t)v + k] = a;
+  }
+}
+
 }  // namespace
+
+int ensure_lines(vine_graph *g) {
+  if (g->line) return VINE_OK;
+  const size_t bytes = sizeof(int4) * 4 * (size_t)g->n;
+  if (cudaMalloc(&g->rline, bytes) != cudaSuccess || cudaMalloc(&g->line, bytes) != cudaSuccess) {
+    cudaFree(g->rline);
+    g->rline = g->line = nullptr;
+    return fail(VINE_ERR_CUDA, "arc lines: allocation failed");
+  }
+  const int blocks = (g->n + 255) / 256;
+  line_kernel<<<blocks, 256>>>(g->n, g->row, g->col, g->w, g->line);
+  line_kernel<<<blocks, 256>>>(g->n, g->rrow, g->rcol, g->rw, g->rline);
+  VINE_CUDA_TRY(cudaGetLastError());
+  VINE_CUDA_TRY(cudaStreamSynchronize(0));  // any stream may use them from here on
+  return VINE_OK;
+}
 
 int order_queries(int32_t nq, const float *d_budget, int32_t *d_order, cudaStream_t stream) {
   if (nq <= 0) return VINE_OK;

@@ -95,8 +95,9 @@ struct SearchParams {
   // corridor of a query (batch engine with bounds; null rf = not used)
   ulonglong2 *rf;
   uint32_t *touch;
-  int32_t *lint;   // local graphs: rows, heads, ids, renumbering
+  int32_t *lint;   // local graphs: heads, ids, renumbering
   float2 *lw;
+  int4 *lline;
   unsigned long long *ldist;
   uint4 *lstate;
   int lv, la;

@@ -325,7 +325,7 @@ __device__ void query_bounds(const VParams &P, VState &st, uint32_t *near, uint3
     W.m.far[1] = W.m.far[0] + W.m.far_cap;
   }
   PassArgs A;
-  A.row = P.g.rrow;
+  A.line = P.g.rline;
   A.col = P.g.rcol;
   A.w = P.g.rw;
   A.n = P.g.n;
@@ -727,6 +727,7 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
   // bounds: integral weights, and their arrays at most a sixteenth of the memory
   const bool bounds = g->integral && n * slots * 3 * sizeof(unsigned long long) <= total_b / 16;
   const int64_t path_cap = std::max<int64_t>((int64_t)nq * 4096, 1 << 20);
+  if (bounds) VINE_TRY(ensure_lines(g));
 
   VParams P;
   std::memset(&P, 0, sizeof(P));

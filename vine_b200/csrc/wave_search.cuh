@@ -34,7 +34,8 @@ constexpr int kWaveGroup = 16;  // waves between two decisions of the bucket pol
 
 // Everything a wave search reads (the arrays are the worker's).
 struct WaveSearch {
-  const int32_t *row, *col;
+  const int4 *line;
+  const int32_t *col;
   const float2 *w;
   const uint4 *state;  // per vertex: delay, length, combined distance to the sink
   int n, sink;
@@ -158,33 +159,24 @@ __device__ __forceinline__ void label_emit(SearchShared &Q, const WaveSearch &S,
                                            const unsigned long long (&key)[K], const uint32_t (&p)[K],
                                            uint32_t par, uint32_t near, uint32_t far) {
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const uint32_t mine = (uint32_t)__popc(near) | (uint32_t)__popc(far) << 16;
-  if (!__any_sync(FULL, mine != 0u)) return;
-  uint32_t incl = mine;
+  uint32_t pos[K];
+  if (__any_sync(FULL, near)) {
+    warp_slots<K>(&Q.nn[nxt], near, pos);
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
+    for (int k = 0; k < K; ++k)
+      if (near >> k & 1u) near_put(Q, S, nxt, pos[k], key[k], par);
   }
-  const uint32_t total = __shfl_sync(FULL, incl, 31), excl = incl - mine;
-  uint32_t base = 0;
-  if (lane == 0 && (total & 0xffffu)) base = atomicAdd(&Q.nn[nxt], total & 0xffffu);
-  if (lane == 1 && (total >> 16)) base = atomicAdd(&Q.nf[fbuf], total >> 16);
-  uint32_t pn = __shfl_sync(FULL, base, 0) + (excl & 0xffffu);
-  uint32_t pf = __shfl_sync(FULL, base, 1) + (excl >> 16);
-  uint32_t least = kNoKey;
+  if (__any_sync(FULL, far)) {
+    warp_slots<K>(&Q.nf[fbuf], far, pos);
+    uint32_t least = kNoKey;
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (near >> k & 1u) near_put(Q, S, nxt, pn++, key[k], par);
-    if (far >> k & 1u) {
-      far_put(Q, S, fbuf, pf++, key[k], par, p[k]);
-      least = min(least, p[k]);
-    }
-  }
-  if (total >> 16) {
+    for (int k = 0; k < K; ++k)
+      if (far >> k & 1u) {
+        far_put(Q, S, fbuf, pos[k], key[k], par, p[k]);
+        least = min(least, p[k]);
+      }
     least = __reduce_min_sync(FULL, least);
-    if (lane == 0) atomicMin(&Q.far_min, least);
+    if ((threadIdx.x & 31) == 0) atomicMin(&Q.far_min, least);
   }
 }
 
@@ -198,12 +190,13 @@ __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearc
   const uint32_t hi = vol(Q.hi);
   int beg = 0, deg = 0;
   const uint32_t d = key_cost(k), dl = key_delay(k);
+  ArcLine line;
   if (kept) {
-    const int v = (int)key_vertex(k);
-    beg = S.row[v];
-    deg = S.row[v + 1] - beg;
+    line = load_line(S.line, (int)key_vertex(k));
+    deg = line.a[0].w;
+    beg = line.a[1].w;
   }
-  auto go = [&](uint32_t on, const int (&u)[kArcBatch], const float2 (&w)[kArcBatch], uint32_t d0, uint32_t dl0,
+  auto go = [&](uint32_t on, const int (&u)[kArcBatch], const int2 (&w)[kArcBatch], uint32_t d0, uint32_t dl0,
                 uint32_t par) {
     unsigned long long key[kArcBatch];
     uint32_t p[kArcBatch], near = 0, far = 0;
@@ -235,13 +228,13 @@ __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearc
     label_emit<kArcBatch>(Q, S, nxt, fbuf, key, p, par, near, far);
   };
   int u[kArcBatch];
-  float2 w[kArcBatch];
+  int2 w[kArcBatch];
   uint32_t on = 0;
 #pragma unroll
   for (int j = 0; j < kArcBatch; ++j)
     if (j < deg) {
-      u[j] = S.col[beg + j];
-      w[j] = S.w[beg + j];
+      u[j] = line.a[j].x;
+      w[j] = make_int2(line.a[j].y, line.a[j].z);
       on |= 1u << j;
     }
   go(on, u, w, d, dl, idx);
@@ -256,8 +249,9 @@ __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearc
       for (int j = 0; j < kArcBatch; ++j) {
         const int e = j0 + 32 * j + lane;
         if (e < e0) {
+          const float2 x = S.w[e];
           u[j] = S.col[e];
-          w[j] = S.w[e];
+          w[j] = make_int2((int)x.x, (int)x.y);
           on |= 1u << j;
         }
       }
