@@ -426,10 +426,7 @@ int vine_solve_device(vine_graph *g, int32_t nq, const int32_t *src, const int32
   key = fnv1a(key, &r.cfg, sizeof(r.cfg));
   key = fnv1a(key, &r.width0, sizeof(r.width0));
   if (w.graph_exec == nullptr || w.graph_key != key) {
-    if (w.graph_exec) {
-      cudaGraphExecDestroy(w.graph_exec);
-      w.graph_exec = nullptr;
-    }
+    w.drop_graph();
     VINE_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     const int st = enqueue();
     cudaGraph_t graph = nullptr;

@@ -151,6 +151,7 @@ __device__ void cta_reverse_search(Ctx &c, const RoundBuf &rb, int which, float 
 // `pending` counts queued labels whose expansion is not finished: children
 // are counted before their parent is uncounted, so pending == 0 with nothing
 // left to take means the bucket is finished.  Every wait is bounded.
+constexpr int kMostShare = 4;    // see share_of
 constexpr uint32_t kSlab = 1024;  // arena slots a warp takes at a time
 
 // Publishes ring entries [base, base + k) once every earlier reservation is
@@ -815,7 +816,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
         st.q = -1;  // a tile buffer may still be written: take no further query
       } else {
         const unsigned long long k = atomicAdd(P.queue, 1ull);
-        st.q = (k < (unsigned long long)P.nq) ? (P.order ? P.order[k] : (int)k) : -1;
+        const unsigned long long nq = P.nq_dev ? *P.nq_dev : (unsigned long long)P.nq;
+        st.q = (k < nq) ? (P.order ? P.order[k] : (int)k) : -1;
       }
     }
     __syncthreads();
@@ -946,6 +948,10 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           // the bucket table lay under the wave state
           for (int i = tid; i < H; i += G) tv[i] = kEmpty;
           for (int i = tid; i < NL; i += G) locks[i] = 0;
+          __syncthreads();
+        }
+        if (how == kCorridorNone && P.redo != nullptr) {
+          if (tid == 0 && !st.abort) fail_query(st, VINE_ERR_CAPACITY, kSiteNear);  // listed in redo below
           __syncthreads();
         }
         if (how == kCorridorNone && P.use_bounds && !st.abort) {
@@ -1311,7 +1317,9 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       atomicAdd(&st.sink_n, alive_local);
     }
     __syncthreads();
-    if (tid == 0) {
+    if (kBounds && P.redo != nullptr && st.abort == VINE_ERR_CAPACITY) {
+      if (tid == 0) P.redo[atomicAdd(P.redo_n, 1ull)] = q;
+    } else if (tid == 0) {
       // a corridor seeds inc_key with its cost bound before a label has it
       const bool ok = st.abort == 0;
       const bool found = ok && st.inc_key != ~0ull && st.inc_idx != 0xffffffffu;
@@ -1358,7 +1366,12 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
 __global__ void epoch_kernel(unsigned long long *counters, int32_t nq) {
   counters[5] = counters[4];
   counters[4] += (unsigned long long)nq;
+  counters[6] = 0;
 }
+
+// Between the two launches of a call with bounds: the second one has the whole
+// arena and its own queue.
+__global__ void redo_kernel(unsigned long long *counters) { counters[0] = counters[1] = 0; }
 
 size_t batch_smem_bytes(int table_log2, int lock_log2, int round_cap, int block_threads,
                         int staging) {
@@ -1380,6 +1393,32 @@ BatchKernel kernel_for(const vine_graph *g, const vine_config &c) {
 }
 
 int lock_log2_for(int table_log2) { return std::max(5, table_log2 - 1); }
+
+// Calls with bounds run in two launches: one for the corridors, then one in the
+// call's own configuration for the queries that have none or did not fit
+// (listed by the first; where there are none it takes a few microseconds).
+// The corridor launch has a smaller table: the searches keep little in shared
+// memory and the L1 cache gets the rest (96 queries on a 264,000-vertex road
+// network: 31.0 ms with 2^13 slots, 28.9 ms with 2^11; 96 on a 150 x 150 grid
+// with anti-correlated weights 7.7 and 7.2 ms).
+constexpr int kCorridorTable = 11;
+bool two_launches(const vine_graph *g, const Resolved &r) {
+  return r.cfg.use_bounds && r.cfg.ctas_per_sm == 0 && r.cfg.max_workers == 0 && !r.cfg.sync_rounds &&
+         r.slots == g->sm_count;
+}
+
+// Workers an SM in the corridor launch, each with its share of one worker's
+// threads and piles.  A corridor search waits most of its time, on chains of
+// dependent reads and on barriers, with few vertices to a round: further workers fill
+// the gaps, but each one is slower, so that the call's longest query ends later.  One, two
+// and four on the road network: 55 / 64 / 83 ms for 600 queries,
+// 90 / 69 / 98 ms for 1,200, 169 / 114 / 110 ms for 2,400 and 295 / 185 /
+// 153 ms for 4,096; on the anti-correlated grid 8.1 / 8.3 / 9.0 ms for 300 and
+// 21 / 12 / 11 ms for 1,200.
+int share_of(const vine_graph *g, const Resolved &r, int32_t nq) {
+  if (!two_launches(g, r)) return 1;
+  return nq > 16 * r.slots ? 4 : nq > 5 * r.slots ? 2 : 1;
+}
 
 }  // namespace
 
@@ -1408,17 +1447,46 @@ void BatchWorkspace::release() {
   cudaFree(ldist);
   cudaFree(lstate);
   cudaFree(lline);
-  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  cudaFree(redo);
+  drop_graph();
   *this = BatchWorkspace();
+}
+
+void BatchWorkspace::drop_graph() {
+  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  graph_exec = nullptr;
+  graph_key = 0;
+}
+
+void BatchWorkspace::release_corridor() {
+  cudaFree(rf);
+  cudaFree(touch);
+  cudaFree(lint);
+  cudaFree(lw);
+  cudaFree(ldist);
+  cudaFree(lstate);
+  cudaFree(lline);
+  rf = nullptr;
+  touch = nullptr;
+  lint = nullptr;
+  lw = nullptr;
+  ldist = nullptr;
+  lstate = nullptr;
+  lline = nullptr;
+  corridor_slots = 0;
+  drop_graph();  // a captured sequence holds these pointers
 }
 
 // The corridor arrays of every worker, allocated by the first call that uses
 // the bounds.  A graph so large that they would take more than an eighth of
 // the device's memory (some 10 million vertices) goes without them: its
 // queries get the two reverse searches over the whole graph.
-static int ensure_corridor(vine_graph *g, const Resolved &r) {
+static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq) {
   BatchWorkspace &w = g->batch;
-  if (!uses_corridors(g, r.cfg) || w.rf != nullptr) return VINE_OK;
+  if (!uses_corridors(g, r.cfg)) return VINE_OK;
+  const int share = share_of(g, r, nq);
+  const int want = share * r.slots;
+  if (w.corridor_slots >= want) return VINE_OK;
   const size_t n = (size_t)g->n;
   const size_t lv = std::min<size_t>(n, kCorridorVertices);
   const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
@@ -1428,8 +1496,16 @@ static int ensure_corridor(vine_graph *g, const Resolved &r) {
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   if (per * r.slots > total_b / 8) return VINE_OK;
-  const size_t k = (size_t)r.slots;
+  size_t k = (size_t)r.slots;
+  // more only where they leave the device as much again
+  for (int f = share; f > 1; f /= 2)
+    if (per * f * r.slots <= std::min(total_b / 8, (free_b + per * w.corridor_slots) / 2)) {
+      k = (size_t)f * r.slots;
+      break;
+    }
+  if ((size_t)w.corridor_slots >= k) return VINE_OK;
   VINE_TRY(ensure_lines(g));
+  w.release_corridor();
   VINE_CUDA_TRY(cudaMalloc(&w.touch, sizeof(uint32_t) * 2 * n * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * k));
   VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * k));
@@ -1440,6 +1516,7 @@ static int ensure_corridor(vine_graph *g, const Resolved &r) {
   VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
   w.lv = (int)lv;
   w.la = (int)la;
+  w.corridor_slots = (int)k;
   return VINE_OK;
 }
 
@@ -1466,8 +1543,8 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     w.max_chunks = 4096;
     VINE_CUDA_TRY(cudaMalloc(&w.chunks, sizeof(uint2) * (size_t)w.max_chunks * r.slots));
     VINE_CUDA_TRY(cudaMalloc(&w.sinklist, sizeof(uint32_t) * (size_t)sink_cap * r.slots));
-    VINE_CUDA_TRY(cudaMalloc(&w.bctr, sizeof(uint32_t) * r.slots));
-    VINE_CUDA_TRY(cudaMemset(w.bctr, 0, sizeof(uint32_t) * r.slots));
+    VINE_CUDA_TRY(cudaMalloc(&w.bctr, sizeof(uint32_t) * kMostShare * r.slots));  // (see share_of)
+    VINE_CUDA_TRY(cudaMemset(w.bctr, 0, sizeof(uint32_t) * kMostShare * r.slots));
     VINE_CUDA_TRY(cudaMalloc(&w.pool, sizeof(Label) * (size_t)c.pool_labels));
     VINE_CUDA_TRY(cudaMalloc(&w.next, sizeof(uint32_t) * (size_t)c.pool_labels));
     VINE_CUDA_TRY(cudaMalloc(&w.counters, sizeof(unsigned long long) * 8));
@@ -1480,9 +1557,12 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     w.pool_cap = c.pool_labels;
     w.epoch_next = 1;
   }
-  VINE_TRY(ensure_corridor(g, r));
+  VINE_TRY(ensure_corridor(g, r, nq));
   if (w.q_cap < nq) {
+    w.drop_graph();  // it holds these pointers
     cudaFree(w.order);
+    cudaFree(w.redo);
+    w.redo = nullptr;
     cudaFree(w.path_start);
     cudaFree(w.path_len);
     cudaFree(w.path_arena);
@@ -1492,6 +1572,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     w.path_arena = nullptr;
     const int64_t cap = std::max<int64_t>(nq, 1024);
     VINE_CUDA_TRY(cudaMalloc(&w.order, sizeof(int32_t) * (size_t)cap));
+    VINE_CUDA_TRY(cudaMalloc(&w.redo, sizeof(int32_t) * (size_t)cap));
     VINE_CUDA_TRY(cudaMalloc(&w.path_start, sizeof(int64_t) * (size_t)cap));
     VINE_CUDA_TRY(cudaMalloc(&w.path_len, sizeof(int32_t) * (size_t)cap));
     w.path_cap = cap * 4096;
@@ -1511,16 +1592,12 @@ int batch_prepare(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t str
   if (w.epoch_next > 0xF0000000u - (uint32_t)nq) {
     // epochs would wrap: forget every tag (and any captured launch sequence)
     VINE_CUDA_TRY(cudaMemsetAsync(w.vs, 0, sizeof(VState) * (size_t)g->n * w.slots, stream));
-    VINE_CUDA_TRY(cudaMemsetAsync(w.bctr, 0, sizeof(uint32_t) * w.slots, stream));
+    VINE_CUDA_TRY(cudaMemsetAsync(w.bctr, 0, sizeof(uint32_t) * kMostShare * w.slots, stream));
     const unsigned long long one = 1;
     VINE_CUDA_TRY(cudaMemcpyAsync(w.counters + 4, &one, sizeof(one), cudaMemcpyHostToDevice, stream));
     VINE_CUDA_TRY(cudaStreamSynchronize(stream));
     w.epoch_next = 1;
-    if (w.graph_exec) {
-      cudaGraphExecDestroy(w.graph_exec);
-      w.graph_exec = nullptr;
-      w.graph_key = 0;
-    }
+    w.drop_graph();
   }
   w.epoch_next += (uint32_t)nq;
   const size_t smem = batch_smem_bytes(r.cfg.table_log2, lock_log2_for(r.cfg.table_log2),
@@ -1627,6 +1704,25 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   VINE_CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(unsigned long long) * 4, stream));
   epoch_kernel<<<1, 1, 0, stream>>>(w.counters, nq);
   if (c.order_queries) VINE_TRY(order_queries(nq, d_budget, w.order, stream));
+  const int share = std::min(share_of(g, r, nq), w.corridor_slots / r.slots);
+  if (share > 1 || (share == 1 && two_launches(g, r) && c.table_log2 > kCorridorTable)) {
+    SearchParams D = P;
+    D.table_log2 = std::min(c.table_log2, kCorridorTable);
+    D.lock_log2 = lock_log2_for(D.table_log2);
+    D.near_mask = (uint32_t)(w.near_cap / share - 1);
+    D.far_cap = w.far_cap / share;
+    D.rest_cap = w.rest_cap / share;
+    D.max_chunks = w.max_chunks / share;
+    D.redo = w.redo;
+    D.redo_n = w.counters + 6;
+    const int threads = std::min(c.block_threads, 512 / share);
+    batch_kernel<true><<<share * r.slots, threads,
+                         batch_smem_bytes(D.table_log2, D.lock_log2, 0, threads, c.split_staging), stream>>>(D);
+    VINE_CUDA_TRY(cudaGetLastError());
+    redo_kernel<<<1, 1, 0, stream>>>(w.counters);
+    P.order = w.redo;
+    P.nq_dev = w.counters + 6;
+  }
   kernel_for(g, c)<<<r.slots, c.block_threads, smem, stream>>>(P);
   VINE_CUDA_TRY(cudaGetLastError());
   if (paths) {

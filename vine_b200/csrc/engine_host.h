@@ -56,11 +56,15 @@ struct BatchWorkspace {
   uint4 *lstate = nullptr;
   int4 *lline = nullptr;
   int lv = 0, la = 0;
+  int corridor_slots = 0;       // workers these arrays are for
+  int32_t *redo = nullptr;      // queries listed for the second launch (batch.cu)
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape
   cudaGraphExec_t graph_exec = nullptr;
   uint64_t graph_key = 0;
   void release();
+  void release_corridor();
+  void drop_graph();
 };
 
 // Device buffers of the plain (whole-GPU, one query at a time) engine.

@@ -33,6 +33,9 @@ struct SearchParams {
   const int32_t *dst;
   const float *budget;
   const int32_t *order;
+  const unsigned long long *nq_dev;  // the number of queries in `order`, when only the device knows it
+  int32_t *redo;                     // queries that need the roomier workers (nullptr: fail them)
+  unsigned long long *redo_n;
   // outputs
   float *cost;
   float *odelay;
