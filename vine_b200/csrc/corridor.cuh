@@ -43,7 +43,7 @@ constexpr uint32_t kNoKey = 0xffffffffu;
 constexpr uint32_t kMemberTag = 0xfffffffeu;   // rf[v].y high word: v has a local id
 constexpr float kIntLimit = 16777216.0f;       // 2^24: budgets and costs handled here
 constexpr int kWaveQ = 2048;                   // queue entries kept in shared memory
-constexpr int kCorridorVertices = 1 << 15;     // largest local graph
+constexpr int kCorridorVertices = 1 << 16;     // largest local graph
 constexpr double kFirstLambda = 0.5;           // first multiplier, in mean lengths per mean delay
 constexpr double kWideGap = 0.3;               // (T - meeting key) / meeting key worth another multiplier
 constexpr int kShrinkTo = 1024;                // local graphs up to this size are not shrunk further
