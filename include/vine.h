@@ -89,11 +89,15 @@ typedef struct {
   int32_t mode;            /* vine_mode                                       */
   int32_t policy;          /* vine_policy                                     */
   int32_t use_bounds;      /* reverse lower bounds (delay and A* cost)        */
-  int32_t block_threads;   /* batch engine: threads per query worker (CTA)    */
+  int32_t block_threads;   /* batch engine: threads per query worker (CTA);
+                              calls with bounds and ctas_per_sm = 0 may share
+                              them among 2 or 4 workers (5, 16 queries an SM) */
   int32_t ctas_per_sm;     /* batch engine: resident workers per SM (0=auto)  */
-  int32_t table_log2;      /* shared-memory bucket table entries (log2)       */
+  int32_t table_log2;      /* shared-memory bucket table entries (log2; the
+                              corridor searches of such calls use at most 11) */
   int32_t spill_log2;      /* reserved (overflow chains have no fixed size)   */
-  float bucket_width;      /* bucket width in cost units (0 = auto)           */
+  float bucket_width;      /* bucket width in cost units (0 = auto); the fixed
+                              policy scales its bound searches' buckets too   */
   int32_t split_threshold; /* max labels expanded per round (0 = auto)        */
   int64_t pool_labels;     /* label arena capacity (0 = auto)                 */
   int64_t far_capacity;    /* per-worker far-pile entries (0 = auto)          */

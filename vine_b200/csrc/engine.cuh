@@ -526,31 +526,59 @@ __host__ __device__ inline void make_features(const BucketStats &s, float *x) {
 // Forward pass of the 16-64-64-2 ReLU MLP by one warp (lanes split the 64
 // hidden units two each).  params layout: W1[64][16] b1[64] W2[64][64] b2[64]
 // W3[2][64] b3[2].  `h` is 128 floats of scratch visible to the warp.
+// Bound by the latency of the weight reads (21 KB from L1 / L2): a lane takes
+// rows lane and lane + 32 together, 16 bytes a read, all reads of eight columns
+// in flight at once.  Sums keep the order of the columns.  `params` is 16-byte
+// aligned, and so is every row.
+template <int N>
+__device__ __forceinline__ void mlp_two_rows(const float *__restrict__ w, int lane, const float *x,
+                                             float &a0, float &a1) {
+  const float4 *r0 = reinterpret_cast<const float4 *>(w + lane * N);
+  const float4 *r1 = reinterpret_cast<const float4 *>(w + (lane + 32) * N);
+#pragma unroll
+  for (int i = 0; i < N / 4; i += 2) {
+    const float4 p0 = __ldg(r0 + i), p1 = __ldg(r0 + i + 1), q0 = __ldg(r1 + i), q1 = __ldg(r1 + i + 1);
+    const float *v = x + 4 * i;
+    a0 += p0.x * v[0], a1 += q0.x * v[0];
+    a0 += p0.y * v[1], a1 += q0.y * v[1];
+    a0 += p0.z * v[2], a1 += q0.z * v[2];
+    a0 += p0.w * v[3], a1 += q0.w * v[3];
+    a0 += p1.x * v[4], a1 += q1.x * v[4];
+    a0 += p1.y * v[5], a1 += q1.y * v[5];
+    a0 += p1.z * v[6], a1 += q1.z * v[6];
+    a0 += p1.w * v[7], a1 += q1.w * v[7];
+  }
+}
+
 __device__ inline void mlp_forward_warp(const float *__restrict__ params, const float *x,
                                         float *h, float *y) {
+  static_assert(kHid == 64 && kFeat % 8 == 0, "two rows a lane, eight columns a step");
   const int lane = threadIdx.x & 31;
   const float *W1 = params, *b1 = W1 + kHid * kFeat, *W2 = b1 + kHid, *b2 = W2 + kHid * kHid,
               *W3 = b2 + kHid, *b3 = W3 + kOut * kHid;
-  for (int j = lane; j < kHid; j += 32) {
-    float acc = b1[j];
-    for (int i = 0; i < kFeat; ++i) acc += W1[j * kFeat + i] * x[i];
-    h[j] = fmaxf(acc, 0.0f);
-  }
+  float a0 = b1[lane], a1 = b1[lane + 32];
+  mlp_two_rows<kFeat>(W1, lane, x, a0, a1);
+  h[lane] = fmaxf(a0, 0.0f);
+  h[lane + 32] = fmaxf(a1, 0.0f);
   __syncwarp();
-  float h2[2];
-  for (int r = 0; r < 2; ++r) {
-    const int j = lane + 32 * r;
-    float acc = b2[j];
-    for (int i = 0; i < kHid; ++i) acc += W2[j * kHid + i] * h[i];
-    h2[r] = fmaxf(acc, 0.0f);
-  }
-  __syncwarp();
-  h[kHid + lane] = h2[0];
-  h[kHid + lane + 32] = h2[1];
+  a0 = b2[lane];
+  a1 = b2[lane + 32];
+  mlp_two_rows<kHid>(W2, lane, h, a0, a1);
+  h[kHid + lane] = fmaxf(a0, 0.0f);
+  h[kHid + lane + 32] = fmaxf(a1, 0.0f);
   __syncwarp();
   if (lane < kOut) {
+    const float4 *r = reinterpret_cast<const float4 *>(W3 + lane * kHid);
+    const float *v = h + kHid;
     float acc = b3[lane];
-    for (int i = 0; i < kHid; ++i) acc += W3[lane * kHid + i] * h[kHid + i];
+#pragma unroll
+    for (int i = 0; i < kHid / 4; ++i) {
+      const float4 p = __ldg(r + i);
+      acc += p.x * v[4 * i];
+      acc += p.y * v[4 * i + 1];
+      acc += p.z * v[4 * i + 2];
+      acc += p.w * v[4 * i + 3];
+    }
     y[lane] = acc;
   }
   __syncwarp();

@@ -13,9 +13,11 @@ Training data comes from the plain method itself: the engine runs query sets
 under the AR policy with every global width multiplier in SCALES
 (vine_config.ar_scale), with tracing on.  Each trace row holds the 16
 features the scheduler saw when a bucket was opened.  For every query the
-multiplier with the fewest SM cycles (VINE_STAT_CYCLES) is its label, kept
+multiplier with the fewest SM cycles outside its bound searches
+(VINE_STAT_CYCLES - VINE_STAT_BOUND_CYCLES: widths do not change the bound
+searches, which are most of a query on the road graphs) is its label, kept
 at the AR rule's own width (1) unless another saves at least MARGIN of the
-query's cycles; every trace row of that query, from every run, becomes one
+these cycles; every trace row of that query, from every run, becomes one
 training example: features -> (log2(best multiplier), gate), gate = 1 when
 the best multiplier is not the AR rule's.  The kernel applies the first
 output only where the second says the departure pays: a network that
@@ -47,13 +49,14 @@ from . import api as v
 
 SCALES = (0.35, 0.5, 0.7, 1.0, 1.4, 2.0, 2.8)  # multipliers on the AR width
 BASE_MULT = 0.3          # initial bucket width / mean arc length
-MARGIN = 0.03            # a multiplier other than 1 must save this share of a query's cycles
+MARGIN = 0.03            # a multiplier other than 1 must save this share of those cycles
 TABLE_LOG2 = 13
 MODEL_DIR = Path(__file__).resolve().parent / "models"
 MODEL_NPY = MODEL_DIR / "scheduler_mlp.npy"
 MODEL_JSON = MODEL_DIR / "scheduler_mlp.json"
 
 STAT_CYCLES = 7  # VINE_STAT_CYCLES
+STAT_BOUND_CYCLES = 10  # VINE_STAT_BOUND_CYCLES
 
 
 def base_config(mean_len: float, **kw):
@@ -73,7 +76,7 @@ def collect(graph: v.Graph, src, dst, budget, mean_len: float):
     for k, sc in enumerate(settings):
         cfg = base_config(mean_len, policy="ar", ar_scale=sc, trace=1)
         r = v.solve(graph, src, dst, budget, cfg, paths=False, stats=True)
-        cycles[k] = r.stats[:, STAT_CYCLES]
+        cycles[k] = r.stats[:, STAT_CYCLES] - r.stats[:, STAT_BOUND_CYCLES]
         traces.append(v.fetch_trace(graph))
     return cycles, traces, settings
 
