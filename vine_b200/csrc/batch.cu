@@ -1413,7 +1413,7 @@ bool two_launches(const vine_graph *g, const Resolved &r) {
 // the gaps, but each one is slower, so that the call's longest query ends later.  One, two
 // and four on the road network: 55 / 64 / 83 ms for 600 queries,
 // 90 / 69 / 98 ms for 1,200, 169 / 114 / 110 ms for 2,400 and 295 / 185 /
-// 153 ms for 4,096; on the anti-correlated grid 8.1 / 8.3 / 9.0 ms for 300 and
+// 157 ms for 4,096; on the anti-correlated grid 8.1 / 8.3 / 9.0 ms for 300 and
 // 21 / 12 / 11 ms for 1,200.
 int share_of(const vine_graph *g, const Resolved &r, int32_t nq) {
   if (!two_launches(g, r)) return 1;
@@ -1488,30 +1488,30 @@ static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq) {
   const int want = share * r.slots;
   if (w.corridor_slots >= want) return VINE_OK;
   const size_t n = (size_t)g->n;
-  const size_t lv = std::min<size_t>(n, kCorridorVertices);
-  const size_t la = std::min<size_t>((size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
-  const size_t ints = corridor_ints((int)lv, (int)la);
-  const size_t per = n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
-                     lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4));
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-  if (per * r.slots > total_b / 8) return VINE_OK;
-  size_t k = (size_t)r.slots;
-  // more only where they leave the device as much again
-  for (int f = share; f > 1; f /= 2)
-    if (per * f * r.slots <= std::min(total_b / 8, (free_b + per * w.corridor_slots) / 2)) {
-      k = (size_t)f * r.slots;
-      break;
-    }
+  // Distances are per worker; the workers of an SM share its local graphs.
+  size_t lv = 0, la = 0, ints = 0;
+  auto bytes = [&](size_t f) {
+    lv = std::min<size_t>(f * n, kCorridorVertices);
+    la = std::min<size_t>(f * (size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
+    ints = corridor_ints((int)lv, (int)la);
+    return (size_t)r.slots * (f * n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
+                              lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4)));
+  };
+  size_t f = (size_t)share;
+  while (f > 1 && bytes(f) > std::min(total_b / 16, free_b / 2)) f /= 2;  // more only where there is room
+  if (bytes(f) > total_b / 8) return VINE_OK;
+  const size_t k = f * (size_t)r.slots, sm = (size_t)r.slots;
   if ((size_t)w.corridor_slots >= k) return VINE_OK;
   VINE_TRY(ensure_lines(g));
   w.release_corridor();
   VINE_CUDA_TRY(cudaMalloc(&w.touch, sizeof(uint32_t) * 2 * n * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lline, sizeof(int4) * 16 * lv * k));
+  VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * sm));
+  VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * sm));
+  VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * sm));
+  VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * sm));
+  VINE_CUDA_TRY(cudaMalloc(&w.lline, sizeof(int4) * 16 * lv * sm));
   VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
   VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
   w.lv = (int)lv;
@@ -1683,8 +1683,8 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.ldist = w.ldist;
   P.lstate = w.lstate;
   P.lline = w.lline;
-  P.lv = w.lv;
-  P.la = w.la;
+  P.lv = std::min(g->n, w.lv);
+  P.la = (int)std::min<int64_t>(std::max<int64_t>(g->m, 1), w.la);
   P.mean_len = g->mean_len;
   P.mean_delay = g->mean_delay;
   // Buckets of the corridor searches.  The fixed policy keeps to the width the
@@ -1720,6 +1720,8 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
     D.far_cap = w.far_cap / share;
     D.rest_cap = w.rest_cap / share;
     D.max_chunks = w.max_chunks / share;
+    D.lv = std::min(g->n, w.lv / share);
+    D.la = (int)std::min<int64_t>(std::max<int64_t>(g->m, 1), w.la / share);
     D.redo = w.redo;
     D.redo_n = w.counters + 6;
     const int threads = std::min(c.block_threads, 512 / share);
