@@ -1481,7 +1481,7 @@ void BatchWorkspace::release_corridor() {
 // the bounds.  A graph so large that they would take more than an eighth of
 // the device's memory (some 10 million vertices) goes without them: its
 // queries get the two reverse searches over the whole graph.
-static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq) {
+static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
   BatchWorkspace &w = g->batch;
   if (!uses_corridors(g, r.cfg)) return VINE_OK;
   const int share = share_of(g, r, nq);
@@ -1513,14 +1513,16 @@ static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq) {
   VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * sm));
   VINE_CUDA_TRY(cudaMalloc(&w.lline, sizeof(int4) * 16 * lv * sm));
   VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
-  VINE_CUDA_TRY(cudaMemset(w.rf, 0xff, sizeof(ulonglong2) * n * k));
+  // On the call's stream: a non-blocking one does not wait for the legacy
+  // default stream, and a search must not start while its pairs are cleared.
+  VINE_CUDA_TRY(cudaMemsetAsync(w.rf, 0xff, sizeof(ulonglong2) * n * k, stream));
   w.lv = (int)lv;
   w.la = (int)la;
   w.corridor_slots = (int)k;
   return VINE_OK;
 }
 
-static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) {
+static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
   BatchWorkspace &w = g->batch;
   const vine_config &c = r.cfg;
   const int64_t near_cap = int64_t(1) << 22;
@@ -1550,6 +1552,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     VINE_CUDA_TRY(cudaMalloc(&w.counters, sizeof(unsigned long long) * 8));
     const unsigned long long init[8] = {0, 0, 0, 0, 1, 1, 0, 0};
     VINE_CUDA_TRY(cudaMemcpy(w.counters, init, sizeof(init), cudaMemcpyHostToDevice));
+    VINE_CUDA_TRY(cudaStreamSynchronize(0));  // any stream may use them from here on
     w.slots = r.slots;
     w.far_cap = c.far_capacity;
     w.near_cap = near_cap;
@@ -1557,7 +1560,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     w.pool_cap = c.pool_labels;
     w.epoch_next = 1;
   }
-  VINE_TRY(ensure_corridor(g, r, nq));
+  VINE_TRY(ensure_corridor(g, r, nq, stream));
   if (w.q_cap < nq) {
     w.drop_graph();  // it holds these pointers
     cudaFree(w.order);
@@ -1587,7 +1590,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
 }
 
 int batch_prepare(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
-  VINE_TRY(ensure_batch_workspace(g, r, nq));
+  VINE_TRY(ensure_batch_workspace(g, r, nq, stream));
   BatchWorkspace &w = g->batch;
   if (w.epoch_next > 0xF0000000u - (uint32_t)nq) {
     // epochs would wrap: forget every tag (and any captured launch sequence)

@@ -355,6 +355,7 @@ static int ensure_plain_workspace(vine_graph *g, const Resolved &r, int32_t nq) 
     VINE_CUDA_TRY(cudaMalloc(&w.sinklist, sizeof(uint32_t) * 4096));
     VINE_CUDA_TRY(cudaMalloc(&w.st, sizeof(QueryState)));
     VINE_CUDA_TRY(cudaMallocHost(&w.st_host, sizeof(QueryState)));
+    VINE_CUDA_TRY(cudaStreamSynchronize(0));  // cleared before a non-blocking stream uses them
     w.n = g->n;
     w.far_cap = far_cap;
     w.pool_cap = c.pool_labels;
