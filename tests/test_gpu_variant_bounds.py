@@ -109,3 +109,23 @@ def test_small_first_arena_is_retried():
     for i in range(3):
         assert a.path(i)[0] == src[i] and a.path(i)[-1] == dst[i]
     g.close()
+
+
+@pytest.mark.parametrize("far", [1, 2, 4097, 4099])
+def test_any_far_capacity(far):
+    """A worker's pile starts at a multiple of 16 bytes whatever its capacity;
+    piles of a few entries give no bounds and no room, which is a status."""
+    import vine_b200 as v
+    g = v.Graph(*_random_graph(36, 150, 3, False))
+    rng = np.random.default_rng(8)
+    src, dst = rng.integers(0, 36, 40), rng.integers(0, 36, 40)
+    limits = (np.full(40, 40, np.float32), np.full(40, 7, np.float32), np.full(40, 59, np.float32))
+    for kind in KINDS:
+        want = v.solve_labels(g, kind, src, dst, *limits)
+        got = v.solve_labels(g, kind, src, dst, *limits, config=v.Config(far_capacity=far), raise_on_error=False)
+        ok = got.status == 0
+        assert set(got.status.tolist()) <= {0, v._lib.VINE_ERR_CAPACITY} and (ok.all() or far < 4)
+        np.testing.assert_array_equal(got.found[ok], want.found[ok])
+        np.testing.assert_array_equal(got.cost[ok], want.cost[ok])
+        np.testing.assert_array_equal(got.delay[ok], want.delay[ok])
+    g.close()

@@ -708,7 +708,8 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
   int slots = g->sm_count;
   if (c.max_workers > 0) slots = std::min(slots, (int)c.max_workers);
   slots = std::min<int>(slots, nq);
-  const int64_t far_cap = c.far_capacity > 0 ? c.far_capacity : (int64_t(1) << 20);
+  // whole 16 bytes a worker: the bound passes use a pile as 64-bit entries
+  const int64_t far_cap = ((c.far_capacity > 0 ? c.far_capacity : (int64_t(1) << 20)) + 3) & ~int64_t(3);
   const uint32_t near_cap = 1u << 20;
   const size_t n = (size_t)g->n;
   size_t free_b = 0, total_b = 0;
