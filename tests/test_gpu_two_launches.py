@@ -108,3 +108,19 @@ def test_captured_sequences_follow_the_workspace(case):
         assert not out["status"].any()
         _same(out["cost"].cpu(), out["delay"].cpu(), out["found"].cpu(), want, order)
     g.close()
+
+
+@pytest.mark.parametrize("threads", [64, 512])
+def test_calls_without_any_corridor(case, threads):
+    """Budgets from 2^24 on: the first launch hands every query to the second."""
+    import vine_b200 as v
+    csr, qs, want = case
+    some = [k for k, x in enumerate(qs) if x[2] >= 2.0 ** 24]
+    order = np.array(some * 100)
+    src, dst, bud = (np.array([qs[k][i] for k in order]) for i in range(3))
+    g = v.Graph(*csr)
+    cfg = v.Config(use_bounds=1, block_threads=threads, pool_labels=1 << 27, table_log2=13)
+    for _ in range(3):
+        res = v.solve(g, src.astype(np.int32), dst.astype(np.int32), bud.astype(np.float32), cfg)
+        _same(res.cost, res.delay, res.found, want, order)
+    g.close()

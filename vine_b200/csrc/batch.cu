@@ -951,6 +951,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           __syncthreads();
         }
         if (how == kCorridorNone && P.redo != nullptr) {
+          __syncthreads();  // every thread has read st.abort above and is on this way
           if (tid == 0 && !st.abort) fail_query(st, VINE_ERR_CAPACITY, kSiteNear);  // listed in redo below
           __syncthreads();
         }
