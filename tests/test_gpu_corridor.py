@@ -171,3 +171,24 @@ def test_pareto_sets(name):
             if want["found"]:
                 assert r.path(q)[0] == s and r.path(q)[-1] == t
     g.close()
+
+
+def _beside(chain, ring):
+    """A chain 0 .. chain of long fast arcs beside a ring of short slow ones."""
+    out = [(i, i + 1, 10, 1) for i in range(chain)]
+    first = chain + 1
+    out += [(first + i, first + (i + 1) % ring, 1, 10) for i in range(ring)]
+    return chain + 1 + ring, out
+
+
+@pytest.mark.parametrize("one_launch", [0, 1])
+def test_first_path_past_the_keys(one_launch):
+    """The first search meets on a path whose key its weights cannot bound."""
+    import vine_b200 as v
+    from oracle import oracle as O
+    n, arcs = _beside(40, 400)
+    csr = _graph(n, arcs)
+    g, og = v.Graph(*csr), O.CsrGraph(*csr)
+    _check(v, O, g, og, 0, 40, [100, 105],
+           v.Config(use_bounds=1, policy="ar", table_log2=13, ctas_per_sm=one_launch, pool_labels=1 << 24))
+    g.close()

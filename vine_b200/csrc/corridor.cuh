@@ -1137,7 +1137,14 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
                                : floor((double)((best >> 32) - (unsigned long long)c.b * B) / (double)c.a);
       k.feasible(cost, (double)(uint32_t)best);
     }
-    if (mu != kUnset && !pure) k.optimum(c, mu);
+    if (mu != kUnset && !pure) {
+      if ((mu >> 32) <= kKeyMax) {
+        k.optimum(c, mu);
+      } else if ((uint32_t)mu <= B) {
+        // a path past the keys kept: not known to be the best one, but real
+        k.feasible(floor(((double)(mu >> 32) - (double)c.b * (double)(uint32_t)mu) / (double)c.a), (double)(uint32_t)mu);
+      }
+    }
     if (k.ub < 0.0) {
       // nothing feasible seen: unreachable, or weigh the delay more, at last alone
       if (pure || (mu == kUnset && !W.clipped)) {
@@ -1150,6 +1157,12 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
       continue;
     }
     if (k.ub >= (double)kIntLimit) break;
+    if (best == kUnset) {
+      // the weights were made for a cheaper path: a * ub + b * B passes
+      // kKeyMax, so no limit holds this one.  Again, with weights for its cost.
+      bi_reset(W, M);
+      continue;
+    }
     // The next multiplier to try: the slope once both sides of the budget
     // are known, else less weight on the delay.
     double next = k.slope();
@@ -1180,8 +1193,14 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
       const int n2 = build_local(cl < 0 ? nullptr : M.loc[cl].gid, M.loc[to],
                                  cl < 0 ? M.lv : ne - ne / 4);
       if (n2 >= 0) {
-        ls = (int)(uint32_t)__ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[ls]) + 1);
-        lt = (int)(uint32_t)__ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[lt]) + 1);
+        const unsigned long long ms = __ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[ls]) + 1);
+        const unsigned long long mt = __ldcg(reinterpret_cast<const unsigned long long *>(&M.rf[lt]) + 1);
+        if (key_hi(ms) != kMemberTag || key_hi(mt) != kMemberTag) {  // both ends lie in every corridor
+          ne = -1;
+          break;
+        }
+        ls = (int)(uint32_t)ms;
+        lt = (int)(uint32_t)mt;
         cl = to;
         ne = n2;
       }
