@@ -192,3 +192,44 @@ def test_first_path_past_the_keys(one_launch):
     _check(v, O, g, og, 0, 40, [100, 105],
            v.Config(use_bounds=1, policy="ar", table_log2=13, ctas_per_sm=one_launch, pool_labels=1 << 24))
     g.close()
+
+
+def _no_delay_forth(n):
+    return n, [a for i in range(n - 1) for a in ((i, i + 1, 10, 0), (i + 1, i, 10, 5))]
+
+
+def _fast_row(k, rng):
+    """A k x k grid of slow streets with one fast, long row at its edge."""
+    out = []
+    for r in range(k):
+        for c in range(k):
+            for rr, cc in ((r, c + 1), (r + 1, c)):
+                if rr < k and cc < k:
+                    fast = r == 0 and rr == 0
+                    for u, x in ((r * k + c, rr * k + cc), (rr * k + cc, r * k + c)):
+                        out.append((u, x, 30, 1) if fast else
+                                   (u, x, int(rng.integers(1, 10)), int(rng.integers(10, 31))))
+    return k * k, out
+
+
+@pytest.mark.parametrize("one_launch", [0, 1])
+@pytest.mark.parametrize("name", ["beside", "no_delay_forth", "fast_row", "halves", "unreachable"])
+def test_paths_longer_than_the_budget_suggests(name, one_launch):
+    """The cheapest path within the budget costs many times what the budget
+    and the mean weights suggest, or there is none at all."""
+    import vine_b200 as v
+    from oracle import oracle as O
+    n, arcs, s, t, budgets = {
+        "beside": lambda: (*_beside(40, 400), 0, 40, [39, 40, 41, 100]),
+        "no_delay_forth": lambda: (*_no_delay_forth(41), 0, 40, [0, 0.5, 3]),
+        "fast_row": lambda: (*_fast_row(60, np.random.default_rng(4)), 0, 59, [58, 59, 60, 100]),
+        # three arcs: the first and the last third fit the first search's keys, two do not
+        "halves": lambda: (4004, [(0, 1, 50, 1), (1, 2, 50, 1), (2, 3, 50, 1)] +
+                           [(4 + i, 4 + (i + 1) % 4000, 1, 1) for i in range(4000)], 0, 3, [2, 3, 4]),
+        "unreachable": lambda: (*_beside(40, 400), 0, 45, [10, 1000, 1e6]),
+    }[name]()
+    csr = _graph(n, arcs)
+    g, og = v.Graph(*csr), O.CsrGraph(*csr)
+    _check(v, O, g, og, s, t, budgets,
+           v.Config(use_bounds=1, policy="ar", table_log2=13, ctas_per_sm=one_launch, pool_labels=1 << 24))
+    g.close()

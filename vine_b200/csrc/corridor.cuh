@@ -134,6 +134,9 @@ struct __align__(16) WaveShared {
   uint32_t delta;
   int fb;
   uint32_t hub[kHubs], nhub;  // vertices of this round whose arcs the block shares
+  // clipped: something was left out because its key, with what the other side
+  // needs at least, passes kKeyMax; until a path is known that is no bound, so
+  // a search that ends without a meeting has then not shown that there is none
   int clipped, overflow, stop;
   int scan[kScanScratch];
 };
@@ -347,10 +350,13 @@ __device__ __forceinline__ void bi_relax(WaveShared &W, const CorridorMem &M,
       const unsigned long long mine = back ? pu[k].y : pu[k].x, other = back ? pu[k].x : pu[k].y;
       // What the other side still needs from u, at least: its own distance
       // where that is final, else the radius up to which it is complete.
-      const uint32_t lb = min(key_hi(other), rdone);
-      if (cand < mine && nk[k] + (unsigned long long)lb <= limit)
+      const unsigned long long sum = nk[k] + (unsigned long long)min(key_hi(other), rdone);
+      if (cand < mine && sum <= limit) {
         old[k] = atomicMin(reinterpret_cast<unsigned long long *>(&M.rf[u[k]]) + (back ? 1 : 0), cand);
-      else on &= ~(1u << k);
+      } else {
+        if (cand < mine && sum > kKeyMax) W.clipped = 1;
+        on &= ~(1u << k);
+      }
     }
   uint32_t near = 0, far = 0, first = 0;
 #pragma unroll
@@ -650,8 +656,11 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
       if (key < hi) {
         const ulonglong2 pv = ld_pair(&M.rf[e >> 1]);
         const unsigned long long mine = e & 1u ? pv.y : pv.x, other = e & 1u ? pv.x : pv.y;
-        if (key_hi(mine) == key && key + (unsigned long long)min(key_hi(other), rdone) <= limit)
-          wave_push(W, M, cur, e);
+        const unsigned long long sum = key + (unsigned long long)min(key_hi(other), rdone);
+        if (key_hi(mine) == key) {
+          if (sum <= limit) wave_push(W, M, cur, e);
+          else if (sum > kKeyMax) W.clipped = 1;
+        }
       } else if (key <= limit) {
         far_push(W, M, fb ^ 1, key, e);
       }
