@@ -162,3 +162,29 @@ def test_limits_are_validated(lib):
     for q, e in enumerate(fx["queries"]):
         check_result(fx, res, q, e)
     g.close()
+
+
+@pytest.mark.parametrize("bounds", [0, 1])
+def test_full_path_arena_is_retried(lib, bounds):
+    """200 paths of 30,000 vertices are more than the 4096 vertices a query
+    (for 1,024 queries at least) that a call's path arena holds: the queries
+    past it fail with VINE_ERR_CAPACITY on the device entry, and the host entry
+    solves them again."""
+    v = lib
+    n, nq = 30000, 200
+    row = np.minimum(np.arange(n + 1), n - 1)
+    g = v.Graph(row, np.arange(1, n), np.ones(n - 1, np.float32), np.ones(n - 1, np.float32))
+    fx = {"queries": range(nq), "src": np.zeros(nq, np.int32), "dst": np.full(nq, n - 1, np.int32),
+          "budget": np.full(nq, n, np.float32)}
+    cfg = v.Config(use_bounds=bounds, pool_labels=1 << 27)
+    dev = _device_solve(v, g, fx, cfg)
+    cap = dev["status"] == v._lib.VINE_ERR_CAPACITY
+    assert set(dev["status"].tolist()) == {0, v._lib.VINE_ERR_CAPACITY}
+    assert not dev["found"][cap].any() and dev["found"][~cap].all()
+    assert set(dev["stats"][cap, v._lib.STAT_ABORT_SITE].tolist()) == {9}  # the path arena
+    res = v.solve(g, fx["src"], fx["dst"], fx["budget"], cfg, path_capacity=nq * n)
+    assert res.retried > 0 and not res.status.any() and res.found.all()
+    assert (res.cost == n - 1).all()
+    for q in range(nq):
+        np.testing.assert_array_equal(res.path(q), np.arange(n))
+    g.close()

@@ -1322,9 +1322,10 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       if (tid == 0) P.redo[atomicAdd(P.redo_n, 1ull)] = q;
     } else if (tid == 0) {
       // a corridor seeds inc_key with its cost bound before a label has it
-      const bool ok = st.abort == 0;
-      const bool found = ok && st.inc_key != ~0ull && st.inc_idx != 0xffffffffu;
-      copy_out_path(P, st, q, found, gid);
+      const bool has = st.abort == 0 && st.inc_key != ~0ull && st.inc_idx != 0xffffffffu;
+      copy_out_path(P, st, q, has, gid);
+      const bool ok = st.abort == 0;  // no path without room for it
+      const bool found = has && ok;
       P.status[q] = ok ? VINE_OK : st.abort;
       P.found[q] = found ? 1 : 0;
       P.cost[q] = found ? key_d(st.inc_key) : INFINITY;
