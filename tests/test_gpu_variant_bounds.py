@@ -129,3 +129,23 @@ def test_any_far_capacity(far):
         np.testing.assert_array_equal(got.cost[ok], want.cost[ok])
         np.testing.assert_array_equal(got.delay[ok], want.delay[ok])
     g.close()
+
+
+def test_bandwidth_paths_past_2_24():
+    """Two ways of equal bandwidth: 2^24 + 2 in two arcs, and 2^24 + 3 whose FP32
+    sum along the path is 2^24.  Costs are FP32 sums, so the second is the answer,
+    as in a search without bounds (halved weights).  The ring of short arcs makes
+    the bound pass's buckets narrow."""
+    import vine_b200 as v
+    arcs = [(0, 1, 0, 9), (0, 7, 8388608, 9), (1, 8, 0, 9), (2, 3, 8388608, 9), (3, 4, 1, 9), (4, 5, 1, 9),
+            (5, 6, 1, 9), (7, 6, 8388610, 9), (8, 2, 8388608, 9)]
+    arcs += [(9 + i, 9 + (i + 1) % 4000, 1, 9) for i in range(4000)]
+    row = np.searchsorted([a[0] for a in arcs], np.arange(9 + 4000 + 1))
+    col, ln, dl = (np.array([a[k] for a in arcs]) for k in (1, 2, 3))
+    for scale in (0.5, 1.0):
+        g = v.Graph(row, col, ln * scale, dl)
+        r = v.solve_labels(g, "qos", [0, 0, 0], [6, 3, 6], [9, 9, 10])
+        assert r.found.tolist() == [1, 1, 0]
+        assert r.cost[:2].tolist() == [16777216 * scale] * 2 and r.delay[:2].tolist() == [9, 9]
+        assert r.path(0).tolist() == [0, 1, 8, 2, 3, 4, 5, 6]
+        g.close()

@@ -356,7 +356,13 @@ __device__ void query_bounds(const VParams &P, VState &st, uint32_t *near, uint3
     local_pass_in<false, true>(P, st, P.bound[kind] + (size_t)slot * P.g.n);
     if (threadIdx.x == 0) {
       // a pass that ran out of room or of key range gives no bound
-      const int ok = !W.overflow && !W.clipped && !st.abort;
+      int ok = !W.overflow && !W.clipped && !st.abort;
+      // a pass that went no farther than the source's distance rules out what
+      // is longer, but from 2^24 on FP32 sums may order two paths the other way
+      if (A.target >= 0) {
+        const unsigned long long x = __ldcg(&P.bound[kind][(size_t)slot * P.g.n + (size_t)A.target]);
+        ok = ok && (x == kUnset || (float)key_hi(x) < kIntLimit);
+      }
       if (kind == 0) st.use_len = ok;
       else if (kind == 1) st.use_del = ok;
       else st.use_hop = ok;
