@@ -118,7 +118,7 @@ int io_reserve(IoCache &c, int32_t k, bool stats, size_t stride, int64_t path_ca
                            cudaMalloc(&io.pareto_dl, sizeof(float) * want_stride * cap) != cudaSuccess ||
                            cudaMalloc(&io.pareto_n, sizeof(int32_t) * cap) != cudaSuccess))) {
     c.b.release();
-    return fail(VINE_ERR_CUDA, "result allocation failed");
+    return VINE_CUDA_FAIL("result allocation failed");
   }
   if (!c.pinned &&
       cudaMallocHost(&c.pinned, 36 * (size_t)kPinnedQueries + 8 + sizeof(int32_t) * kPinnedPath) != cudaSuccess) {
@@ -139,7 +139,7 @@ int io_reserve_big_path(IoCache &c, int64_t n) {
   c.big_cap = 0;
   const int64_t cap = n + n / 4 + 1024;
   if (cudaMalloc(&c.b.big_path, sizeof(int32_t) * (size_t)cap) != cudaSuccess)
-    return fail(VINE_ERR_CUDA, "path allocation failed");
+    return VINE_CUDA_FAIL("path allocation failed");
   c.big_cap = cap;
   return VINE_OK;
 }
@@ -322,7 +322,7 @@ int vine_graph_create(int32_t device, int32_t n, int64_t m, const int64_t *row_p
       cudaMalloc(&g->rrow, sizeof(int32_t) * ((size_t)n + 1)) != cudaSuccess ||
       cudaMalloc(&g->rcol, sizeof(int32_t) * mb) != cudaSuccess ||
       cudaMalloc(&g->rw, sizeof(float2) * mb) != cudaSuccess)
-    return cleanup(fail(VINE_ERR_CUDA, "graph allocation failed"));
+    return cleanup(VINE_CUDA_FAIL("graph allocation failed"));
   if (cudaMemcpy(g->row, row32.data(), sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
       (m > 0 && cudaMemcpy(g->col, col, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice) != cudaSuccess) ||
       (m > 0 && cudaMemcpy(g->w, w.data(), sizeof(float2) * (size_t)m, cudaMemcpyHostToDevice) != cudaSuccess) ||

@@ -101,7 +101,7 @@ extern "C" int vine_autotune(vine_graph *g, int32_t nq, const int32_t *src, cons
       cudaMalloc(&d_budget, 4 * (size_t)nq) != cudaSuccess || cudaMalloc(&d_cost, 4 * (size_t)nq) != cudaSuccess ||
       cudaMalloc(&d_delay, 4 * (size_t)nq) != cudaSuccess) {
     cleanup();
-    return fail(VINE_ERR_CUDA, "autotune allocation failed");
+    return VINE_CUDA_FAIL("autotune allocation failed");
   }
   cudaMemcpy(d_src, src, 4 * (size_t)nq, cudaMemcpyHostToDevice);
   cudaMemcpy(d_dst, dst, 4 * (size_t)nq, cudaMemcpyHostToDevice);

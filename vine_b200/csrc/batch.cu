@@ -1481,7 +1481,8 @@ void BatchWorkspace::release_corridor() {
 
 // The corridor arrays of every worker, allocated by the first call that uses
 // the bounds.  A graph so large that they would take more than an eighth of
-// the device's memory (some 10 million vertices) goes without them: its
+// the device's memory (some 10 million vertices), and a device on which they
+// do not fit beside what is allocated, goes without them: its
 // queries get the two reverse searches over the whole graph.
 static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
   BatchWorkspace &w = g->batch;
@@ -1489,7 +1490,7 @@ static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStr
   const int share = share_of(g, r, nq);
   const int want = share * r.slots;
   if (w.corridor_slots >= want) return VINE_OK;
-  const size_t n = (size_t)g->n;
+  const size_t n = (size_t)g->n, sm = (size_t)r.slots;
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   // Distances are per worker; the workers of an SM share its local graphs.
@@ -1498,29 +1499,35 @@ static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStr
     lv = std::min<size_t>(f * n, kCorridorVertices);
     la = std::min<size_t>(f * (size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
     ints = corridor_ints((int)lv, (int)la);
-    return (size_t)r.slots * (f * n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
-                              lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4)));
+    return sm * (f * n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
+                 lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4)));
   };
   size_t f = (size_t)share;
   while (f > 1 && bytes(f) > std::min(total_b / 16, free_b / 2)) f /= 2;  // more only where there is room
-  if (bytes(f) > total_b / 8) return VINE_OK;
-  const size_t k = f * (size_t)r.slots, sm = (size_t)r.slots;
-  if ((size_t)w.corridor_slots >= k) return VINE_OK;
+  if ((size_t)w.corridor_slots >= f * sm) return VINE_OK;
+  // a 64th of the memory is left to the call's other buffers and the caller's
+  if (bytes(f) > total_b / 8 || bytes(f) + total_b / 64 > free_b) return VINE_OK;
   VINE_TRY(ensure_lines(g));
+  if (g->line == nullptr) return VINE_OK;
   w.release_corridor();
-  VINE_CUDA_TRY(cudaMalloc(&w.touch, sizeof(uint32_t) * 2 * n * k));
-  VINE_CUDA_TRY(cudaMalloc(&w.lint, sizeof(int32_t) * ints * sm));
-  VINE_CUDA_TRY(cudaMalloc(&w.lw, sizeof(float2) * 4 * la * sm));
-  VINE_CUDA_TRY(cudaMalloc(&w.ldist, sizeof(unsigned long long) * 4 * lv * sm));
-  VINE_CUDA_TRY(cudaMalloc(&w.lstate, sizeof(uint4) * lv * sm));
-  VINE_CUDA_TRY(cudaMalloc(&w.lline, sizeof(int4) * 16 * lv * sm));
-  VINE_CUDA_TRY(cudaMalloc(&w.rf, sizeof(ulonglong2) * n * k));
-  // On the call's stream: a non-blocking one does not wait for the legacy
-  // default stream, and a search must not start while its pairs are cleared.
-  VINE_CUDA_TRY(cudaMemsetAsync(w.rf, 0xff, sizeof(ulonglong2) * n * k, stream));
-  w.lv = (int)lv;
-  w.la = (int)la;
-  w.corridor_slots = (int)k;
+  // (free memory may lie in pieces: an allocation can fail all the same)
+  auto got = [](auto **p, size_t count) { return cudaMalloc(p, sizeof(**p) * count) == cudaSuccess; };
+  for (; f >= 1; f /= 2) {
+    bytes(f);  // sets the sizes
+    const size_t k = f * sm;
+    if (got(&w.touch, 2 * n * k) && got(&w.lint, ints * sm) && got(&w.lw, 4 * la * sm) &&
+        got(&w.ldist, 4 * lv * sm) && got(&w.lstate, lv * sm) && got(&w.lline, 16 * lv * sm) && got(&w.rf, n * k)) {
+      // On the call's stream: a non-blocking one does not wait for the legacy
+      // default stream, and a search must not start while its pairs are cleared.
+      VINE_CUDA_TRY(cudaMemsetAsync(w.rf, 0xff, sizeof(ulonglong2) * n * k, stream));
+      w.lv = (int)lv;
+      w.la = (int)la;
+      w.corridor_slots = (int)k;
+      return VINE_OK;
+    }
+    cudaGetLastError();  // not an error of the call
+    w.release_corridor();
+  }
   return VINE_OK;
 }
 
@@ -1562,7 +1569,6 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq, 
     w.pool_cap = c.pool_labels;
     w.epoch_next = 1;
   }
-  VINE_TRY(ensure_corridor(g, r, nq, stream));
   if (w.q_cap < nq) {
     w.drop_graph();  // it holds these pointers
     cudaFree(w.order);
@@ -1588,7 +1594,7 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq, 
     w.trace_cap = 1 << 20;
     VINE_CUDA_TRY(cudaMalloc(&w.trace, sizeof(float) * VINE_TRACE_COLS * (size_t)w.trace_cap));
   }
-  return VINE_OK;
+  return ensure_corridor(g, r, nq, stream);  // last: a call can do without
 }
 
 int batch_prepare(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {

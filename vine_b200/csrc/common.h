@@ -19,13 +19,19 @@ inline int fail(int status, const std::string &msg) {
 }  // namespace vine
 
 // Evaluates a CUDA runtime call; on failure records the error and returns
-// VINE_ERR_CUDA from the enclosing function.
+// VINE_ERR_CUDA from the enclosing function.  The runtime's own record of it
+// is taken back, so that the next call does not find it at its launches.
 #define VINE_CUDA_TRY(expr)                                                         \
   do {                                                                              \
     cudaError_t _e = (expr);                                                        \
-    if (_e != cudaSuccess)                                                          \
+    if (_e != cudaSuccess) {                                                        \
+      cudaGetLastError();                                                           \
       return vine::fail(VINE_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
+    }                                                                               \
   } while (0)
+
+// VINE_ERR_CUDA for a runtime call that the caller has seen fail.
+#define VINE_CUDA_FAIL(msg) (cudaGetLastError(), vine::fail(VINE_ERR_CUDA, msg))
 
 #define VINE_TRY(expr)          \
   do {                          \

@@ -187,7 +187,8 @@ struct Resolved {
 
 int resolve_config(const vine_graph *g, const vine_config *in, Resolved *out);
 
-// Makes the graph's arc lines (integral weights only) unless it has them.
+// Makes the graph's arc lines (integral weights only) unless it has them; none
+// where there is no memory for them.
 int ensure_lines(vine_graph *g);
 
 // Batch engine: solves nq queries whose inputs are on the device.

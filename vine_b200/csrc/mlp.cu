@@ -498,7 +498,7 @@ class Scratch {
   int reserve(size_t bytes) {
     bytes = std::max<size_t>(bytes, 256);
     if (bytes > kScratchKeep) {
-      if (cudaMalloc(&base_, bytes) != cudaSuccess) return fail(VINE_ERR_CUDA, "allocation failed");
+      if (cudaMalloc(&base_, bytes) != cudaSuccess) return VINE_CUDA_FAIL("allocation failed");
       own_ = true;
       return VINE_OK;
     }
@@ -507,7 +507,7 @@ class Scratch {
       m_->scratch = nullptr;
       m_->scratch_cap = 0;
       const size_t cap = std::min(kScratchKeep, bytes + bytes / 2);
-      if (cudaMalloc(&m_->scratch, cap) != cudaSuccess) return fail(VINE_ERR_CUDA, "allocation failed");
+      if (cudaMalloc(&m_->scratch, cap) != cudaSuccess) return VINE_CUDA_FAIL("allocation failed");
       m_->scratch_cap = cap;
     }
     base_ = m_->scratch;
@@ -570,7 +570,7 @@ int vine_mlp_create(int32_t device, uint64_t seed, const float *params, vine_mlp
       cudaMalloc(&m->adam_m, sizeof(float) * kMlpParams) != cudaSuccess ||
       cudaMalloc(&m->adam_v, sizeof(float) * kMlpParams) != cudaSuccess) {
     vine_mlp_destroy(m);
-    return fail(VINE_ERR_CUDA, "parameter allocation failed");
+    return VINE_CUDA_FAIL("parameter allocation failed");
   }
   if (cudaMemcpy(m->params, p.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(m->adam_m, 0, sizeof(float) * kMlpParams) != cudaSuccess ||

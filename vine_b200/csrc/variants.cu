@@ -732,9 +732,12 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
   if (per_worker < 1024) return fail(VINE_ERR_CAPACITY, "variant engine: label arena too small");
   const bool hops = call.kind == VINE_LABEL_HOP || call.kind == VINE_LABEL_MAXCOST;
   // bounds: integral weights, and their arrays at most a sixteenth of the memory
-  const bool bounds = g->integral && n * slots * 3 * sizeof(unsigned long long) <= total_b / 16;
+  bool bounds = g->integral && n * slots * 3 * sizeof(unsigned long long) <= total_b / 16;
   const int64_t path_cap = std::max<int64_t>((int64_t)nq * 4096, 1 << 20);
-  if (bounds) VINE_TRY(ensure_lines(g));
+  if (bounds) {
+    VINE_TRY(ensure_lines(g));
+    bounds = g->line != nullptr;
+  }
 
   VParams P;
   std::memset(&P, 0, sizeof(P));
@@ -750,6 +753,7 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
     B.take(&P.far, (size_t)slots * far_cap);
     B.take(&P.pool, (size_t)slots * per_worker);
     B.take(&P.path_arena, path_cap);
+    P.bound[0] = nullptr;
     if (bounds) {
       B.take(&P.bound[0], (size_t)slots * n);
       B.take(&P.bound[1], (size_t)slots * n);
@@ -785,7 +789,11 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
     if (B.used > w.cap) {
       w.release();
       const size_t cap = std::min(kKeepBytes, B.used + B.used / 4);
-      if (cudaMalloc(&w.base, cap) != cudaSuccess) return fail(VINE_ERR_CUDA, "variant engine: allocation failed");
+      if (cudaMalloc(&w.base, cap) != cudaSuccess) {  // an arena of what is free
+        cudaGetLastError();
+        w.base = nullptr;
+        return solve_variants(call, nq, src, dst, L, H, M, 0, out);
+      }
       w.cap = cap;
     }
     B.base = w.base;
@@ -799,7 +807,18 @@ int solve_variants(const VCall &call, int32_t nq, const int32_t *src, const int3
     epoch_base = w.epoch_next;
     w.epoch_next += (uint32_t)nq;
   } else {
-    if (cudaMalloc(&own.p, B.used) != cudaSuccess) return fail(VINE_ERR_CUDA, "variant engine: allocation failed");
+    cudaError_t e = cudaMalloc(&own.p, B.used);
+    if (e != cudaSuccess && arena > 0) {
+      cudaGetLastError();
+      return solve_variants(call, nq, src, dst, L, H, M, 0, out);
+    }
+    if (e != cudaSuccess && bounds) {
+      cudaGetLastError();
+      bounds = false;
+      layout();
+      e = cudaMalloc(&own.p, B.used);
+    }
+    if (e != cudaSuccess) return VINE_CUDA_FAIL("variant engine: allocation failed");
     B.base = own.p;
     VINE_CUDA_TRY(cudaMemsetAsync(own.p, 0, head_bytes, s));
   }
