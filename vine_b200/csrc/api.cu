@@ -86,13 +86,19 @@ struct IoCache {
   size_t stride = 0;
   int64_t path_cap = 0, big_cap = 0;
   char *pinned = nullptr;  // staging of calls of up to kPinnedQueries
+  int calls = 0;           // host calls that could use it so far, up to kPinnedAfter
 };
 
-// Calls of up to this many queries go through a pinned block (12 + 24 bytes a
-// query and kPinnedPath path vertices): results, offsets and most paths then
-// come back in one copy and one wait (a local query: 0.86 -> 0.71 ms).
+// Calls of up to this many queries get results, offsets and the first path
+// vertices in one copy and one wait, and pack their paths on the device behind
+// the results; a larger call reads its results and then its paths.  From the
+// handle's kPinnedAfter-th such call on, the copies go through a pinned block
+// (12 + 24 bytes a query and kPinnedPath path vertices: 212 KB): that saves 20
+// to 30 us a call (a local query 729 -> 710 us), but making the block takes 2
+// to 5 ms, as much as it saves in some 128 calls.
 constexpr int32_t kPinnedQueries = 4096;
 constexpr int64_t kPinnedPath = 1 << 14;
+constexpr int kPinnedAfter = 128;
 
 IoCache &io_cache(vine_graph *g) {
   if (!g->io_cache) g->io_cache = new IoCache();
@@ -119,11 +125,6 @@ int io_reserve(IoCache &c, int32_t k, bool stats, size_t stride, int64_t path_ca
                            cudaMalloc(&io.pareto_n, sizeof(int32_t) * cap) != cudaSuccess))) {
     c.b.release();
     return VINE_CUDA_FAIL("result allocation failed");
-  }
-  if (!c.pinned &&
-      cudaMallocHost(&c.pinned, 36 * (size_t)kPinnedQueries + 8 + sizeof(int32_t) * kPinnedPath) != cudaSuccess) {
-    c.pinned = nullptr;  // staging is a convenience: go without
-    cudaGetLastError();
   }
   c.cap_q = (int64_t)cap;
   c.stats = want_stats;
@@ -356,7 +357,6 @@ void vine_graph_destroy(vine_graph *g) {
   cudaFree(g->rcol);
   cudaFree(g->rw);
   cudaFree(g->line);
-  cudaFree(g->rline);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
 }
@@ -487,6 +487,11 @@ int vine_solve(vine_graph *g, int32_t nq, const int32_t *src, const int32_t *dst
     const bool direct = k <= kPinnedQueries;
     const int64_t path_cap = want_paths && direct ? 4096 * std::max<int64_t>(k, 1024) : 0;
     VINE_TRY(io_reserve(cache, k, out->stats != nullptr, stride, path_cap));
+    if (direct && cache.calls < kPinnedAfter && ++cache.calls == kPinnedAfter &&
+        cudaMallocHost(&cache.pinned, 36 * (size_t)kPinnedQueries + 8 + sizeof(int32_t) * kPinnedPath) != cudaSuccess) {
+      cache.pinned = nullptr;  // staging is a convenience: go without
+      cudaGetLastError();
+    }
     IoBuffers &io = cache.b;
     const size_t head = io.place((size_t)k);
     const bool pinned = cache.pinned != nullptr && direct;

@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 namespace vine {
 
@@ -1442,14 +1443,7 @@ void BatchWorkspace::release() {
   cudaFree(counters);
   cudaFree(order);
   cudaFree(trace);
-  cudaFree(rf);
-  cudaFree(touch);
-  cudaFree(lint);
-  cudaFree(lw);
-  cudaFree(ldist);
-  cudaFree(lstate);
-  cudaFree(lline);
-  cudaFree(redo);
+  cudaFree(corridor);
   drop_graph();
   *this = BatchWorkspace();
 }
@@ -1461,13 +1455,8 @@ void BatchWorkspace::drop_graph() {
 }
 
 void BatchWorkspace::release_corridor() {
-  cudaFree(rf);
-  cudaFree(touch);
-  cudaFree(lint);
-  cudaFree(lw);
-  cudaFree(ldist);
-  cudaFree(lstate);
-  cudaFree(lline);
+  cudaFree(corridor);
+  corridor = nullptr;
   rf = nullptr;
   touch = nullptr;
   lint = nullptr;
@@ -1479,54 +1468,80 @@ void BatchWorkspace::release_corridor() {
   drop_graph();  // a captured sequence holds these pointers
 }
 
-// The corridor arrays of every worker, allocated by the first call that uses
-// the bounds.  A graph so large that they would take more than an eighth of
+// Workers of a call: no more than it has queries where they use corridors,
+// so that the arrays of a small call stay small.
+static int workers_of(const vine_graph *g, const Resolved &r, int32_t nq) {
+  return uses_corridors(g, r.cfg) ? std::min(r.slots, (int)nq) : r.slots;
+}
+
+// The corridor arrays, allocated by the first call that uses them.  A graph so
+// large that those of every SM would take more than an eighth of
 // the device's memory (some 10 million vertices), and a device on which they
 // do not fit beside what is allocated, goes without them: its
 // queries get the two reverse searches over the whole graph.
+//
+// One block, for as many workers as the call has queries (a power of two from
+// 16 on, at most one an SM), or for `share` of them an SM.  On a
+// 264,000-vertex road network those of 148 workers are 5.9 GB, and seven
+// allocations of that made the first call of a handle with one query 6 ms
+// longer; 16 workers' in one block take 0.4 ms.
 static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
   BatchWorkspace &w = g->batch;
   if (!uses_corridors(g, r.cfg)) return VINE_OK;
   const int share = share_of(g, r, nq);
-  const int want = share * r.slots;
-  if (w.corridor_slots >= want) return VINE_OK;
-  const size_t n = (size_t)g->n, sm = (size_t)r.slots;
+  if (w.corridor_slots >= (share > 1 ? share * r.slots : workers_of(g, r, nq))) return VINE_OK;
+  int few = 16;
+  while (few < nq && few < r.slots) few *= 2;
+  const size_t n = (size_t)g->n, sms = (size_t)(share > 1 ? r.slots : std::min(few, r.slots));
   size_t free_b = 0, total_b = 0;
   VINE_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
   // Distances are per worker; the workers of an SM share its local graphs.
-  size_t lv = 0, la = 0, ints = 0;
-  auto bytes = [&](size_t f) {
+  size_t lv = 0, la = 0;
+  auto layout = [&](size_t f, size_t sm) {  // sets lv, la and the pointers; returns the bytes
     lv = std::min<size_t>(f * n, kCorridorVertices);
     la = std::min<size_t>(f * (size_t)std::max<int64_t>(g->m, 1), 4 * (size_t)kCorridorVertices);
-    ints = corridor_ints((int)lv, (int)la);
-    return sm * (f * n * (sizeof(ulonglong2) + 2 * sizeof(uint32_t)) + ints * 4 + la * 4 * sizeof(float2) +
-                 lv * (4 * sizeof(unsigned long long) + sizeof(uint4) + 16 * sizeof(int4)));
+    size_t used = 0;
+    auto take = [&](auto **p, size_t count) {
+      if (w.corridor) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(w.corridor + used);
+      used += (sizeof(**p) * count + 255) & ~(size_t)255;
+    };
+    take(&w.rf, f * n * sm);
+    take(&w.touch, 2 * f * n * sm);
+    take(&w.lint, corridor_ints((int)lv, (int)la) * sm);
+    take(&w.lw, 4 * la * sm);
+    take(&w.ldist, 4 * lv * sm);
+    take(&w.lstate, lv * sm);
+    take(&w.lline, 16 * lv * sm);
+    return used;
+  };
+  auto bytes = [&](size_t f, size_t sm) {
+    char *held = w.corridor;
+    w.corridor = nullptr;  // sizes only
+    const size_t b = layout(f, sm);
+    w.corridor = held;
+    return b;
   };
   size_t f = (size_t)share;
-  while (f > 1 && bytes(f) > std::min(total_b / 16, free_b / 2)) f /= 2;  // more only where there is room
-  if ((size_t)w.corridor_slots >= f * sm) return VINE_OK;
+  while (f > 1 && bytes(f, sms) > std::min(total_b / 16, free_b / 2)) f /= 2;  // more only where there is room
+  if ((size_t)w.corridor_slots >= f * sms) return VINE_OK;
   // a 64th of the memory is left to the call's other buffers and the caller's
-  if (bytes(f) > total_b / 8 || bytes(f) + total_b / 64 > free_b) return VINE_OK;
+  if (bytes(f, (size_t)r.slots) > total_b / 8 || bytes(f, sms) + total_b / 64 > free_b) return VINE_OK;
   VINE_TRY(ensure_lines(g));
   if (g->line == nullptr) return VINE_OK;
   w.release_corridor();
-  // (free memory may lie in pieces: an allocation can fail all the same)
-  auto got = [](auto **p, size_t count) { return cudaMalloc(p, sizeof(**p) * count) == cudaSuccess; };
-  for (; f >= 1; f /= 2) {
-    bytes(f);  // sets the sizes
-    const size_t k = f * sm;
-    if (got(&w.touch, 2 * n * k) && got(&w.lint, ints * sm) && got(&w.lw, 4 * la * sm) &&
-        got(&w.ldist, 4 * lv * sm) && got(&w.lstate, lv * sm) && got(&w.lline, 16 * lv * sm) && got(&w.rf, n * k)) {
+  for (; f >= 1; f /= 2) {  // (free memory may lie in pieces)
+    if (cudaMalloc(&w.corridor, bytes(f, sms)) == cudaSuccess) {
+      layout(f, sms);
       // On the call's stream: a non-blocking one does not wait for the legacy
       // default stream, and a search must not start while its pairs are cleared.
-      VINE_CUDA_TRY(cudaMemsetAsync(w.rf, 0xff, sizeof(ulonglong2) * n * k, stream));
+      VINE_CUDA_TRY(cudaMemsetAsync(w.rf, 0xff, sizeof(ulonglong2) * n * f * sms, stream));
       w.lv = (int)lv;
       w.la = (int)la;
-      w.corridor_slots = (int)k;
+      w.corridor_slots = (int)(f * sms);
       return VINE_OK;
     }
     cudaGetLastError();  // not an error of the call
-    w.release_corridor();
+    w.corridor = nullptr;
   }
   return VINE_OK;
 }
@@ -1572,7 +1587,6 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq, 
   if (w.q_cap < nq) {
     w.drop_graph();  // it holds these pointers
     cudaFree(w.order);
-    cudaFree(w.redo);
     w.redo = nullptr;
     cudaFree(w.path_start);
     cudaFree(w.path_len);
@@ -1582,8 +1596,8 @@ static int ensure_batch_workspace(vine_graph *g, const Resolved &r, int32_t nq, 
     w.path_len = nullptr;
     w.path_arena = nullptr;
     const int64_t cap = std::max<int64_t>(nq, 1024);
-    VINE_CUDA_TRY(cudaMalloc(&w.order, sizeof(int32_t) * (size_t)cap));
-    VINE_CUDA_TRY(cudaMalloc(&w.redo, sizeof(int32_t) * (size_t)cap));
+    VINE_CUDA_TRY(cudaMalloc(&w.order, sizeof(int32_t) * 2 * (size_t)cap));
+    w.redo = w.order + cap;
     VINE_CUDA_TRY(cudaMalloc(&w.path_start, sizeof(int64_t) * (size_t)cap));
     VINE_CUDA_TRY(cudaMalloc(&w.path_len, sizeof(int32_t) * (size_t)cap));
     w.path_cap = cap * 4096;
@@ -1687,7 +1701,9 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   P.split_staging = c.split_staging;
   P.wait_limit = c.wait_limit;
   P.time_limit_ns = c.time_limit_ms > 0 ? (unsigned long long)c.time_limit_ms * 1000000ull : 0ull;
-  P.rf = uses_corridors(g, c) ? w.rf : nullptr;
+  const int workers = workers_of(g, r, nq);
+  const bool corridors = uses_corridors(g, c) && w.corridor_slots >= workers;
+  P.rf = corridors ? w.rf : nullptr;
   P.touch = w.touch;
   P.lint = w.lint;
   P.lw = w.lw;
@@ -1722,7 +1738,8 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
   VINE_CUDA_TRY(cudaMemsetAsync(w.counters, 0, sizeof(unsigned long long) * 4, stream));
   epoch_kernel<<<1, 1, 0, stream>>>(w.counters, nq);
   if (c.order_queries) VINE_TRY(order_queries(nq, d_budget, w.order, stream));
-  const int share = std::min(share_of(g, r, nq), w.corridor_slots / r.slots);
+  int share = corridors ? share_of(g, r, nq) : 0;
+  if (share > 1) share = std::min(share, w.corridor_slots / r.slots);
   if (share > 1 || (share == 1 && two_launches(g, r) && c.table_log2 > kCorridorTable)) {
     SearchParams D = P;
     D.table_log2 = std::min(c.table_log2, kCorridorTable);
@@ -1736,14 +1753,14 @@ int batch_enqueue(vine_graph *g, const Resolved &r, int32_t nq, const int32_t *d
     D.redo = w.redo;
     D.redo_n = w.counters + 6;
     const int threads = std::min(c.block_threads, 512 / share);
-    batch_kernel<true><<<share * r.slots, threads,
+    batch_kernel<true><<<share * workers, threads,
                          batch_smem_bytes(D.table_log2, D.lock_log2, 0, threads, c.split_staging), stream>>>(D);
     VINE_CUDA_TRY(cudaGetLastError());
     redo_kernel<<<1, 1, 0, stream>>>(w.counters);
     P.order = w.redo;
     P.nq_dev = w.counters + 6;
   }
-  kernel_for(g, c)<<<r.slots, c.block_threads, smem, stream>>>(P);
+  kernel_for(g, c)<<<workers, c.block_threads, smem, stream>>>(P);
   VINE_CUDA_TRY(cudaGetLastError());
   if (paths) {
     paths->arena = w.path_arena;

@@ -48,6 +48,7 @@ struct BatchWorkspace {
   int64_t trace_cap = 0;
   // corridors (calls with bounds): two-sided distances, touched vertices and
   // the local graphs of every worker
+  char *corridor = nullptr;     // the block that holds them
   ulonglong2 *rf = nullptr;
   uint32_t *touch = nullptr;
   int32_t *lint = nullptr;
@@ -57,7 +58,7 @@ struct BatchWorkspace {
   int4 *lline = nullptr;
   int lv = 0, la = 0;
   int corridor_slots = 0;       // workers these arrays are for
-  int32_t *redo = nullptr;      // queries listed for the second launch (batch.cu)
+  int32_t *redo = nullptr;      // queries listed for the second launch (batch.cu; behind `order`)
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape
   cudaGraphExec_t graph_exec = nullptr;
@@ -113,7 +114,7 @@ struct vine_graph {
   float mean_delay = 1.0f;
   int32_t *row = nullptr, *col = nullptr, *rrow = nullptr, *rcol = nullptr;
   float2 *w = nullptr, *rw = nullptr;
-  int4 *line = nullptr, *rline = nullptr;  // arc lines, made when first needed
+  int4 *line = nullptr, *rline = nullptr;  // arc lines (one block), made when first needed
   uint64_t fingerprint = 0;
   cudaStream_t stream = nullptr;
   std::mutex mu;  // one solve at a time per handle

@@ -139,12 +139,12 @@ __global__ void line_kernel(int32_t n, const int32_t *row, const int32_t *col, c
 int ensure_lines(vine_graph *g) {
   if (g->line) return VINE_OK;
   const size_t bytes = sizeof(int4) * 4 * (size_t)g->n;
-  if (cudaMalloc(&g->rline, bytes) != cudaSuccess || cudaMalloc(&g->line, bytes) != cudaSuccess) {
+  if (cudaMalloc(&g->line, 2 * bytes) != cudaSuccess) {
     cudaGetLastError();  // the caller can do without
-    cudaFree(g->rline);
-    g->rline = g->line = nullptr;
+    g->line = nullptr;
     return VINE_OK;
   }
+  g->rline = g->line + 4 * (size_t)g->n;
   const int blocks = (g->n + 255) / 256;
   line_kernel<<<blocks, 256>>>(g->n, g->row, g->col, g->w, g->line);
   line_kernel<<<blocks, 256>>>(g->n, g->rrow, g->rcol, g->rw, g->rline);
