@@ -188,3 +188,24 @@ def test_full_path_arena_is_retried(lib, bounds):
     for q in range(nq):
         np.testing.assert_array_equal(res.path(q), np.arange(n))
     g.close()
+
+
+@pytest.mark.parametrize("mode,bounds", [("optimal", 1), ("pareto", 0)])
+def test_time_limit_with_corridors(lib, mode, bounds):
+    """Buckets so wide that a query's label search is one wave: the limit is
+    looked at there too (every 64 rounds and 32 batches, some milliseconds)."""
+    v = lib
+    fx, g = _graph(v, "grid")
+    hard = np.argsort([-q["delay"] if q["found"] else 0.0 for q in fx["queries"]])[:16]
+    args = [fx[k][hard] for k in ("src", "dst", "budget")]
+    cfg = v.Config(mode=mode, use_bounds=bounds, bucket_width=1e7, time_limit_ms=1, pool_labels=1 << 28)
+    res = v.solve(g, *args, cfg, stats=True, raise_on_error=False, pareto_stride=64 if mode == "pareto" else 0)
+    print(f"slowest query {res.stats[:, v._lib.STAT_TIME_NS].max() / 1e6:.2f} ms, statuses {res.status.tolist()}")
+    late = res.status == v._lib.VINE_ERR_TIMEOUT
+    assert set(res.status.tolist()) <= {0, v._lib.VINE_ERR_TIMEOUT} and late.any()
+    assert set(res.stats[late, v._lib.STAT_ABORT_SITE].tolist()) == {v._lib.SITE_TIME}
+    assert res.stats[:, v._lib.STAT_TIME_NS].max() < 6e6
+    again = v.solve(g, fx["src"], fx["dst"], fx["budget"], v.Config(use_bounds=1))
+    for q, e in enumerate(fx["queries"]):
+        check_result(fx, again, q, e)
+    g.close()

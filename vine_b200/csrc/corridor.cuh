@@ -520,8 +520,19 @@ __device__ __forceinline__ uint32_t bi_hubs(const DevGraph &g, WaveShared &W, co
   return relaxed;
 }
 
-// Runs rounds until the queue is empty (all threads).  Returns arcs relaxed
-// by the calling thread.
+// A bucket or a wave may take any number of rounds, so the query's limits are
+// looked at between them too: warp 0 leaves a run of narrow rounds (about 1 us
+// each) after kNarrowRun, and the block looks at every kLookAt-th turn.  That
+// costs 1 to 3 % of a call's cycles (96 road pairs 2,017 -> 2,037 M, 64 queries
+// on a power-law graph 1,993 -> 2,037 M), 8 and 512 in place of 32 and 128 as much.
+constexpr uint32_t kNarrowRun = 128, kLookAt = 32;
+static __device__ __noinline__ void look_at_limits(const SearchParams &P, QueryState &st) {
+  if (st.n_rounds > kMaxRounds) fail_query(st, VINE_ERR_TIMEOUT, kSiteRounds);
+  over_time(P, st);
+}
+
+// Runs rounds until the queue is empty or kLookAt turns are over (all threads).
+// Returns arcs relaxed by the calling thread.
 //
 // Bound by latency: a round is a chain of dependent reads (queue, row and
 // pair, arcs, their pairs), one atomic and the push.  A lane takes a whole
@@ -535,16 +546,16 @@ __device__ __forceinline__ uint32_t bi_rounds(QueryState &st, WaveShared &W, int
   const Combo &c = W.c;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   uint32_t relaxed = 0;
-  for (;;) {
+  for (uint32_t turn = 0;; ++turn) {
     __syncthreads();
     const uint32_t nc = min(W.nq[cur], (uint32_t)kWaveQ + M.ovf_cap);
-    if (nc == 0 || W.stop) break;  // W.stop changes only between the barriers below
+    if (nc == 0 || W.stop || turn == kLookAt) break;  // W.stop changes only between the barriers below
     if (nc <= 32u) __syncthreads();  // every warp has read the count
     const bool narrow = nc <= 32u;
     const uint32_t take = narrow ? 32u : min(32u, (nc + (uint32_t)nw - 1u) / (uint32_t)nw);
     uint32_t n = nc;
     if (!narrow || warp == 0) {
-      for (;;) {
+      for (uint32_t run = 1;; ++run) {
         for (uint32_t base = (uint32_t)warp * take; base < n; base += (uint32_t)nw * take)
           relaxed += bi_chunk(g, W, M, c, cur, fb, base, min(take, n - base));
         if (!narrow) break;
@@ -556,7 +567,7 @@ __device__ __forceinline__ uint32_t bi_rounds(QueryState &st, WaveShared &W, int
         cur ^= 1;
         __syncwarp();
         n = vol(W.nq[cur]);
-        if (n == 0 || n > 32u || vol(W.nhub) != 0) break;
+        if (n == 0 || n > 32u || vol(W.nhub) != 0 || run == kNarrowRun) break;
       }
     }
     if (!narrow) __syncthreads();
@@ -629,6 +640,14 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
   uint32_t relaxed = 0;
   for (;;) {
     relaxed += bi_rounds(st, W, cur, fb);
+    if (W.nq[cur] != 0 && !W.stop) {  // (the same for every thread: nothing changes until the barrier)
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        look_at_limits(P, st);
+        if (st.abort) W.stop = 1;
+      }
+      continue;
+    }
     // nothing unsettled lies below far_min on either side
     const uint32_t fm = W.far_min, lo = max(W.hi, fm);
     const bool stop = fm == kNoKey || W.stop || (to_meeting && 2ull * lo >= (vol(W.mu) >> 32));
@@ -944,7 +963,7 @@ static __device__ __noinline__ uint32_t local_pass_in(const Params &P, State &st
     W.mu = kUnset;
     W.q[0][0] = (uint32_t)A.root;
   }
-  uint32_t relaxed = 0;
+  uint32_t relaxed = 0, turn = 0;
   int cur = 0, fb = 0;
   for (;;) {
     __syncthreads();
@@ -978,7 +997,7 @@ static __device__ __noinline__ uint32_t local_pass_in(const Params &P, State &st
     if (nc <= 32u) {
       __syncthreads();  // every warp has read the count
       if (warp == 0) {
-        uint32_t n = nc;
+        uint32_t n = nc, run = 0;
         do {
           relaxed += local_chunk<kShared, kWhole>(W, D, cur, fb, 0, n);
           __syncwarp();
@@ -989,7 +1008,7 @@ static __device__ __noinline__ uint32_t local_pass_in(const Params &P, State &st
           cur ^= 1;
           __syncwarp();
           n = vol(W.nq[cur]);
-        } while (n != 0 && n <= 32u);
+        } while (n != 0 && n <= 32u && ++run != kNarrowRun);
         if (lane == 0) W.cur = cur;
       }
     } else {
@@ -1003,7 +1022,10 @@ static __device__ __noinline__ uint32_t local_pass_in(const Params &P, State &st
         st.n_rounds++;
       }
     }
-    if (tid == 0 && (W.overflow || st.abort)) W.stop = 1;
+    if (tid == 0) {
+      if (++turn % kLookAt == 0) look_at_limits(P, st);
+      if (W.overflow || st.abort) W.stop = 1;
+    }
     __syncthreads();
     cur = W.cur;
   }

@@ -210,6 +210,9 @@ struct VState {
 // over_time of a query of this engine (called by the bound passes).
 __device__ __forceinline__ bool over_time(const VParams &P, VState &st);
 
+// The bound passes' look at the query's limits.
+static __device__ __noinline__ void look_at_limits(const VParams &P, VState &st) { over_time(P, st); }
+
 constexpr int kVBatch = 2;  // labels per thread per round
 
 __device__ __forceinline__ void vfail(VState &st, int status, int site) {

@@ -541,7 +541,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
   }
   RunCounters C{0u, 0u, 0u};
   int cur = 0, fbuf = 0;
-  uint32_t waves = 0;
+  uint32_t waves = 0, turn = 0;
   for (;;) {
     __syncthreads();
     const uint32_t nc = min(Q.nn[cur], (uint32_t)S.nb + S.novf_cap);
@@ -628,7 +628,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
     if (nc <= 32u) {
       __syncthreads();  // every warp has read the count
       if (warp == 0) {
-        uint32_t n = nc;
+        uint32_t n = nc, run = 0;
         do {
           batch_warp(P, st, Q, S, cur, fbuf, 0, n, C);
           if (lane == 0) {
@@ -639,12 +639,15 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
           cur ^= 1;
           __syncwarp();
           n = vol(Q.nn[cur]);
-        } while (n != 0 && n <= 32u && !vol(*reinterpret_cast<const uint32_t *>(&Q.stop)));
+        } while (n != 0 && n <= 32u && !vol(*reinterpret_cast<const uint32_t *>(&Q.stop)) && ++run != kNarrowRun);
         if (lane == 0) Q.cur = cur;
       }
     } else {
-      for (uint32_t i0 = 0; i0 < nc && !Q.stop; i0 += batch_size())
+      for (uint32_t i0 = 0; i0 < nc && !Q.stop; i0 += batch_size()) {
+        // (sets st.abort, at which the batch stops the search)
+        if (tid == 0 && i0 / batch_size() % kLookAt == kLookAt - 1) look_at_limits(P, st);
         batch_block(P, st, Q, S, cur, fbuf, i0, min(batch_size(), nc - i0), C);
+      }
       __syncthreads();
       if (tid == 0) {
         Q.nn[cur] = 0;
@@ -653,7 +656,10 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
         st.b_rounds++;
       }
     }
-    if (tid == 0 && (Q.overflow || st.abort)) Q.stop = 1;
+    if (tid == 0) {
+      if (++turn % kLookAt == 0) look_at_limits(P, st);
+      if (Q.overflow || st.abort) Q.stop = 1;
+    }
     __syncthreads();
     cur = Q.cur;
   }
