@@ -233,3 +233,31 @@ def test_paths_longer_than_the_budget_suggests(name, one_launch):
     _check(v, O, g, og, s, t, budgets,
            v.Config(use_bounds=1, policy="ar", table_log2=13, ctas_per_sm=one_launch, pool_labels=1 << 24))
     g.close()
+
+
+@pytest.mark.parametrize("mode,far", [("pareto", 1024), ("pareto", 0), ("optimal", 1024)])
+def test_searches_that_do_not_fit_the_piles(mode, far):
+    """Waves hold labels that the bucketed search drops earlier, in half of its piles:
+    a query that does not fit is searched again without its corridor within the
+    call, which needs no retry.  Such piles held these queries before there were corridors."""
+    import vine_b200 as v
+    from oracle import oracle as O
+    w = v.Workload.generate(1, rows=30, cols=30, n_pairs=24, alpha=(1.0,))
+    og, g = O.CsrGraph(w.row_ptr, w.col, w.len, w.delay), w.graph()
+    cfg = v.Config(mode=mode, use_bounds=int(mode == "optimal"), ctas_per_sm=1, far_capacity=far, pool_labels=1 << 27)
+    res = v.solve(g, w.src, w.dst, w.budget, cfg, pareto_stride=512 if mode == "pareto" else 0)
+    assert not res.status.any() and res.retried == 0
+    for q in range(w.nq):
+        s, t, b = int(w.src[q]), int(w.dst[q]), float(w.budget[q])
+        h_len, h_del = O.lower_bounds(og, t)
+        want = O.solve_label_setting(og, s, t, b, h_len if mode == "optimal" else None, h_del,
+                                     use_incumbent=mode == "optimal")
+        assert bool(res.found[q]) == want["found"]
+        if want["found"]:
+            assert (float(res.cost[q]), float(res.delay[q])) == (want["cost"], want["delay"])
+            assert res.path(q)[0] == s and res.path(q)[-1] == t
+        if mode == "pareto":
+            front = want["pareto"]
+            assert res.pareto_n[q] == len(front)
+            np.testing.assert_array_equal(res.pareto(q), front[np.argsort(front[:, 0])])
+    g.close()

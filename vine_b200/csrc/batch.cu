@@ -734,6 +734,42 @@ __device__ __forceinline__ void corridor_mem(const SearchParams &P, int slot, Co
   M.state = P.lstate + (size_t)slot * lv;
 }
 
+// Search state at the start of a query's label search (one thread).
+__device__ __forceinline__ void search_start(const SearchParams &P, QueryState &st) {
+  st.inc_key = ~0ull;
+  st.inc_idx = 0xffffffffu;
+  st.far_n = 0;
+  st.far_wpos = 0;
+  st.far_min_bits = kInfBits;
+  st.rest_n = 0;
+  st.rest_wpos = 0;
+  st.rest_min_bits = kInfBits;
+  st.band_hi = INFINITY;
+  st.near_head = st.near_tail = 0;
+  st.abort = 0;
+  st.abort_site = 0;
+  st.done = 0;
+  st.hist_n = 0;
+  st.sink_n = 0;
+  st.b_labels = st.b_expanded = st.b_rounds = st.b_dominated = 0;
+  st.b_candidates = st.b_spilled = st.b_relaxed = 0;
+  st.width = P.width0;
+  st.ar_width = P.width0;
+  st.split_cap = P.round_cap;
+  for (int i = 0; i < kFeat; ++i) st.x_prev[i] = 0.0f;
+}
+
+// The source's label, the first of the worker's arena (one thread; placed
+// in the first bucket by the caller).
+__device__ __forceinline__ void source_label(const SearchParams &P, QueryState &st, int s) {
+  pool_rewind(P, st);
+  pool_reserve(P, st, 1);
+  if (st.abort) return;
+  const uint32_t idx = st.chunk_fill++;
+  P.pool[idx] = Label{s, 0.0f, 0.0f, -1};
+  st.inc_idx = idx;
+}
+
 // kBounds: the call uses corridors (lower bounds, or a Pareto set).  Without them the corridor
 // code and its state are compiled out: they would cost the plain bucketed
 // search registers (12 % on a 45 x 45 grid with default settings).
@@ -835,24 +871,12 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       st.epoch = (uint32_t)*P.epoch_ptr + (uint32_t)q;
       st.bcur += 1;
       st.qbase = st.bcur;
-      st.inc_key = ~0ull;
-      st.inc_idx = 0xffffffffu;
+      search_start(P, st);
       st.inc_lock = 0;
       st.chunk_lock = 0;
       for (int i = 0; i < 32; ++i) st.slab_fill[i] = st.slab_end[i] = 0;
       st.pending = 0;
       st.near_commit = 0;
-      st.far_n = 0;
-      st.far_wpos = 0;
-      st.far_min_bits = kInfBits;
-      st.rest_n = 0;
-      st.rest_wpos = 0;
-      st.rest_min_bits = kInfBits;
-      st.band_hi = INFINITY;
-      st.near_head = st.near_tail = 0;
-      st.abort = 0;
-      st.abort_site = 0;
-      st.done = 0;
       st.n_expanded = st.n_relaxed = st.n_inserted = st.n_dominated = 0;
       st.n_buckets = st.n_rounds = st.n_spills = 0;
       st.n_chain_steps = 0;
@@ -860,15 +884,7 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       st.split_cycles = st.split_items = st.policy_cycles = st.rest_items = 0;
       st.idle_cycles = st.publish_cycles = 0;
       st.load_cycles = st.relax_cycles = 0;
-      st.hist_n = 0;
-      st.sink_n = 0;
-      st.b_labels = st.b_expanded = st.b_rounds = st.b_dominated = 0;
-      st.b_candidates = st.b_spilled = st.b_relaxed = 0;
       st.r_live = 0;
-      st.width = P.width0;
-      st.ar_width = P.width0;
-      st.split_cap = P.round_cap;
-      for (int i = 0; i < kFeat; ++i) st.x_prev[i] = 0.0f;
       const int s = st.src, t = st.dst;
       const float L = st.budget;
       if (s < 0 || s >= P.g.n || t < 0 || t >= P.g.n || isnan(L)) {
@@ -876,12 +892,9 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
       } else if (0.0f > L) {
         st.done = 1;  // even the source label violates the budget
       } else {
-        pool_rewind(P, st);
-        pool_reserve(P, st, 1);
+        source_label(P, st, s);
         if (!st.abort) {
-          const uint32_t idx = st.chunk_fill++;
-          P.pool[idx] = Label{s, 0.0f, 0.0f, -1};
-          st.inc_idx = idx;  // the source label (placed below)
+          const uint32_t idx = st.inc_idx;
           if (s == t) {
             // the source label is the unique Pareto-optimal sink label
             st.inc_key = pack_key(0.0f, 0.0f);
@@ -950,6 +963,21 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           for (int i = tid; i < H; i += G) tv[i] = kEmpty;
           for (int i = tid; i < NL; i += G) locks[i] = 0;
           __syncthreads();
+        }
+        // A corridor or its search that did not fit the piles: the query is left
+        // to the second launch where there is one (below), else it is searched
+        // as a call without corridors would.
+        if (P.rf != nullptr && P.redo == nullptr && st.abort == VINE_ERR_CAPACITY) {
+          __syncthreads();  // read by all
+          if (tid == 0) {
+            search_start(P, st);
+            st.src = P.src[q];
+            st.dst = P.dst[q];
+            source_label(P, st, st.src);
+          }
+          __syncthreads();
+          gid = nullptr;
+          how = kCorridorNone;
         }
         if (how == kCorridorNone && P.redo != nullptr) {
           __syncthreads();  // every thread has read st.abort above and is on this way
