@@ -261,3 +261,24 @@ def test_searches_that_do_not_fit_the_piles(mode, far):
             assert res.pareto_n[q] == len(front)
             np.testing.assert_array_equal(res.pareto(q), front[np.argsort(front[:, 0])])
     g.close()
+
+
+@pytest.mark.parametrize("width,threads", [(0.0, 512), (1.0, 128), (1e7, 512)])
+def test_large_pareto_fronts(width, threads):
+    """Loose budgets on a 60 x 60 grid: up to 194 labels a vertex are kept, over many
+    waves, over waves of a single cost and in one wave."""
+    import vine_b200 as v
+    from oracle import oracle as O
+    w = v.Workload.generate(1, rows=60, cols=60, n_pairs=6, query_seed=5, alpha=(1.0,))
+    og, g = O.CsrGraph(w.row_ptr, w.col, w.len, w.delay), w.graph()
+    cfg = v.Config(mode="pareto", bucket_width=width, block_threads=threads, pool_labels=1 << 28)
+    res = v.solve(g, w.src, w.dst, np.floor(1.5 * w.budget), cfg, pareto_stride=1024)
+    assert not res.status.any() and res.pareto_n.max() > 100
+    for q in range(w.nq):
+        _, h_del = O.lower_bounds(og, int(w.dst[q]))
+        want = O.solve_label_setting(og, int(w.src[q]), int(w.dst[q]), float(np.floor(1.5 * w.budget[q])), None, h_del,
+                                     use_incumbent=False)
+        front = want["pareto"]
+        assert res.pareto_n[q] == len(front)
+        np.testing.assert_array_equal(res.pareto(q), front[np.argsort(front[:, 0])])
+    g.close()

@@ -931,7 +931,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
               S.state = M.state;
               S.n = L.g.n;
               S.sink = st.dst;
-              S.sinks = P.mode == VINE_MODE_PARETO ? c.sinks : nullptr;
+              S.sinks = c.sinks;
+              S.seen = reinterpret_cast<uint2 *>(M.dist[2]);  // (not used by the bounds of this mode)
               S.sink_cap = P.sink_cap;
               S.B = (uint32_t)floorf(st.budget);
               S.a = st.lam_a;
@@ -954,7 +955,8 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
               st.n_bound_rounds = st.n_rounds - r_b;
             }
             const long long t_w = clock64();
-            wave_search(P, st);
+            if (P.mode == VINE_MODE_PARETO) wave_search<true>(P, st);
+            else wave_search<false>(P, st);
             if (tid == 0) st.relax_cycles += clock64() - t_w;
           } else if (how == kCorridorInfeasible && tid == 0) {
             st.done = 1;

@@ -86,7 +86,7 @@ struct CorridorMem {
   int lv, la;          // capacity of a local graph: vertices, arcs
   uint32_t *map;       // [lv] old local id -> new local id
   unsigned long long *dist[4];  // [lv] distances on the local graph
-  uint4 *state;        // [lv] delay, length and combined distance to the sink
+  uint4 *state;        // [lv] delay, length and combined distance to the sink (and see WaveSearch)
 };
 
 // Weights of one search.  pure: key = delay, the second value is the length;
@@ -1319,7 +1319,7 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
       const unsigned long long hd = __ldcg(&D0[i]), hl = __ldcg(&D1[i]);
       const uint32_t hm = use.a ? key_hi(__ldcg(&Hbest[i])) : 0u;
       const bool in = hd != kUnset && hl != kUnset && hm != kNoKey;
-      M.state[i] = make_uint4(key_hi(hd), in ? key_hi(hl) : kNoKey, hm, 0u);
+      M.state[i] = make_uint4(key_hi(hd), in ? key_hi(hl) : kNoKey, hm, kNoKey);
     }
     if (tid == 0) {
       st.src = ls;
@@ -1330,6 +1330,10 @@ static __device__ __noinline__ int corridor_prepare(const SearchParams &P, Query
       st.inc_key = pack_key((float)k.ub, INFINITY);
       Combo o = use;  // the search's order: the same weights, else both criteria alike
       if (use.a == 0 && !pick_combo(unit, k.ub, (double)B, &o)) o.a = o.b = 1;
+      if (pareto) {  // by cost alone (see known_better)
+        o.a = 1;
+        o.b = 0;
+      }
       st.ord_a = o.a;
       st.ord_b = o.b;
     }

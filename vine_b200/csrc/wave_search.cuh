@@ -37,10 +37,12 @@ struct WaveSearch {
   const int4 *line;
   const int32_t *col;
   const float2 *w;
-  const uint4 *state;  // per vertex: delay, length, combined distance to the sink
+  uint4 *state;        // per vertex: delay, length, combined distance to the sink; Pareto mode:
+                       // least delay kept in finished waves (see known_better)
   int n, sink;
-  uint32_t *sinks;       // Pareto mode: arena slots of the sink's kept labels (null otherwise)
+  uint32_t *sinks;       // Pareto mode: arena slots of the sink's kept labels
   int sink_cap;
+  uint2 *seen;           // Pareto mode, per vertex: wave of its runs, their least delay
   uint32_t B, a, b, bB;  // budget, pruning multiplier, b * B
   uint32_t pa, pb;       // order
   Label *pool;
@@ -116,6 +118,49 @@ __device__ __forceinline__ bool run_dominates(const WaveSearch &S, uint32_t run,
   return false;
 }
 
+// True when a label kept before rules the candidate (v, d, dl) out; h: v's state.
+//
+// Pareto sets are searched in order of d alone.  What finished waves kept at v
+// then has a smaller d than any candidate, so one number a vertex, the least delay among
+// it, stands for all of it, and a vertex's runs are those of the wave in
+// progress.  (In the order of the optimal mode runs had to be kept for good:
+// a vertex of a loose 60 x 60 grid query has some 200 labels in as many runs, which
+// every candidate walked: 8 queries 66 ms, in this order 14.6 ms.)  The first
+// run that a vertex gets in a wave folds the older ones into h.w; until then
+// `seen` holds their least delay.
+template <bool kPareto>
+__device__ __forceinline__ bool known_better(const WaveSearch &S, uint32_t v, const uint4 &h, uint32_t d, uint32_t dl,
+                                             uint32_t wave) {
+  if (kPareto) {
+    if (dl >= h.w) return true;
+    const uint2 s = S.seen[v];
+    if (s.x != wave) return dl >= s.y;
+  }
+  return run_dominates(S, S.head[v], d, dl);
+}
+
+// Adds the run of `len` labels from arena slot idx on, the least delay among
+// them `least`, to v (one thread a vertex).
+template <bool kPareto>
+__device__ __forceinline__ void add_run(const WaveSearch &S, uint32_t v, uint32_t idx, uint32_t len, uint32_t least,
+                                        uint32_t wave) {
+  uint32_t before = S.head[v];
+  if (kPareto) {
+    uint2 s = S.seen[v];
+    if (s.x != wave) {
+      // (other threads may read the word meanwhile: both values hold)
+      S.state[v].w = min(S.state[v].w, s.y);
+      s = make_uint2(wave, kNoKey);
+      before = kNone;
+    }
+    s.y = min(s.y, least);
+    S.seen[v] = s;
+  }
+  S.next[idx] = before;
+  if (len > 1) S.next[idx + 1] = len;
+  S.head[v] = len > 1 ? idx : idx | 0x80000000u;
+}
+
 __device__ __forceinline__ void near_get(const WaveSearch &S, int cur, uint32_t i, unsigned long long *k,
                                          uint32_t *par) {
   if (i < (uint32_t)S.nb) {
@@ -182,6 +227,7 @@ __device__ __forceinline__ void label_emit(SearchShared &Q, const WaveSearch &S,
 
 // Expands the kept labels of a warp, one a lane (all lanes call): arena slot
 // idx, key k.  *best / *best_par: the best sink label this lane has seen.
+template <bool kPareto>
 __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearch &S, bool kept,
                                                 unsigned long long k, uint32_t idx, int nxt, int fbuf,
                                                 unsigned long long *best, uint32_t *best_par) {
@@ -211,7 +257,8 @@ __device__ __forceinline__ uint32_t expand_kept(SearchShared &Q, const WaveSearc
         const unsigned long long inc = vol(Q.inc);
         // (a single arc may be as long as 2^24: sums stay below 2^25)
         if (label_beyond(S, h[j], nd, nl, inc)) continue;
-        if (u[j] == S.sink && S.sinks == nullptr) {
+        if (kPareto && nl >= h[j].w) continue;  // a finished wave kept a better one
+        if (!kPareto && u[j] == S.sink) {
           const unsigned long long c = (unsigned long long)nd << 32 | nl;
           if (c < *best && c < inc) {
             atomicMin(&Q.inc, c);
@@ -288,8 +335,9 @@ __device__ __forceinline__ uint32_t segment_min(uint32_t v, uint32_t dl, uint32_
 }
 
 // Pareto mode: a kept label of the sink is listed and not expanded.
+template <bool kPareto>
 __device__ __forceinline__ bool list_sink(QueryState &st, const WaveSearch &S, bool kept, uint32_t v, uint32_t idx) {
-  if (S.sinks == nullptr || !kept || v != (uint32_t)S.sink) return false;
+  if (!kPareto || !kept || v != (uint32_t)S.sink) return false;
   const uint32_t k = atomicAdd(&st.sink_n, 1u);
   if (k < (uint32_t)S.sink_cap) S.sinks[k] = idx;
   else fail_query(st, VINE_ERR_CAPACITY, kSiteSink);
@@ -301,9 +349,10 @@ struct RunCounters {
 };
 
 // A batch of n <= 32 candidates [i0, i0 + n) by the calling warp alone.
+template <bool kPareto>
 __device__ __forceinline__ void batch_warp(const SearchParams &P, QueryState &st, SearchShared &Q,
                                            const WaveSearch &S, int cur, int fbuf, uint32_t i0, uint32_t n,
-                                           RunCounters &C) {
+                                           uint32_t wave, RunCounters &C) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   unsigned long long k = kUnset;
@@ -311,9 +360,10 @@ __device__ __forceinline__ void batch_warp(const SearchParams &P, QueryState &st
   if ((uint32_t)lane < n) {
     near_get(S, cur, i0 + (uint32_t)lane, &k, &par);
     const uint32_t v = key_vertex(k);
-    if (label_beyond(S, S.state[v], key_cost(k), key_delay(k), vol(Q.inc))) {
+    const uint4 h = S.state[v];
+    if (label_beyond(S, h, key_cost(k), key_delay(k), vol(Q.inc))) {
       k = kUnset;
-    } else if (run_dominates(S, S.head[v], key_cost(k), key_delay(k))) {
+    } else if (known_better<kPareto>(S, v, h, key_cost(k), key_delay(k), wave)) {
       k = kUnset;
       C.dominated++;
     }
@@ -356,17 +406,14 @@ __device__ __forceinline__ void batch_warp(const SearchParams &P, QueryState &st
   }
   // the first kept lane of a vertex writes its run
   const unsigned same = __match_any_sync(FULL, v) & km;
-  if (kept && (int)__ffs(same) - 1 == lane) {
-    const uint32_t len = (uint32_t)__popc(same);
-    S.next[idx] = S.head[v];
-    if (len > 1) S.next[idx + 1] = len;
-    S.head[v] = len > 1 ? idx : idx | 0x80000000u;
-  }
+  // along a run delays fall: the last label has the least
+  const uint32_t least = kPareto ? __shfl_sync(FULL, key_delay(k), 31 - __clz((int)(same | 1u))) : 0u;
+  if (kept && (int)__ffs(same) - 1 == lane) add_run<kPareto>(S, v, idx, (uint32_t)__popc(same), least, wave);
   __syncwarp();
   unsigned long long best = kUnset;
   uint32_t best_par = 0;
-  const bool listed = list_sink(st, S, kept, v, idx);
-  C.relaxed += expand_kept(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
+  const bool listed = list_sink<kPareto>(st, S, kept, v, idx);
+  C.relaxed += expand_kept<kPareto>(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
   __syncwarp();
   if (best != kUnset && best == vol(Q.inc)) Q.inc_parent = best_par;
   __syncwarp();
@@ -376,18 +423,20 @@ __device__ __forceinline__ void batch_warp(const SearchParams &P, QueryState &st
 __device__ __forceinline__ uint32_t batch_size() { return 1u << (31 - __clz((int)blockDim.x)); }
 
 // A batch of n <= batch_size() candidates by the whole block.
+template <bool kPareto>
 __device__ __forceinline__ void batch_block(const SearchParams &P, QueryState &st, SearchShared &Q,
                                             const WaveSearch &S, int cur, int fbuf, uint32_t i0, uint32_t n,
-                                            RunCounters &C) {
+                                            uint32_t wave, RunCounters &C) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long k = kUnset;
   uint32_t par = 0;
   if ((uint32_t)tid < n) {
     near_get(S, cur, i0 + (uint32_t)tid, &k, &par);
     const uint32_t v = key_vertex(k);
-    if (label_beyond(S, S.state[v], key_cost(k), key_delay(k), vol(Q.inc))) {
+    const uint4 h = S.state[v];
+    if (label_beyond(S, h, key_cost(k), key_delay(k), vol(Q.inc))) {
       k = kUnset;
-    } else if (run_dominates(S, S.head[v], key_cost(k), key_delay(k))) {
+    } else if (known_better<kPareto>(S, v, h, key_cost(k), key_delay(k), wave)) {
       k = kUnset;
       C.dominated++;
     }
@@ -474,22 +523,21 @@ __device__ __forceinline__ void batch_block(const SearchParams &P, QueryState &s
       }
       const uint32_t end = hi < lim ? Q.xp[hi] : (uint32_t)total;
       const uint32_t len = end - (uint32_t)rank;
-      S.next[idx] = S.head[v];
-      if (len > 1) S.next[idx + 1] = len;
-      S.head[v] = len > 1 ? idx : idx | 0x80000000u;
+      add_run<kPareto>(S, v, idx, len, kPareto ? (uint32_t)S.pool[idx + len - 1].dl : 0u, wave);
     }
   }
   unsigned long long best = kUnset;
   uint32_t best_par = 0;
-  const bool listed = list_sink(st, S, kept, v, idx);
+  const bool listed = list_sink<kPareto>(st, S, kept, v, idx);
   if (warp * 32 < (int)n)
-    C.relaxed += expand_kept(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
+    C.relaxed += expand_kept<kPareto>(Q, S, kept && !listed, k, idx, cur ^ 1, fbuf, &best, &best_par);
   __syncthreads();
   if (best != kUnset && best == vol(Q.inc)) Q.inc_parent = best_par;
   __syncthreads();
 }
 
 // Runs the search set up in SearchShared::s (all threads).  On return st.inc_key / st.inc_idx hold the answer.
+template <bool kPareto>
 static __device__ __noinline__ void wave_search(const SearchParams &P, QueryState &st) {
   extern __shared__ __align__(16) unsigned char smem[];
   SearchShared &Q = *reinterpret_cast<SearchShared *>(smem);
@@ -519,7 +567,10 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
     if ((size_t)(p - smem) + (size_t)S.n * 4 <= kSearchBytes + region) S.head = reinterpret_cast<uint32_t *>(p);
   }
   __syncthreads();
-  for (int i = tid; i < S.n; i += G) S.head[i] = kNone;
+  for (int i = tid; i < S.n; i += G) {
+    S.head[i] = kNone;
+    if (kPareto) S.seen[i] = make_uint2(kNone, kNoKey);
+  }
   // wave width: the policy's bucket width, from cost units to p units (the
   // p of a mean arc for a mean length)
   const float unit = ((float)S.pa * P.mean_len + (float)S.pb * P.mean_delay) / fmaxf(P.mean_len, 1e-3f);
@@ -630,7 +681,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
       if (warp == 0) {
         uint32_t n = nc, run = 0;
         do {
-          batch_warp(P, st, Q, S, cur, fbuf, 0, n, C);
+          batch_warp<kPareto>(P, st, Q, S, cur, fbuf, 0, n, waves, C);
           if (lane == 0) {
             Q.nn[cur] = 0;
             st.n_rounds++;
@@ -646,7 +697,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
       for (uint32_t i0 = 0; i0 < nc && !Q.stop; i0 += batch_size()) {
         // (sets st.abort, at which the batch stops the search)
         if (tid == 0 && i0 / batch_size() % kLookAt == kLookAt - 1) look_at_limits(P, st);
-        batch_block(P, st, Q, S, cur, fbuf, i0, min(batch_size(), nc - i0), C);
+        batch_block<kPareto>(P, st, Q, S, cur, fbuf, i0, min(batch_size(), nc - i0), waves, C);
       }
       __syncthreads();
       if (tid == 0) {
@@ -676,7 +727,7 @@ static __device__ __noinline__ void wave_search(const SearchParams &P, QueryStat
     st.n_buckets++;
     if (Q.overflow && !st.abort) fail_query(st, VINE_ERR_CAPACITY, Q.overflow == 1 ? kSiteNear : kSiteBand);
     st.inc_idx = 0xffffffffu;
-    if (S.sinks != nullptr) st.inc_key = ~0ull;  // the cost bound is no answer
+    if (kPareto) st.inc_key = ~0ull;  // the cost bound is no answer
     if (!st.abort && Q.inc_parent != kNone) {
       pool_reserve(P, st, 1);
       if (!st.abort) {
