@@ -567,7 +567,8 @@ __device__ __forceinline__ uint32_t bi_rounds(QueryState &st, WaveShared &W, int
         cur ^= 1;
         __syncwarp();
         n = vol(W.nq[cur]);
-        if (n == 0 || n > 32u || vol(W.nhub) != 0 || run == kNarrowRun) break;
+        // (a vote: a lane that went on may list a hub before another one has looked)
+        if (__any_sync(0xffffffffu, n == 0 || n > 32u || vol(W.nhub) != 0 || run == kNarrowRun)) break;
       }
     }
     if (!narrow) __syncthreads();
