@@ -282,3 +282,18 @@ def test_large_pareto_fronts(width, threads):
         assert res.pareto_n[q] == len(front)
         np.testing.assert_array_equal(res.pareto(q), front[np.argsort(front[:, 0])])
     g.close()
+
+
+def test_ends_apart_by_a_small_part():
+    """One end reaches a few vertices only, the other one a chain of 55,000: the
+    search ends with the small part (it had walked the chain, 140 ms)."""
+    import vine_b200 as v
+    n = 60000
+    row = np.minimum(np.arange(n + 1), n - 1)
+    g = v.Graph(row, np.arange(1, n), np.ones(n - 1, np.float32), np.ones(n - 1, np.float32))
+    src, dst = [5000, 5000, 10, n - 3, 0], [3, 4999, 12, n - 6, 40]
+    res = v.solve(g, src, dst, [1e6] * 5, v.Config(use_bounds=1, pool_labels=1 << 24), stats=True)
+    assert res.found.tolist() == [0, 0, 1, 0, 1] and res.cost[2] == 2 and res.cost[4] == 40
+    # rounds: as many as the small part has vertices, and a bucket on
+    assert res.stats[0, 5] < 200 and res.stats[1, 5] < 6000
+    g.close()

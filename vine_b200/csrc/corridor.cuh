@@ -133,6 +133,7 @@ struct __align__(16) WaveShared {
   DevGraph g;
   uint32_t delta;
   int fb;
+  uint32_t sides;  // two-sided search: bit s: side s still has vertices to go on from
   uint32_t hub[kHubs], nhub;  // vertices of this round whose arcs the block shares
   // clipped: something was left out because its key, with what the other side
   // needs at least, passes kKeyMax; until a path is known that is no bound, so
@@ -612,6 +613,7 @@ __device__ __forceinline__ void bi_start(WaveShared &W, const DevGraph &g, const
     W.far_min = kNoKey;
     W.hi = delta;
     W.rdone = 0;
+    W.sides = 3;
     W.clipped = 0;
     W.stop = 0;
     W.ntouch[0] = W.ntouch[1] = 1;
@@ -651,7 +653,10 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
     }
     // nothing unsettled lies below far_min on either side
     const uint32_t fm = W.far_min, lo = max(W.hi, fm);
-    const bool stop = fm == kNoKey || W.stop || (to_meeting && 2ull * lo >= (vol(W.mu) >> 32));
+    // Once one side has no vertex left, it has reached all that a path can take:
+    // without a meeting, and with nothing left out for its key, there is none.
+    const bool apart = W.sides != 3u && vol(W.mu) == kUnset && vol(W.best) == kUnset && !W.clipped;
+    const bool stop = fm == kNoKey || W.stop || (to_meeting && (apart || 2ull * lo >= (vol(W.mu) >> 32)));
     __syncthreads();
     if (threadIdx.x == 0) {
       W.rdone = fm == kNoKey ? kKeyMax : lo;
@@ -660,6 +665,7 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
         W.hi = min(lo, kKeyMax + 1u - W.delta) + W.delta;
         W.far_min = kNoKey;
         W.nfar[fb ^ 1] = 0;
+        W.sides = 0;
       } else {
         W.cur = cur;
         W.fb = fb;
@@ -670,9 +676,11 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
     // far entries below the new upper key join the queue; one that a shorter
     // way overtook or that the bound rules out is dropped
     const uint32_t fn = min(W.nfar[fb], M.far_cap), hi = W.hi, limit = combo_limit(W, c), rdone = W.rdone;
+    uint32_t sides = 0;
     for (uint32_t i = threadIdx.x; i < fn; i += blockDim.x) {
       const unsigned long long x = __ldcg(&M.far[fb][i]);
       const uint32_t key = key_hi(x), e = (uint32_t)x;
+      sides |= 1u << (e & 1u);
       if (key < hi) {
         const ulonglong2 pv = ld_pair(&M.rf[e >> 1]);
         const unsigned long long mine = e & 1u ? pv.y : pv.x, other = e & 1u ? pv.x : pv.y;
@@ -685,6 +693,7 @@ static __device__ __noinline__ uint32_t bi_run(const SearchParams &P, QueryState
         far_push(W, M, fb ^ 1, key, e);
       }
     }
+    if (sides) atomicOr(&W.sides, sides);
     fb ^= 1;
   }
   return relaxed;
