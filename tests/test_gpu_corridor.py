@@ -297,3 +297,18 @@ def test_ends_apart_by_a_small_part():
     # rounds: as many as the small part has vertices, and a bucket on
     assert res.stats[0, 5] < 200 and res.stats[1, 5] < 6000
     g.close()
+
+
+@pytest.mark.parametrize("engine", ["batch", "plain"])
+@pytest.mark.parametrize("width", [0.01, 0.3, 1.0])
+def test_narrow_buckets_of_large_costs(engine, width):
+    """The first bucket starts at the source's bound, where the next float is
+    1 away: it holds the source whatever its width (budgets without corridors)."""
+    import vine_b200 as v
+    arcs = [(0, 1, 5000000, 3), (1, 2, 5000001, 4), (2, 3, 4000000, 5), (0, 3, 15000000, 1)]
+    g = v.Graph(*_graph(4, arcs))
+    cfg = v.Config(engine=engine, use_bounds=1, bucket_width=width, pool_labels=1 << 22)
+    res = v.solve(g, [0, 0, 1], [3, 3, 3], [2.0 ** 24, np.inf, 2.0 ** 25], cfg)
+    assert res.found.tolist() == [1, 1, 1]
+    assert res.cost.tolist() == [14000001, 14000001, 9000001] and res.delay.tolist() == [12, 12, 9]
+    g.close()

@@ -1003,9 +1003,11 @@ __global__ void __launch_bounds__(512, 1) batch_kernel(const __grid_constant__ S
           st.done = 1;  // the sink lies beyond the budget
         } else {
           st.lo = sv.hlen;
-          st.hi_bits = __float_as_uint(sv.hlen + P.width0);
+          // (a width below the spacing of floats there still holds the source)
+          const float hi = fmaxf(sv.hlen + P.width0, nextafterf(sv.hlen, INFINITY));
+          st.hi_bits = __float_as_uint(hi);
           st.band_lo = sv.hlen;
-          st.band_hi = sv.hlen + P.width0 * (float)P.band_mult;
+          st.band_hi = fmaxf(sv.hlen + P.width0 * (float)P.band_mult, hi);
           st.bin_inv = (float)kBins / (st.band_hi - st.band_lo);
           if (!(st.bin_inv < INFINITY)) st.bin_inv = 0.0f;
           for (int j = 0; j < kBins; ++j) {

@@ -193,7 +193,7 @@ __global__ void plain_setup_kernel(PlainArgs A, int q, int phase) {
       return;
     }
     st.lo = sv.hlen;
-    st.hi_bits = __float_as_uint(sv.hlen + st.width);
+    st.hi_bits = __float_as_uint(fmaxf(sv.hlen + st.width, nextafterf(sv.hlen, INFINITY)));
     // a chain of one label at the source
     VState *vs = &c.vs[st.src];
     P.next[idx] = kNone;
