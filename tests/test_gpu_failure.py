@@ -209,3 +209,23 @@ def test_time_limit_with_corridors(lib, mode, bounds):
     for q, e in enumerate(fx["queries"]):
         check_result(fx, again, q, e)
     g.close()
+
+
+def test_time_limit_in_reverse_bounds_and_variants(lib):
+    """Limits that run out between two buckets of the reverse bound searches (no
+    corridors: budgets of 2^24) and of the label variants."""
+    v = lib
+    fx, g = _graph(v, "grid")
+    nq = len(fx["src"])
+    far = np.full(nq, 2.0 ** 24, np.float32)
+    hops = np.full(nq, 300, np.float32)
+    for _ in range(4):
+        res = v.solve(g, fx["src"], fx["dst"], far, v.Config(use_bounds=1, time_limit_ms=1), raise_on_error=False)
+        assert set(res.status.tolist()) <= {0, v._lib.VINE_ERR_TIMEOUT}
+        lab = v.solve_labels(g, "hop", fx["src"], fx["dst"], fx["budget"], hops,
+                             config=v.Config(time_limit_ms=1), raise_on_error=False)
+        assert set(lab.status.tolist()) <= {0, v._lib.VINE_ERR_TIMEOUT}
+    again = v.solve(g, fx["src"], fx["dst"], fx["budget"], v.Config(use_bounds=1))
+    for q, e in enumerate(fx["queries"]):
+        check_result(fx, again, q, e)
+    g.close()

@@ -73,6 +73,7 @@ __device__ void cta_reverse_search(Ctx &c, const RoundBuf &rb, int which, float 
     const uint32_t avail = st.near_tail - st.near_head;
     if (avail == 0) {
       if (st.far_n == 0) break;
+      __syncthreads();  // every thread has read st.abort: it may be set here
       if (tid == 0) {
         over_time(P, st);
         st.lo = fmaxf(bucket_hi(st), __uint_as_float(st.far_min_bits));

@@ -501,6 +501,7 @@ __global__ void __launch_bounds__(512, 1) variant_kernel(const __grid_constant__
       if (avail == 0) {
         // ---- next bucket: its key range starts at the far pile's minimum
         if (st.far_n == 0) break;
+        __syncthreads();  // every thread has read st.abort: it may be set here
         if (tid == 0) {
           st.n_buckets++;
           if (P.time_limit_ns && global_ns() - st.g0 > P.time_limit_ns)
