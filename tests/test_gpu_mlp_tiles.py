@@ -53,3 +53,54 @@ def test_training_steps(n, batch):
     np.testing.assert_allclose(m.params[ok], p[ok], rtol=0, atol=2e-5 * steps)
     wl, _ = mlp_ref.loss_grad(p, x, y)
     assert abs(loss - wl) <= 2e-3 * max(1.0, abs(wl))
+
+
+def _mt19937_64(seed):
+    """std::mt19937_64 (the C++ standard's linear_congruential-seeded 64-bit
+    Mersenne twister with its published parameters)."""
+    mask = (1 << 64) - 1
+    x = [seed & mask]
+    for i in range(1, 312):
+        x.append((6364136223846793005 * (x[-1] ^ (x[-1] >> 62)) + i) & mask)
+    i = 312
+    while True:
+        if i == 312:
+            for k in range(312):
+                y = (x[k] & 0xFFFFFFFF80000000) | (x[(k + 1) % 312] & 0x7FFFFFFF)
+                x[k] = x[(k + 156) % 312] ^ (y >> 1) ^ (0xB5026F5AA96619E9 if y & 1 else 0)
+            i = 0
+        y = x[i]
+        y ^= (y >> 29) & 0x5555555555555555
+        y ^= (y << 17) & 0x71D67FFFEDA60000
+        y ^= (y << 37) & 0xFFF7EEE000000000
+        yield y ^ (y >> 43)
+        i += 1
+
+
+@pytest.mark.parametrize("n,batch,epochs", [(513, 513, 1), (2048, 2048, 1), (100, 32, 1), (700, 129, 2),
+                                            (1030, 515, 1), (1500, 600, 1), (2049, 1024, 1), (4200, 2100, 1)])
+def test_training_reads_the_rows_of_each_batch(n, batch, epochs):
+    """Rows that all differ, in the order of the seeded shuffle (Fisher-Yates):
+    a batch that reads other rows than its own, one row twice or a neighbour's,
+    takes other steps.  A parameter is compared where its gradient stands clear of
+    FP32 noise in every step; a step moves it by up to 1e-3."""
+    import vine_b200 as v
+    from oracle import mlp_ref
+    x, y = _data(n, 31)
+    m = v.MLP(seed=9)
+    p = m.params.astype(np.float64)
+    mm, vv, k = np.zeros_like(p), np.zeros_like(p), 0
+    rng, order, clear = _mt19937_64(77), np.arange(n), np.ones(p.shape, bool)
+    for _ in range(epochs):
+        for i in range(n - 1, 0, -1):
+            j = next(rng) % (i + 1)
+            order[i], order[j] = order[j], order[i]
+        for b in range(0, n, batch):
+            rows = order[b:b + batch]
+            _, g = mlp_ref.loss_grad(p, x[rows], y[rows])
+            clear &= np.abs(g) > 1e-3 * np.abs(g).max()
+            k += 1
+            p, mm, vv = mlp_ref.adam_step(p, mm, vv, g, k, 1e-3)
+    m.train(x, y, epochs=epochs, batch=batch, lr=1e-3, seed=77)
+    assert clear.mean() > 0.2
+    np.testing.assert_allclose(m.params[clear], p[clear], rtol=0, atol=2e-5 * k)
