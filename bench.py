@@ -519,16 +519,20 @@ def run_vine(args):
     peak, peak_kind = measured_peak_hbm()
     roof = None
     if work is not None and work.get("nq") == nq:
+        # What the engine itself counted: 32 bytes an arc relaxed (its share of an
+        # arc line, the head's pair of distances), 80 a label expanded (label,
+        # line).  They come from L2 mostly; the launch is bound by the latency of
+        # its rounds.  The whole-graph label setting that the oracle counts would
+        # read more: given as the rate it would have needed, not as one achieved.
+        counted = 32.0 * work_line["gpu_arcs_relaxed"] + 80.0 * work_line["gpu_labels_expanded"]
+        achieved = counted / (kern_ms / 1e3) / 1e9
         alg = algorithmic_bytes(work)
-        achieved = alg / (kern_ms / 1e3) / 1e9
-        # the numerator is the label setting's work under whole-graph bounds;
-        # the engine's corridors look at a part of it
-        traffic = None
-        roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                "algorithmic_bytes_per_launch": alg, "kernel_ms": kern_ms,
+        roof = {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                "frac": achieved / peak, "peak_kind": peak_kind, "kernel_ms": kern_ms,
+                "counted_bytes_per_launch": counted,
                 "kernel": "batch_kernel (corridors, then the remaining queries)",
-                "numerator": "label setting with whole-graph bounds (oracle counts)"}
+                "numerator": "arcs relaxed and labels expanded as the engine counts them, against HBM",
+                "label_setting_bytes": alg, "label_setting_equivalent_gbs": alg / (kern_ms / 1e3) / 1e9}
     line = {
         "metric": METRIC, "value": value, "unit": "queries/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_max / args.steps,
