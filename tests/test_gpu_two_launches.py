@@ -110,6 +110,60 @@ def test_captured_sequences_follow_the_workspace(case):
     g.close()
 
 
+def test_captures_of_the_caller(case):
+    """Calls captured by the caller, on the arrays of a small call (20 queries) and past
+    them (40), replayed before and after larger calls have made others."""
+    import torch
+    import vine_b200 as v
+    csr, qs, want = case
+    g = v.Graph(*csr)
+    rng = np.random.default_rng(7)
+    cfg = v.Config(use_bounds=1, pool_labels=1 << 27)
+
+    def call(n):
+        order = rng.integers(0, len(qs), n)
+        ins = [torch.tensor(np.array([qs[k][i] for k in order]), dtype=t, device="cuda")
+               for i, t in enumerate((torch.int32, torch.int32, torch.float32))]
+        out = {k: torch.empty(n, dtype=t, device="cuda") for k, t in
+               (("cost", torch.float32), ("delay", torch.float32), ("found", torch.int32), ("status", torch.int32))}
+        return order, ins, out
+
+    def check(order, ins, out):
+        torch.cuda.synchronize()
+        assert not out["status"].any()
+        _same(out["cost"].cpu(), out["delay"].cpu(), out["found"].cpu(), want, order)
+
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        first = call(20)
+        v.solve_device(g, *first[1], first[2], cfg, s.cuda_stream)
+    check(*first)
+    held = []
+    for n in (20, 40):
+        c, graph = call(n), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=s):
+            v.solve_device(g, *c[1], c[2], cfg, s.cuda_stream)
+        held.append((c, graph))
+    for larger in (100, 5 * _sms() + 1):
+        for c, graph in held:
+            for x in c[2].values():
+                x.zero_()
+            graph.replay()
+            check(*c)
+        c = call(larger)
+        torch.cuda.synchronize()
+        v.solve_device(g, *c[1], c[2], cfg, s.cuda_stream)
+        check(*c)
+    for c, graph in held:
+        for x in c[2].values():
+            x.zero_()
+        graph.replay()
+        check(*c)
+    del held, graph
+    g.close()
+
+
 @pytest.mark.parametrize("threads", [64, 512])
 def test_calls_without_any_corridor(case, threads):
     """Budgets from 2^24 on: the first launch hands every query to the second."""

@@ -1477,6 +1477,7 @@ void BatchWorkspace::release() {
   cudaFree(order);
   cudaFree(trace);
   cudaFree(corridor);
+  for (char *p : corridors_kept) cudaFree(p);
   drop_graph();
   *this = BatchWorkspace();
 }
@@ -1488,7 +1489,9 @@ void BatchWorkspace::drop_graph() {
 }
 
 void BatchWorkspace::release_corridor() {
-  cudaFree(corridor);
+  if (corridor_captured) corridors_kept.push_back(corridor);
+  else cudaFree(corridor);
+  corridor_captured = false;
   corridor = nullptr;
   rf = nullptr;
   touch = nullptr;
@@ -1518,9 +1521,23 @@ static int workers_of(const vine_graph *g, const Resolved &r, int32_t nq) {
 // 264,000-vertex road network those of 148 workers are 5.9 GB, and seven
 // allocations of that made the first call of a handle with one query 6 ms
 // longer; 16 workers' in one block take 0.4 ms.
+//
+// A call that the caller captures on its stream allocates nothing: it takes the arrays that
+// are there or goes without.  Replays of it use these arrays, so they are kept
+// until the workspace goes when a larger call makes others (at most one set
+// of each power of two, twice the largest together).
 static int ensure_corridor(vine_graph *g, const Resolved &r, int32_t nq, cudaStream_t stream) {
   BatchWorkspace &w = g->batch;
   if (!uses_corridors(g, r.cfg)) return VINE_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream during a capture elsewhere: no allocation either
+    capture = cudaStreamCaptureStatusActive;
+  }
+  if (capture != cudaStreamCaptureStatusNone) {
+    w.corridor_captured = w.corridor != nullptr;
+    return VINE_OK;
+  }
   const int share = share_of(g, r, nq);
   if (w.corridor_slots >= (share > 1 ? share * r.slots : workers_of(g, r, nq))) return VINE_OK;
   int few = 16;

@@ -58,6 +58,8 @@ struct BatchWorkspace {
   int4 *lline = nullptr;
   int lv = 0, la = 0;
   int corridor_slots = 0;       // workers these arrays are for
+  bool corridor_captured = false;      // a stream capture of the caller's holds the arrays
+  std::vector<char *> corridors_kept;  // earlier arrays that such a capture holds
   int32_t *redo = nullptr;      // queries listed for the second launch (batch.cu; behind `order`)
   uint32_t epoch_next = 1;
   // captured launch sequence (CUDA graph) for the current shape
