@@ -1450,7 +1450,8 @@ bool two_launches(const vine_graph *g, const Resolved &r) {
 // and four on the road network: 55 / 64 / 83 ms for 600 queries,
 // 90 / 69 / 98 ms for 1,200, 169 / 114 / 110 ms for 2,400 and 295 / 185 /
 // 157 ms for 4,096; on the anti-correlated grid 8.1 / 8.3 / 9.0 ms for 300 and
-// 21 / 12 / 11 ms for 1,200.
+// 21 / 12 / 11 ms for 1,200.  (Taken before paths were gathered and limits looked at
+// inside a bucket: the 4,096 take 170 ms with both.)
 int share_of(const vine_graph *g, const Resolved &r, int32_t nq) {
   if (!two_launches(g, r)) return 1;
   return nq > 16 * r.slots ? 4 : nq > 5 * r.slots ? 2 : 1;
